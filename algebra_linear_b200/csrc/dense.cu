@@ -3,11 +3,13 @@
 //
 // Schedule for an m x nc matrix (m >= nc), block-panel width nb, leaf nbl:
 //   for each block-panel [k0, k0+kb):
-//     for each leaf [c0, c0+w) inside it:
-//       K1 panel_cluster_kernel   : factor rows [c0, m) of the leaf columns,
-//                                   swap the block-panel's other columns
-//       K3 trsm (w rows)          : U of the leaf's rows, block-panel columns right of it
-//       K4 gemm (k = w)           : rows below, block-panel columns right of the leaf
+//     K1r panel_reg_kernel        : up to 64 columns per launch where rows
+//                                   [c0, m) of them fit a cluster's shared
+//                                   memory, else a leaf [c0, c0+w) of nbl;
+//                                   swaps the block-panel's other columns
+//     and for block-panel columns right of what one launch factors:
+//       K3 trsm (w rows)          : U of its rows
+//       K4 gemm (k = w)           : the rows below
 //     K2 laswp_outside            : the block-panel's interchanges, all other columns
 //     K3 trsm (kb rows)           : U12 = L11^{-1} A12
 //     K4 gemm (k = kb)            : A22 -= L21 U12
@@ -39,10 +41,11 @@ LuPlan default_plan(int n, int elem_bytes) {
 namespace {
 
 // Rows per CTA the cluster size aims for: fewer rows per CTA shorten each
-// column step, more CTAs lengthen the cluster barrier. ALG_PANEL_ROWS
-// overrides it (tuning). 256 (one register row per thread up to 4 096 rows)
-// measured 171.4 ms against 175.4 ms for 512 (fp64_fma, n = 16384) and
-// 229 ms against 264 ms per 48^3 sparse round.
+// column step, the exchange between CTAs costs about 0.35 us a column.
+// ALG_PANEL_ROWS overrides it (tuning). 256 (one register row per thread up
+// to 4 096 rows): a 64-column block of 256 / 512 / 1 024 / 2 048 FP64 rows in
+// 59 / 74 / 77 / 81 us; 128 rows per CTA: 63 / 66 / 72 / 86 us; 512 rows per
+// CTA leave no room for the block (120 us and more, leaf by leaf).
 int panel_target_rows() {
   static int v = [] {
     const char* e = std::getenv("ALG_PANEL_ROWS");
@@ -94,16 +97,44 @@ int launch_panel_w(alg_ctx* ctx, const PanelArgs<T>& args) {
   return ALG_OK;
 }
 
-template <typename T, int W, int RPT, bool EXACT>
+// Leaf width of the register panel and the dynamic shared memory it may use.
+template <typename T>
+constexpr int panel_leaf_w() {
+  return sizeof(T) == 8 ? 16 : 32;
+}
+constexpr size_t kBlockPanelSmem = 200 * 1024;
+
+// CTAs of the cluster for an m-row panel, and whether a block of kBlockMaxW
+// columns fits their shared memory (one launch instead of a leaf panel, a
+// TRSM and an update per leaf).
+int panel_ctas(int m) {
+  int C = 1;
+  while (C < kPanelMaxC && (m + C - 1) / C > panel_target_rows()) C *= 2;
+  return C;
+}
+template <typename T>
+bool block_panel_fits(int m) {
+  const int C = panel_ctas(m), R = (m + C - 1) / C;
+  return R <= 512 && block_panel_smem<T, panel_leaf_w<T>()>(R, kBlockMaxW) <= kBlockPanelSmem &&
+         !std::getenv("ALG_PANEL_SMEM");
+}
+
+template <typename T, int W, int NT, int RPT, bool EXACT>
 int launch_panel_reg(alg_ctx* ctx, const PanelArgs<T>& args, int C) {
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(panel_reg_kernel<T, W, RPT, EXACT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  static const cudaError_t configured = [] {
+    cudaError_t e = cudaFuncSetAttribute(panel_reg_kernel<T, W, NT, RPT, EXACT>,
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(panel_reg_kernel<T, W, NT, RPT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kBlockPanelSmem);
+    return e;
+  }();
   ALG_CUDA_TRY(configured);
   const int m = args.n - args.c0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
-  cfg.blockDim = dim3(kPanelRThreads, 1, 1);
-  cfg.dynamicSmemBytes = 0;
+  cfg.blockDim = dim3(NT, 1, 1);
+  cfg.dynamicSmemBytes = block_panel_smem<T, W>((m + C - 1) / C, args.w);
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -115,38 +146,35 @@ int launch_panel_reg(alg_ctx* ctx, const PanelArgs<T>& args, int C) {
   double pflops = 0;
   for (int j = 0; j < args.w; ++j) pflops += double(m - j - 1) * (1.0 + 2.0 * (args.w - j - 1));
   const int tok = prof_begin(ctx, ALG_K_PANEL);
-  ALG_CUDA_TRY(cudaLaunchKernelEx(&cfg, panel_reg_kernel<T, W, RPT, EXACT>, args));
+  ALG_CUDA_TRY(cudaLaunchKernelEx(&cfg, panel_reg_kernel<T, W, NT, RPT, EXACT>, args));
   count_launches();
   prof_end(ctx, tok, pflops, 2.0 * sizeof(T) * m * args.w);
   return ALG_OK;
 }
 
-// Register-resident rows when a 16-CTA cluster can hold the panel's rows at
-// up to four rows per thread (two for 32 double columns); the shared-memory
-// slab kernel otherwise.
+// Register-resident rows when a 16-CTA cluster holds the panel's rows at up
+// to three rows per thread (16 384 rows); the shared-memory slab kernel for
+// longer panels and for 32 double columns. One row per thread while 256
+// threads suffice (two rows on half the threads: 69 us against 59 us for a
+// 64-column block of 256 rows); beyond that more rows per thread, since more
+// warps lengthen every barrier and reduction (8 192 rows, 16 columns: 256 x 2
+// 23.2 us, 512 x 1 23.8 us; 16 384 rows: 352 x 3 30.3 us, 512 x 2 31.0 us).
+// Measured (FP64 exact form, all kernels of 16 columns / of a 64-column
+// block, us; before: a kernel that moved the rows, with labels and row j in
+// its records, and a TRSM and an update launch per leaf):
+//   rows      256       1 024     4 096     6 000     16 384
+//   before    45 / 237  47 / 243  49 / 249   - / 292  102 /  -
+//   now       14 / 60   18 / 78   19 / 95    - / 113   32 /  -
 template <typename T, bool EXACT>
 int launch_panel(alg_ctx* ctx, const PanelArgs<T>& args) {
+  constexpr int W = panel_leaf_w<T>();
   const int m = args.n - args.c0;
-  const int max_rpt = (args.w > 16 && sizeof(T) == 8) ? 2 : 4;
-  const int target = std::max(1, panel_target_rows());
-  if (m <= kPanelMaxC * kPanelRThreads * max_rpt && !std::getenv("ALG_PANEL_SMEM")) {
-    int C = 1;
-    while (C < kPanelMaxC && (m + C - 1) / C > std::min(target, max_rpt * kPanelRThreads)) C *= 2;
-    while (C < kPanelMaxC && (m + C - 1) / C > max_rpt * kPanelRThreads) C *= 2;
-    const int R = (m + C - 1) / C;
-    const int rpt = R <= kPanelRThreads ? 1 : (R <= 2 * kPanelRThreads ? 2 : 4);
-    if (args.w <= 16) {
-      if (rpt == 1) return launch_panel_reg<T, 16, 1, EXACT>(ctx, args, C);
-      if (rpt == 2) return launch_panel_reg<T, 16, 2, EXACT>(ctx, args, C);
-      return launch_panel_reg<T, 16, 4, EXACT>(ctx, args, C);
-    }
-    if (rpt == 1) return launch_panel_reg<T, 32, 1, EXACT>(ctx, args, C);
-    if constexpr (sizeof(T) == 8) {
-      return launch_panel_reg<T, 32, 2, EXACT>(ctx, args, C);
-    } else {
-      if (rpt == 2) return launch_panel_reg<T, 32, 2, EXACT>(ctx, args, C);
-      return launch_panel_reg<T, 32, 4, EXACT>(ctx, args, C);
-    }
+  const int C = panel_ctas(m), R = (m + C - 1) / C;
+  if ((args.w <= W || block_panel_fits<T>(m)) && R <= 1024 && !std::getenv("ALG_PANEL_SMEM")) {
+    if (R <= 128) return launch_panel_reg<T, W, 128, 1, EXACT>(ctx, args, C);
+    if (R <= 256) return launch_panel_reg<T, W, 256, 1, EXACT>(ctx, args, C);
+    if (R <= 512) return launch_panel_reg<T, W, 256, 2, EXACT>(ctx, args, C);
+    return launch_panel_reg<T, W, 352, 3, EXACT>(ctx, args, C);
   }
   if (args.w <= 16) return launch_panel_w<T, 16, EXACT>(ctx, args);
   return launch_panel_w<T, 32, EXACT>(ctx, args);
@@ -339,8 +367,10 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
 
   // the leaf panels of block [k0, k0 + kb), with their in-block updates
   auto factor_block = [&](int k0, int kb, int* lb) -> int {
-    for (int c0 = k0; c0 < k0 + kb; c0 += nbl) {
-      const int w = std::min(nbl, k0 + kb - c0);
+    for (int c0 = k0, w = 0; c0 < k0 + kb; c0 += w) {
+      // a whole block per launch where it fits on the chip, else leaf by leaf
+      const bool whole = !tslu_ws && nbl == panel_leaf_w<T>() && block_panel_fits<T>(m - c0);
+      w = std::min(whole ? kBlockMaxW : nbl, k0 + kb - c0);
       PanelArgs<T> pa;
       pa.a = a;
       pa.lda = lda;

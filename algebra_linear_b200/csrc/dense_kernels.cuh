@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace alg {
@@ -147,14 +149,14 @@ __device__ __forceinline__ void mbar_arm(uint32_t bar, int bytes) {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, int parity) {
   uint32_t done = 0;
   uint64_t t0 = 0;
-  for (int it = 0;; ++it) {
+  for (int it = 1;; ++it) {
     asm volatile(
         "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
-    if ((it & 63) == 0) {
+    if ((it & 63) == 0) {  // the timer is read only once the wait is long
       const uint64_t t = global_timer_ns();
-      if (it == 0) t0 = t;
+      if (t0 == 0) t0 = t;
       else if (t - t0 > kWaitLimitNs) return false;
     }
   }
@@ -485,31 +487,157 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(PanelAr
 }
 
 // ---------------------------------------------------------------------------
-// K1r: leaf panel LU with register-resident rows (m <= 16 * 256 * RPT).
+// K1r: LU of a block of columns by one thread-block cluster, rows resident on
+// the chip (m <= 16 * NT * RPT).
 //
-// Same cluster decomposition and st.async pivot exchange as K1, but every
-// thread keeps RPT whole rows of the slab (W entries each) in registers for
-// the whole panel, so the per-column update is W independent multiply-
-// subtracts per row with no shared-memory round trips, and the column loop is
-// unrolled (register indices are static). Per column: candidate from
-// registers -> warp shuffle -> one CTA barrier -> warp 0 sends the CTA record
-// -> every thread waits on its CTA's mbarrier -> swap / divide / update.
+// Factors columns [c0, c0 + bw) of rows [c0, n) in leaves of W columns. The
+// kernel is bound by the latency of its column chain (search, exchange,
+// divide, update), so each link is kept short and nothing else is launched
+// between the leaves:
+//  * A thread keeps RPT whole rows of the current leaf in registers. Rows
+//    never move: a row carries its current position instead, an interchange
+//    of rows j and p sets two positions, and the rows are written to their
+//    final positions at the end.
+//  * The rank-1 update writes entry c into entry c - 1, so the pivot column
+//    is always entry 0 and one copy of the column's code (small enough for
+//    the instruction cache: unrolled by four columns, fetching it was a third
+//    of the time) serves the whole leaf with static register indices. What
+//    leaves the register row is final and goes to the tile in shared memory:
+//    a multiplier from its own thread, a pivot row from its record.
+//  * Candidates are compared as integers by redux.sync over the high word,
+//    the low word and the position.
+//  * The reciprocal of a candidate is formed beside the search and travels
+//    in its record, so no thread divides after the exchange.
+//  * A pivot is filed (its U entries, its multipliers, the interchange) by one
+//    warp, another each column; what it fetches is stored a column later.
+// Per column: candidate -> redux -> the warp's best lane stages its row ->
+// one CTA barrier -> the CTA's best record to every mailbox (16-byte st.async,
+// the CTAs spread over the warps, completing on the receiver's mbarrier) ->
+// wait on the own mbarrier -> redux over the C records -> divide and update.
+// C == 1 skips the exchange. Mailboxes and mbarriers alternate by column
+// parity as in K1.
+//
+// With more than one leaf (bw > W) the columns right of the leaf wait in the
+// tile (tile[col][row]). A pivot row's entries there, and its multipliers,
+// are pulled from its owner's tile by the filing warp of every CTA (the owner's record vouches for its tile: it was sent after
+// the CTA barrier that follows the last update). At the leaf's end every CTA
+// solves U12 = L11^{-1} A12 for itself and updates its own rows, each entry's
+// terms in increasing k.
 //
 // Division: the multiplier is the correctly rounded quotient a/d
-// (mod.rs:154). With y = RN(1/d) computed once per column, q = RN(a*y) is
-// within one ulp of a/d, the remainder a - q*d is exact under an FMA, and
-// RN(q + (a - q*d)*y) is the correctly rounded quotient (Markstein's
-// theorem), as long as nothing over- or underflows; entries and pivots outside
-// [2^-500, 2^500] in magnitude, zeros and non-finite values take the plain
-// IEEE division instead.
+// (mod.rs:154). With y = RN(1/d), q = RN(a*y) is within one ulp of a/d, the
+// remainder a - q*d is exact under an FMA, and RN(q + (a - q*d)*y) is the
+// correctly rounded quotient (Markstein's theorem), as long as nothing over-
+// or underflows; a zero a keeps q, the zero with the quotient's sign; other
+// entries and pivots outside [2^-500, 2^500] in magnitude and non-finite
+// values take the plain IEEE division instead.
 // ---------------------------------------------------------------------------
-constexpr int kPanelRThreads = 256;
 
-template <typename T, int W, int RPT, bool EXACT>
-__global__ void __launch_bounds__(kPanelRThreads, 1) panel_reg_kernel(PanelArgs<T> p) {
-  using Rec = PanelRec<T, W>;
-  constexpr int NT = kPanelRThreads;
+// A pivot candidate: |v|'s bits as an ordered integer and the row's position;
+// (0, INT_MAX) is no candidate (a zero entry is (0, its position), which wins
+// over it). The reference's NaN rule (mod.rs:123-134): +inf on the diagonal,
+// never chosen elsewhere.
+__device__ __forceinline__ void pivot_candidate(double v, int pos, int J, unsigned long long& key, int& kpos) {
+  key = pos >= J ? (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull : 0ull;
+  kpos = pos >= J ? pos : INT_MAX;
+  if (v != v) {
+    key = pos == J ? 0x7ff0000000000000ull : 0ull;
+    kpos = pos == J ? J : INT_MAX;
+  }
+}
+__device__ __forceinline__ void pivot_candidate(float v, int pos, int J, unsigned& key, int& kpos) {
+  key = pos >= J ? __float_as_uint(v) & 0x7fffffffu : 0u;
+  kpos = pos >= J ? pos : INT_MAX;
+  if (v != v) {
+    key = pos == J ? 0x7f800000u : 0u;
+    kpos = pos == J ? J : INT_MAX;
+  }
+}
+// Warp-wide: the largest key, and among its lanes the smallest tag; true on
+// the lanes that hold both.
+__device__ __forceinline__ bool warp_pivot(unsigned long long key, int tag, unsigned long long& mk, int& mt) {
+  const unsigned hi = (unsigned)(key >> 32);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)key : 0u);
+  const bool eq = hi == mh && (unsigned)key == ml;
+  mt = __reduce_min_sync(0xffffffffu, eq ? tag : INT_MAX);
+  mk = ((unsigned long long)mh << 32) | ml;
+  return eq && tag == mt;
+}
+__device__ __forceinline__ bool warp_pivot(unsigned key, int tag, unsigned& mk, int& mt) {
+  mk = __reduce_max_sync(0xffffffffu, key);
+  const bool eq = key == mk;
+  mt = __reduce_min_sync(0xffffffffu, eq ? tag : INT_MAX);
+  return eq && tag == mt;
+}
+// The same over the records rec[0 .. count) (one lane each): the winner's
+// index; its position in mp. Positions are below 2^20 (longer panels take
+// another kernel), so position and index share one reduction.
+template <typename Rec>
+__device__ __forceinline__ int warp_pick(const Rec* rec, int count, int lane, int& mp) {
+  typename Rec::Key k = 0, mk;
+  int t = INT_MAX, mt;
+  if (lane < count) {
+    const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(&rec[lane]);  // key; position and slot
+    k = (typename Rec::Key)h.x;
+    const unsigned pos = (unsigned)h.y;
+    t = pos < (1u << 20) ? (int)(pos << 5 | (unsigned)lane) : INT_MAX - 31 + lane;
+  }
+  warp_pivot(k, t, mk, mt);
+  mp = mt >> 5;
+  return mt & 31;
+}
+// div_fast_ok on the exponent bits (also false for zero, infinity and NaN)
+__device__ __forceinline__ bool exp_fast_ok(double v) {
+  const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+  return e - (1023u - 500u) < 1000u;  // [2^-500, 2^500)
+}
+__device__ __forceinline__ bool exp_fast_ok(float v) {
+  const unsigned e = (__float_as_uint(v) >> 23) & 0xffu;
+  return e - (127u - 60u) < 120u;  // [2^-60, 2^60)
+}
+__device__ __forceinline__ void st_async_v2(uint32_t remote, ulonglong2 v, uint32_t remote_bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];"
+               :: "r"(remote), "l"(v.x), "l"(v.y), "r"(remote_bar) : "memory");
+}
+__device__ __forceinline__ void ld_cluster(double& v, uint32_t a) {
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ld_cluster(float& v, uint32_t a) {
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+}
+
+// A pivot record, in 16-byte chunks: (key; position and the row's slot in its
+// CTA), (reciprocal, unused), then the leaf's row, rotated as in registers.
+template <typename T, int W>
+struct alignas(16) PivotRec {
+  using Key = std::conditional_t<sizeof(T) == 8, unsigned long long, unsigned>;
+  unsigned long long key;
+  unsigned pos, slot;
+  T recip;
+  alignas(16) T row[W];
+  static constexpr int kChunks = 2 + W * (int)sizeof(T) / 16;
+};
+
+constexpr int kBlockMaxW = 64;  // columns of a block that one launch factors
+
+// Dynamic shared memory: the tile and, with more than one leaf, the U12 rows
+// of the current leaf ([col][k]) and its unit-lower block.
+template <typename T, int W>
+__host__ __device__ inline size_t block_panel_smem(int rows_per_cta, int bw) {
+  return sizeof(T) * ((size_t)bw * ((rows_per_cta + 1) & ~1) + (bw > W ? (size_t)bw * W : 0));
+}
+
+template <typename T, int W, int NT, int RPT, bool EXACT>
+__global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
+  using Rec = PivotRec<T, W>;
+  using Key = typename Rec::Key;
+  static_assert(sizeof(Rec) == 16 * Rec::kChunks && Rec::kChunks <= 16, "record layout");
   constexpr int NW = NT / 32;
+  constexpr int kVec = 16 / (int)sizeof(T);
+  struct alignas(16) Vec {
+    T e[kVec];
+  };
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks();
   const int q = (int)cl.block_rank();
@@ -518,292 +646,315 @@ __global__ void __launch_bounds__(kPanelRThreads, 1) panel_reg_kernel(PanelArgs<
   const int m = p.n - p.c0;
   const int R = (m + C - 1) / C;
   const int rb = q * R;
-  const int re = min(m, rb + R);
-  const int nr = max(0, re - rb);
-  const int w = p.w;
-  const int step_bytes = C * Rec::kBytes + Rec::kDiagBytes;
+  const int nr = max(0, min(m, rb + R) - rb);
+  const int bw = p.w;  // columns of this launch
+  const bool multi = bw > W;
+  const int ldt = (R + 1) & ~1;  // tile column stride
+  const int step_bytes = C * (int)sizeof(Rec);
 
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* l11 = reinterpret_cast<T*>(smem_raw);       // W x W: the leaf's unit-lower block, [row][col]
+  T* ubuf = l11 + W * W;                         // (bw - W) x W: its U12, [col][k]
+  T* tile = l11 + (multi ? (size_t)bw * W : 0);  // bw x ldt
   __shared__ unsigned long long mbar[2];
-  __shared__ __align__(16) unsigned long long rec[2][kPanelMaxC][Rec::kWords];
-  __shared__ __align__(16) unsigned long long diag[2][Rec::kDiagWords];
-  __shared__ double cand_key[2][NW];
-  __shared__ int cand_idx[2][NW];
-  __shared__ int cand_lab[2][NW][2];
-  __shared__ T stage[2][NW][W];
-  __shared__ T dstage[2][W];
-  __shared__ int dlab[2][2];
-  __shared__ T side_vals[4 * kPanelMaxW][kSideCols];
-  __shared__ int side_rows[4 * kPanelMaxW];
-  __shared__ int side_src[4 * kPanelMaxW];
+  // [par][0, C): the mailboxes; [par][kPanelMaxC + warp]: the warps' stages
+  __shared__ Rec rec[2][kPanelMaxC + NW];
+  __shared__ int side_src[2 * kBlockMaxW];
+  __shared__ int side_dst[2 * kBlockMaxW];
   __shared__ int side_cnt;
 
-  // ---- rows into registers ----------------------------------------------
+  // ---- load --------------------------------------------------------------
   T v[RPT][W];
-  int lab[RPT], loc[RPT];
+  int pos[RPT];  // the row's position in the panel (-1: no row)
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int r = tid + k * NT;  // local row
     const bool in = r < nr;
-    const int gr = p.c0 + rb + r;
+    const T* row = p.a + (size_t)(p.c0 + rb + r) + (size_t)p.c0 * p.lda;
+    pos[k] = in ? rb + r : -1;
 #pragma unroll
-    for (int cc = 0; cc < W; ++cc)
-      v[k][cc] = (in && cc < w) ? p.a[(size_t)gr + (size_t)(p.c0 + cc) * p.lda] : T(0);
-    lab[k] = in ? (p.first_leaf ? gr : p.lab[gr]) : 0;
-    loc[k] = gr;
+    for (int c = 0; c < W; ++c) v[k][c] = (in && c < bw) ? row[(size_t)c * p.lda] : T(0);
+    if (multi && r < ldt) {
+#pragma unroll 8
+      for (int c = W; c < bw; ++c) tile[c * ldt + r] = in ? row[(size_t)c * p.lda] : T(0);
+    }
   }
-  if (tid == 0 && C > 1) {
-    mbar_init(smem_u32(&mbar[0]), 1);
-    mbar_init(smem_u32(&mbar[1]), 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_arm(smem_u32(&mbar[0]), step_bytes);
-    if (w > 1) mbar_arm(smem_u32(&mbar[1]), step_bytes);
+  if (tid == 0) {
+    side_cnt = 0;
+    if (C > 1) {
+      mbar_init(smem_u32(&mbar[0]), 1);
+      mbar_init(smem_u32(&mbar[1]), 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      mbar_arm(smem_u32(&mbar[0]), step_bytes);
+      if (bw > 1) mbar_arm(smem_u32(&mbar[1]), step_bytes);
+    }
   }
   cl.sync();
 
-  const uint32_t rec_base = smem_u32(&rec[0][0][0]);
-  const uint32_t diag_base = smem_u32(&diag[0][0]);
   const uint32_t bar_base = smem_u32(&mbar[0]);
+  const uint32_t tile_base = smem_u32(tile);
   bool ok_wait = true;
+  // the mailboxes (slot q, this lane's chunk) and mbarriers this lane sends to
+  constexpr int kSends = (kPanelMaxC + 2 * NW - 1) / (2 * NW);
+  const int chunk = lane & 15;
+  uint32_t rem_rec[kSends], rem_bar[kSends];
+#pragma unroll
+  for (int i = 0; i < kSends; ++i) {
+    const int t = min(warp + NW * (2 * i + (lane >> 4)), C - 1);
+    rem_rec[i] = mapa_u32(smem_u32(&rec[0][q]) + 16u * chunk, t);
+    rem_bar[i] = mapa_u32(bar_base, t);
+  }
 
-  // The column loop stays rolled: one copy of its code serves every column
-  // (an unrolled loop does not fit the instruction cache). Register entries
-  // are addressed with static indices under the predicates c == j / c > j.
 #pragma unroll 1
-  for (int j = 0; j < w; ++j) {
-    {
-      const int par = j & 1;
-      // ---- 1. candidate for column j from the registers ---------------------
-      double bk = -CUDART_INF;
-      int bi = INT_MAX;
+  for (int cl0 = 0; cl0 < bw; cl0 += W) {
+    const int w = min(W, bw - cl0);
+    const int tc = bw - cl0 - w;  // columns of the block right of the leaf
+    // the filed pivot row's multipliers and its entries right of the leaf,
+    // fetched in one column and stored in the next
+    T pull[2];
+    auto keep_pull = [&](int j) {
 #pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        const int r = tid + k * NT;
-        T vj = v[k][0];
+      for (int i = 0; i < 2; ++i) {
+        const int c = lane + 32 * i;
+        if (c < j) l11[j * W + c] = pull[i];
+        else if (c >= W && c < W + tc) ubuf[(c - W) * W + j] = pull[i];
+      }
+    };
+#pragma unroll 1
+    for (int j = 0; j < w; ++j) {
+      const int J = cl0 + j;  // column of the launch = row position of its pivot
+      const int par = J & 1;
+      int mp;
+      // ---- 1. the thread's, then the warp's candidate ------------------------
+      Key key, mk;
+      int kpos, kslot = tid;
+      T cand = v[0][0];
+      pivot_candidate(v[0][0], pos[0], J, key, kpos);
 #pragma unroll
-        for (int cc = 1; cc < W; ++cc)
-          if (cc == j) vj = v[k][cc];
-        if (r < nr && rb + r >= j) {
-          const double key = pivot_key((double)vj, rb + r == j);
-          if (key > bk) { bk = key; bi = rb + r; }
+      for (int k = 1; k < RPT; ++k) {
+        Key kk;
+        int kp;
+        pivot_candidate(v[k][0], pos[k], J, kk, kp);
+        if (kk > key || (kk == key && kp < kpos)) {
+          key = kk;
+          kpos = kp;
+          kslot = tid + k * NT;
+          cand = v[k][0];
         }
       }
-      // owner of row j stages it (and its labels) for the diagonal record
+      const T crecip = rcp_rn(exp_fast_ok(cand) ? cand : T(1));
+      if (warp_pivot(key, kpos, mk, mp)) {  // (no candidate at all: any lanes, an empty record)
+        Rec& s = rec[par][kPanelMaxC + warp];
+        s.key = mk;
+        s.pos = (unsigned)mp;
+        s.slot = kslot;
+        s.recip = crecip;
 #pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        if (tid + k * NT < nr && rb + tid + k * NT == j) {
+        for (int k = 0; k < RPT; ++k)
+          if (RPT == 1 || kslot == tid + k * NT) {
 #pragma unroll
-          for (int cc = 0; cc < W; ++cc) dstage[par][cc] = v[k][cc];
-          dlab[par][0] = lab[k];
-          dlab[par][1] = loc[k];
-        }
-      }
-      double wk = bk;
-      int wi = bi;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const double ok = __shfl_xor_sync(0xffffffffu, wk, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, wi, off);
-        keyidx_combine(wk, wi, ok, oi);
-      }
-      // the lane holding the warp's best row stages it
-      if (wi != INT_MAX) {
-#pragma unroll
-        for (int k = 0; k < RPT; ++k) {
-          if (tid + k * NT < nr && rb + tid + k * NT == wi) {
-            cand_key[par][warp] = wk;
-            cand_idx[par][warp] = wi;
-            cand_lab[par][warp][0] = lab[k];
-            cand_lab[par][warp][1] = loc[k];
-#pragma unroll
-            for (int cc = 0; cc < W; ++cc) stage[par][warp][cc] = v[k][cc];
+            for (int c = 0; c < W; ++c) s.row[c] = v[k][c];
           }
-        }
-      } else if (lane == 0) {
-        cand_key[par][warp] = -CUDART_INF;
-        cand_idx[par][warp] = INT_MAX;
       }
       __syncthreads();
-      // ---- 2. the CTA record (and row j) to every mailbox: each of the first
-      // min(NW, C) warps forms the record and sends it to the CTAs t with
-      // t % NW == warp (C == 1: warp 0 into the own mailbox) -------------------
-      if (warp < (C > 1 ? min(NW, C) : 1)) {
-        double ck = -CUDART_INF;
-        int ci = INT_MAX, cw = 0;
-        if (lane < NW) { ck = cand_key[par][lane]; ci = cand_idx[par][lane]; cw = lane; }
+      // ---- 2. the CTA's candidate ----------------------------------------
+      int win = kPanelMaxC + warp_pick(&rec[par][kPanelMaxC], NW, lane, mp), owner = q;
+      if (C > 1) {
+        // the record to every mailbox: half-warps of 16-byte chunks, CTAs
+        // t = warp, warp + NW, ... (slot q of the mailboxes)
+        if (chunk < Rec::kChunks) {
+          const ulonglong2 val = reinterpret_cast<const ulonglong2*>(&rec[par][win])[chunk];
+          const uint32_t off = (uint32_t)(par * (kPanelMaxC + NW) * (int)sizeof(Rec));
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          const double ok = __shfl_xor_sync(0xffffffffu, ck, off);
-          const int oi = __shfl_xor_sync(0xffffffffu, ci, off);
-          const int ow = __shfl_xor_sync(0xffffffffu, cw, off);
-          if (ok > ck || (ok == ck && oi < ci)) { ck = ok; ci = oi; cw = ow; }
+          for (int i = 0; i < kSends; ++i)
+            if (warp + NW * (2 * i + (lane >> 4)) < C) st_async_v2(rem_rec[i] + off, val, rem_bar[i] + 8u * par);
         }
-        const bool have = ci != INT_MAX;
-        const T* crow = &stage[par][cw][0];
-        const bool own_j = j >= rb && j < re;
-        // lane kw builds word kw of the record in a register and stores it
-        // into slot q of its CTAs' mailboxes with st.async (each 8-byte store
-        // completes on that CTA's mbarrier); C == 1: straight into the own
-        // mailbox. No staging in shared memory, no proxy fence, no bulk copy.
-        const uint32_t bar_par = bar_base + 8u * par;
-        for (int kw = lane; kw < Rec::kWords; kw += 32) {
-          unsigned long long val = 0;
-          if (kw == 0) val = (unsigned long long)__double_as_longlong(ck);
-          else if (kw == 1) val = pack_ii(ci, have ? cand_lab[par][cw][0] : 0);
-          else if (kw == 2) val = pack_ii(have ? cand_lab[par][cw][1] : 0, 0);
-          else if (kw < 3 + Rec::kRowWords) val = row_word<T, W>(crow, kw - 3);
-          if (C > 1) {
-            const uint32_t la = rec_base + 8u * (uint32_t)((par * kPanelMaxC + q) * Rec::kWords + kw);
-            for (int t = warp; t < C; t += NW) st_async_b64(mapa_u32(la, t), val, mapa_u32(bar_par, t));
-          } else {
-            rec[par][0][kw] = val;
-          }
-        }
-        if (own_j) {
-          for (int kw = lane; kw < Rec::kDiagWords; kw += 32) {
-            unsigned long long val = 0;
-            if (kw == 0) val = pack_ii(dlab[par][0], dlab[par][1]);
-            else if (kw < 1 + Rec::kRowWords) val = row_word<T, W>(&dstage[par][0], kw - 1);
-            if (C > 1) {
-              const uint32_t ld = diag_base + 8u * (uint32_t)(par * Rec::kDiagWords + kw);
-              for (int t = warp; t < C; t += NW) st_async_b64(mapa_u32(ld, t), val, mapa_u32(bar_par, t));
-            } else {
-              diag[par][kw] = val;
-            }
-          }
-        }
-      }
-      // ---- 3. wait for this column's records; every warp picks the winner ---
-      if (C == 1) {
-        __syncthreads();
-      } else {
-        if (ok_wait && !mbar_wait(bar_base + 8u * par, (j >> 1) & 1)) {
+        // ---- 3. wait for this column's records; every warp picks the winner
+        // (a wait that ran out stays failed: the rest of the launch runs
+        // through without waiting and the host reports ALG_TIMEOUT)
+        if (ok_wait && !mbar_wait(bar_base + 8u * par, (J >> 1) & 1)) {
           ok_wait = false;
           atomicExch(&p.status->timeout, 1);
         }
-        if (tid == 0 && j + 2 < w) mbar_arm(bar_base + 8u * par, step_bytes);
+        if (tid == 0 && J + 2 < bw) mbar_arm(bar_base + 8u * par, step_bytes);
+        __syncwarp();
+        win = owner = warp_pick(&rec[par][0], C, lane, mp);
       }
-      double xk = -CUDART_INF;
-      int xi = INT_MAX, xs = 0;
-      if (lane < C) {
-        xk = __longlong_as_double((long long)rec[par][lane][0]);
-        xi = (int)(unsigned)(rec[par][lane][1] & 0xffffffffu);
-        xs = lane;
-      }
+      if (multi && j > 0 && warp == ((j - 1) % NW)) keep_pull(j - 1);
+      const Rec& wr = rec[par][win];
+      const int pr = ok_wait ? mp : J;  // winning row's position (>= J)
+      const T d = wr.row[0];
+      const T y = wr.recip;
+      // one warp files the pivot row ------------------------------------
+      if (warp == (j % NW)) {
+        const int slot = ok_wait ? (int)wr.slot : 0;
+        if (owner == q && lane < w - j) tile[(J + lane) * ldt + slot] = wr.row[lane];
+        if (lane == 0 && q == 0) {
+          p.ipiv[p.c0 + J] = p.c0 + pr;
+          if (d == T(0)) atomicMin(&p.status->singular_col, p.c0 + J);
+        }
+        if (multi) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const double ok = __shfl_xor_sync(0xffffffffu, xk, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, xi, off);
-        const int os = __shfl_xor_sync(0xffffffffu, xs, off);
-        if (ok > xk || (ok == xk && oi < xi)) { xk = ok; xi = oi; xs = os; }
-      }
-      const int pr = xi;  // winning panel row (>= j)
-      const int ps = xs;  // CTA that sent it
-      T u[W];
-#pragma unroll
-      for (int cc = 0; cc < W; ++cc) u[cc] = rec_entry<T>(&rec[par][ps][3], cc);
-      const T d = rec_entry<T>(&rec[par][ps][3], j);
-      // ---- 4. swap rows j and pr (registers of their owners) ----------------
-#pragma unroll
-      for (int k = 0; k < RPT; ++k) {
-        const int r = tid + k * NT;
-        if (r < nr) {
-          if (rb + r == j) {
-#pragma unroll
-            for (int cc = 0; cc < W; ++cc) v[k][cc] = u[cc];
-            lab[k] = (int)(unsigned)(rec[par][ps][1] >> 32);
-            loc[k] = (int)(unsigned)(rec[par][ps][2] & 0xffffffffu);
-          } else if (rb + r == pr) {
-#pragma unroll
-            for (int cc = 0; cc < W; ++cc) v[k][cc] = rec_entry<T>(&diag[par][1], cc);
-            lab[k] = (int)(unsigned)(diag[par][0] & 0xffffffffu);
-            loc[k] = (int)(unsigned)(diag[par][0] >> 32);
+          for (int i = 0; i < 2; ++i) {
+            const int c = lane + 32 * i;
+            if (c < j || (c >= W && c < W + tc))
+              ld_cluster(pull[i], mapa_u32(tile_base + (uint32_t)sizeof(T) * ((cl0 + c) * ldt + slot), owner));
           }
         }
       }
-      if (tid == 0 && q == 0) {
-        p.ipiv[p.c0 + j] = p.c0 + pr;
-        if (fabs((double)d) <= 0.0) atomicMin(&p.status->singular_col, p.c0 + j);
-      }
-      // ---- 5. divide and update the rows below j -----------------------------
-      const bool fast = div_fast_ok(d);
-      const T y = fast ? rcp_rn(d) : T(1);
+      // ---- 4. rows J and pr change places; divide and update below J -------
+      const bool fast = exp_fast_ok(d);
       T l[RPT];
-      bool fix = false;
-      T av[RPT];
+      bool odd = false;
 #pragma unroll
       for (int k = 0; k < RPT; ++k) {
-        av[k] = v[k][0];
-#pragma unroll
-        for (int cc = 1; cc < W; ++cc)
-          if (cc == j) av[k] = v[k][cc];
-        const T qv = mul_rn(av[k], y);
-        l[k] = fma_rn(fma_rn(-qv, d, av[k]), y, qv);
-        fix |= !(fast && div_fast_ok(av[k])) && (tid + k * NT < nr) && (rb + tid + k * NT > j);
+        if (pos[k] == pr) pos[k] = J;
+        else if (pos[k] == J) pos[k] = pr;
+        const T av = v[k][0];
+        const T qv = mul_rn(av, y);
+        l[k] = fma_rn(fma_rn(-qv, d, av), y, qv);
+        odd |= !(fast && exp_fast_ok(av)) && pos[k] > J;
       }
-      if (fix) {  // zeros, non-finite values, extreme exponents: plain IEEE division
+      if (odd) {  // zeros; rarely the plain IEEE division
 #pragma unroll
-        for (int k = 0; k < RPT; ++k)
-          if (!(fast && div_fast_ok(av[k]))) l[k] = div_rn(av[k], d);
+        for (int k = 0; k < RPT; ++k) {
+          const T av = v[k][0];
+          if (!(fast && exp_fast_ok(av))) l[k] = (fast && av == T(0)) ? mul_rn(av, y) : div_rn(av, d);
+        }
       }
+#pragma unroll
+      for (int k = 0; k < RPT; ++k)
+        if (pos[k] > J) tile[J * ldt + tid + k * NT] = l[k];
+      // (entries past the leaf's live columns, and rows that have left, hold
+      // values that nothing reads)
+#pragma unroll
+      for (int c = 1; c < W; ++c) {
+        const T u = wr.row[c];
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) v[k][c - 1] = msub<EXACT>(v[k][c], l[k], u);
+      }
+    }
+    if (multi && warp == ((w - 1) % NW)) keep_pull(w - 1);
+    if (tc > 0) {  // (then w == W)
+      __syncthreads();
+      if (tid < tc) {
+        T* x = ubuf + tid * W;
+        T xr[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) xr[i] = x[i];
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+#pragma unroll
+          for (int i = k + 1; i < W; ++i) xr[i] = msub<EXACT>(xr[i], l11[i * W + k], xr[k]);
+#pragma unroll
+        for (int i = 0; i < W; ++i) x[i] = xr[i];
+        if (q == 0) {
+          T* out = p.a + (size_t)(p.c0 + cl0) + (size_t)(p.c0 + cl0 + w + tid) * p.lda;
+#pragma unroll
+          for (int i = 0; i < W; ++i) out[i] = xr[i];
+        }
+      }
+      __syncthreads();
 #pragma unroll
       for (int k = 0; k < RPT; ++k) {
         const int r = tid + k * NT;
-        if (r < nr && rb + r > j) {
+        if (pos[k] >= cl0 + w) {
 #pragma unroll
-          for (int cc = 0; cc < W; ++cc) {
-            if (cc == j) v[k][cc] = l[k];
-            else if (cc > j) v[k][cc] = msub<EXACT>(v[k][cc], l[k], u[cc]);
+          for (int i = 0; i < W; ++i) v[k][i] = tile[(cl0 + i) * ldt + r];
+          T* trow = tile + (size_t)(cl0 + w) * ldt + r;
+#pragma unroll 1
+          for (int c = 0; c < tc; c += 4) {  // tc: a multiple of 4 unless the block is ragged
+            T acc[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] = c + e < tc ? trow[(c + e) * ldt] : T(0);
+#pragma unroll
+            for (int i = 0; i < W; i += kVec)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const Vec u = *reinterpret_cast<const Vec*>(ubuf + min(c + e, tc - 1) * W + i);
+#pragma unroll
+                for (int t = 0; t < kVec; ++t) acc[e] = msub<EXACT>(acc[e], v[k][i + t], u.e[t]);
+              }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (c + e < tc) trow[(c + e) * ldt] = acc[e];
           }
         }
       }
+      // the next leaf's rows
+#pragma unroll
+      for (int k = 0; k < RPT; ++k) {
+        const int r = tid + k * NT;
+#pragma unroll
+        for (int c = 0; c < W; ++c) v[k][c] = (c < tc && r < ldt) ? tile[(cl0 + w + c) * ldt + r] : T(0);
+      }
     }
   }
-  cl.sync();  // every record consumed; no DSMEM access outlives its owner
-
-  // ---- swap the block-panel's other columns by this leaf's interchanges -----
-  if (tid == 0) side_cnt = 0;
   __syncthreads();
+
+  // ---- rows to their final positions; swap the block-panel's other columns --
+  // The row loaded from c0 + rb + r moved to position pos: its content in the
+  // other columns goes the same way. All reads of a pass precede the cluster
+  // barrier, all writes follow it; the first barrier also ends the DSMEM
+  // exchange (every record and pull done before a CTA may exit).
+  int lab[RPT];  // the rows' source labels, read before any CTA writes one
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int r = tid + k * NT;
-    if (r < nr && loc[k] != p.c0 + rb + r) {
+    lab[k] = p.c0 + rb + r;
+    if (pos[k] >= 0 && !p.first_leaf) lab[k] = p.lab[p.c0 + rb + r];
+    if (pos[k] >= 0 && pos[k] != rb + r) {
       const int s = atomicAdd(&side_cnt, 1);
-      if (s < 4 * kPanelMaxW) { side_rows[s] = r; side_src[s] = loc[k]; }
+      if (s < 2 * kBlockMaxW) {
+        side_src[s] = p.c0 + rb + r;
+        side_dst[s] = p.c0 + pos[k];
+      }
     }
   }
   __syncthreads();
-  const int n_side = min(side_cnt, 4 * kPanelMaxW);
-  const int side_w = (p.kb1 - p.kb0) - w;
-  for (int cbase = 0; cbase < side_w; cbase += kSideCols) {
-    const int ncol = min(kSideCols, side_w - cbase);
-    for (int idx = tid; idx < n_side * kSideCols; idx += NT) {
-      const int s = idx / kSideCols, cc = idx % kSideCols;
-      if (cc >= ncol) continue;
-      int col = p.kb0 + cbase + cc;
-      if (col >= p.c0) col += w;
-      side_vals[s][cc] = p.a[(size_t)side_src[s] + (size_t)col * p.lda];
+  const int side_w = (p.kb1 - p.kb0) - bw;
+  const int n_side = min(side_cnt, 2 * kBlockMaxW);
+  // A pass takes the same columns in every CTA (a CTA moves at most 2 bw rows).
+  constexpr int kSidePer = 16;  // values in flight per thread and pass
+  const int pass_w = kSidePer * NT / (2 * bw);
+  const int passes = (side_w + pass_w - 1) / pass_w;
+  for (int ps = 0; ps < passes; ++ps) {
+    const int s0 = ps * pass_w;
+    const int n_move = n_side * min(pass_w, side_w - s0);
+    T sv[kSidePer];
+#pragma unroll
+    for (int i = 0; i < kSidePer; ++i) {
+      const int e = i * NT + tid;
+      if (e < n_move) {
+        int col = p.kb0 + s0 + e / n_side;
+        if (col >= p.c0) col += bw;
+        sv[i] = p.a[(size_t)side_src[e % n_side] + (size_t)col * p.lda];
+      }
     }
     cl.sync();
-    for (int idx = tid; idx < n_side * kSideCols; idx += NT) {
-      const int s = idx / kSideCols, cc = idx % kSideCols;
-      if (cc >= ncol) continue;
-      int col = p.kb0 + cbase + cc;
-      if (col >= p.c0) col += w;
-      p.a[(size_t)(p.c0 + rb + side_rows[s]) + (size_t)col * p.lda] = side_vals[s][cc];
+#pragma unroll
+    for (int i = 0; i < kSidePer; ++i) {
+      const int e = i * NT + tid;
+      if (e < n_move) {
+        int col = p.kb0 + s0 + e / n_side;
+        if (col >= p.c0) col += bw;
+        p.a[(size_t)side_dst[e % n_side] + (size_t)col * p.lda] = sv[i];
+      }
     }
-    cl.sync();
   }
+  if (passes == 0) cl.sync();
 
-  // ---- registers back to the matrix -------------------------------------
+  // ---- back to the matrix -----------------------------------------------
+  // (a pivot row's U entries right of its leaf are already there)
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
-    const int r = tid + k * NT;
-    if (r < nr) {
-      const int gr = p.c0 + rb + r;
-#pragma unroll
-      for (int cc = 0; cc < W; ++cc)
-        if (cc < w) p.a[(size_t)gr + (size_t)(p.c0 + cc) * p.lda] = v[k][cc];
-      p.lab[gr] = lab[k];
+    if (pos[k] >= 0) {
+      T* row = p.a + (size_t)(p.c0 + pos[k]) + (size_t)p.c0 * p.lda;
+      const int ce = pos[k] < bw ? min(bw, (pos[k] / W + 1) * W) : bw;
+      const T* trow = tile + tid + k * NT;
+#pragma unroll 8
+      for (int c = 0; c < ce; ++c) row[(size_t)c * p.lda] = trow[c * ldt];
+      p.lab[p.c0 + pos[k]] = lab[k];
     }
   }
 }
