@@ -6,12 +6,14 @@
 // multipliers by division, then the forward/back sweeps. A CTA pulls systems
 // from a queue ordered by decreasing order n (largest first, for balance) and
 // factorizes each one in place in its global buffer with a right-looking
-// blocked schedule: a 16- or 32-column panel factored in shared memory, its row
-// interchanges applied to the other columns by one gather, U12 by a
-// row-block triangular solve, and the trailing update in 64 x 64 tiles (U12
-// staged in shared memory, a register micro-tile per thread). The mixed form factorizes an FP32 copy and refines
-// x in FP64 against the FP64 matrix until the system's normwise backward
-// error is within tol.
+// blocked schedule: a 16- or 32-column panel factored in shared memory with
+// its rows in registers (cta_leaf), then the columns right of it in chunks:
+// gathered in the panel's row order, U12 by a blocked unit-lower solve, and
+// the trailing update on the FP64 tensor cores (FP32: register tiles). In the
+// FP64 form the right-hand side is one more column of that sweep, so the
+// forward substitution costs nothing of its own. The mixed form factorizes an
+// FP32 copy and refines x in FP64 against the FP64 matrix until the system's
+// normwise backward error is within tol.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -19,6 +21,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include <cuda.h>
@@ -26,13 +29,13 @@
 #include <math_constants.h>
 
 #include "batched.cuh"
+#include "pivot.cuh"
 
 namespace alg {
 namespace {
 
 constexpr int kMaxN = 512;    // largest order a CTA handles
-constexpr int kT = 64;        // trailing-update tile
-constexpr int kTR = 4;        // rows of a thread's micro-tile in the trailing update
+constexpr int kLeafW = 16;    // columns a leaf keeps in registers
 
 template <typename T>
 __device__ __forceinline__ T fma_t(T a, T b, T c);
@@ -41,252 +44,481 @@ __device__ __forceinline__ double fma_t<double>(double a, double b, double c) { 
 template <>
 __device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
-__device__ __forceinline__ double pkey(double v, bool diag) {
-  const double a = fabs(v);
-  if (isnan(a)) return diag ? CUDART_INF : -CUDART_INF;
-  return a;
+// Column strides in shared memory: 4 mod 16 entries, so that a half-warp's
+// DMMA fragment loads (4 k x 4 rows or columns) fall in distinct banks.
+__host__ __device__ constexpr int panel_ld(int cap) { return ((cap + 15) & ~15) + 4; }
+// Columns of the trailing matrix taken at a time.
+template <int NT>
+__host__ __device__ constexpr int chunk_cols() {
+  return NT / 4;
 }
 
-// Block-wide first-index argmax of keys (largest key, lowest index among
-// equals); returns the winning index to all threads. One barrier: each warp
-// posts its best in a mailbox slot double-buffered by `par` (the caller
-// alternates it per call, and its other barriers separate two calls with the
-// same parity), and every warp reduces the mailboxes itself.
-__device__ int block_argmax(double key, int idx, double* red_k, int* red_i, int par) {
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ok = __shfl_down_sync(0xffffffffu, key, off);
-    const int oi = __shfl_down_sync(0xffffffffu, idx, off);
-    if (ok > key || (ok == key && oi < idx)) { key = ok; idx = oi; }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) { red_k[16 * par + warp] = key; red_i[16 * par + warp] = idx; }
-  __syncthreads();
-  const int nw = (int)(blockDim.x >> 5);
-  double k = lane < nw ? red_k[16 * par + lane] : -CUDART_INF;
-  int i = lane < nw ? red_i[16 * par + lane] : INT_MAX;
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ok = __shfl_xor_sync(0xffffffffu, k, off);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, off);
-    if (ok > k || (ok == k && oi < i)) { k = ok; i = oi; }
-  }
-  return i;
+// Shared memory of cta_getrf for panels of up to `cap` rows: the leaf's
+// records, the panel [col][row], two U12 chunks [k][col] and 2 pb + 4 ints.
+// A chunk's row stride is odd in FP64: its columns arrive 32 k at a time
+// (cp.async, a row of U each), and an even stride made those stores 8-way
+// bank conflicts; the FP32 tiles need rows of whole 16 bytes.
+template <typename T, int NT>
+__host__ __device__ constexpr int chunk_ld() {
+  return chunk_cols<NT>() + (sizeof(T) == 8 ? 5 : 4);
 }
-
-// LU with partial pivoting of the n x n matrix a (global, leading dim n),
-// in place; ipiv (global, n ints); returns 0 or 1 + the first singular column.
-// Shared memory of cta_getrf for panels of up to `cap` rows.
-template <typename T>
+template <typename T, int NT>
 __host__ __device__ constexpr size_t getrf_smem(int cap, int pb) {
-  return sizeof(T) * ((size_t)cap * pb + 2 * pb * kT) + 32 * 8 + 32 * 4 + (4 * pb + 4) * 4;
+  return 2 * (NT / 32) * sizeof(PivotRec<T, kLeafW>) + sizeof(T) * (size_t)panel_ld(cap) * pb +
+         2 * sizeof(T) * (size_t)chunk_ld<T, NT>() * pb + (2 * pb + 4) * 4;
 }
 
-// NT: threads of the CTA; kPB: panel width (16 or 32, the autotuner's choice).
-template <typename T, int NT, int kPB>
-__device__ int cta_getrf(T* a, int n, int* ipiv, unsigned char* smem, int cap) {
-  const int kMaxN = cap;                                   // panel stride (rows)
-  T* panel = reinterpret_cast<T*>(smem);                   // cap x kPB, [col][row]
-  T* ut = panel + (size_t)cap * kPB;                       // kPB x kT (U12 tile), [col][row]
-  T* ct = ut + kPB * kT;                                   // staging (row labels)
-  double* red_k = reinterpret_cast<double*>(ct + kT * kPB);
-  int* red_i = reinterpret_cast<int*>(red_k + 32);
-  int* mv = red_i + 32;        // row moves of the panel: dst [2*kPB], src [2*kPB]
-  int* cnt = mv + 4 * kPB;
-  int* info_s = cnt + 1;
-  if (threadIdx.x == 0) *info_s = 0;
-  __syncthreads();
-  for (int k0 = 0; k0 < n; k0 += kPB) {
-    const int w = min(kPB, n - k0);
+__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// An entry copied asynchronously from global to shared memory.
+template <typename T>
+__device__ __forceinline__ void cp_async_entry(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "n"(sizeof(T))
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// A 32 x 16 tile at (r0, c0) of C (mt x cw) -= L U held by one warp: L[k][row]
+// (stride ldl) and U[k][col] (stride ldu) in shared memory, C global (leading
+// dimension n). K terms in increasing k, each one fused multiply-add.
+// Rows and columns past the edge read padding and are not stored.
+struct TileF64 {  // FP64 tensor cores; U is negated, so a load is not touched before its tile's turn
+  double acc[4][2][2];
+  __device__ __forceinline__ void load(const double* C, int n, int r0, int c0, int mt, int cw) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * j + 2 * t + e;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = r0 + 8 * i + g;
+          acc[i][j][e] = (c < cw && r < mt) ? C[c * n + r] : 0.0;
+        }
+      }
+  }
+  template <int K>
+  __device__ __forceinline__ void update(const double* L, int ldl, const double* U, int ldu, int r0, int c0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int k = 0; k < K; k += 4) {
+      double av[4], bv[2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) av[i] = L[(k + t) * ldl + r0 + 8 * i + g];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) bv[j] = -U[(k + t) * ldu + c0 + 8 * j + g];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
+    }
+  }
+  __device__ __forceinline__ void store(double* C, int n, int r0, int c0, int mt, int cw) const {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * j + 2 * t + e;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = r0 + 8 * i + g;
+          if (c < cw && r < mt) C[c * n + r] = acc[i][j][e];
+        }
+      }
+  }
+};
+struct TileF32 {  // CUDA cores; a lane has rows 4 rg .. 4 rg + 3 and columns 4 cg .. 4 cg + 3
+  float acc[4][4];
+  __device__ __forceinline__ void load(const float* C, int n, int r0, int c0, int mt, int cw) {
+    const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + 4 * cg + j;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 4 * rg + i;
+        acc[i][j] = (c < cw && r < mt) ? C[c * n + r] : 0.f;
+      }
+    }
+  }
+  template <int K>
+  __device__ __forceinline__ void update(const float* L, int ldl, const float* U, int ldu, int r0, int c0) {
+    const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) {
+      const float4 l = *reinterpret_cast<const float4*>(L + k * ldl + r0 + 4 * rg);
+      const float4 u = *reinterpret_cast<const float4*>(U + k * ldu + c0 + 4 * cg);
+      const float lv[4] = {l.x, l.y, l.z, l.w}, uv[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][j] = __fmaf_rn(-lv[i], uv[j], acc[i][j]);
+    }
+  }
+  __device__ __forceinline__ void store(float* C, int n, int r0, int c0, int mt, int cw) const {
+    const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + 4 * cg + j;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 4 * rg + i;
+        if (c < cw && r < mt) C[c * n + r] = acc[i][j];
+      }
+    }
+  }
+};
+
+// All tiles of C (mt x cw) -= L U, dealt to the CTA's NW warps; a warp loads
+// its next tile while it updates one (the loads' latency was most of the
+// update's time: n = 400, 670 us per system without).
+template <int K, int NW, typename T>
+__device__ __noinline__ void cta_update(const T* L, int ldl, const T* U, int ldu, T* C, int n, int mt, int cw) {
+  using Tile = std::conditional_t<sizeof(T) == 8, TileF64, TileF32>;
+  const int tr = (mt + 31) / 32, tiles = tr * ((cw + 15) / 16);
+  int cur = threadIdx.x >> 5;
+  if (cur >= tiles) return;
+  Tile t0, t1;
+  int r0 = 32 * (cur % tr), c0 = 16 * (cur / tr), r1 = 0, c1 = 0;
+  t0.load(C, n, r0, c0, mt, cw);
+  for (;;) {
+    if ((cur += NW) < tiles) {
+      r1 = 32 * (cur % tr), c1 = 16 * (cur / tr);
+      t1.load(C, n, r1, c1, mt, cw);
+    }
+    t0.template update<K>(L, ldl, U, ldu, r0, c0);
+    t0.store(C, n, r0, c0, mt, cw);
+    if (cur >= tiles) return;
+    if ((cur += NW) < tiles) {
+      r0 = 32 * (cur % tr), c0 = 16 * (cur / tr);
+      t0.load(C, n, r0, c0, mt, cw);
+    }
+    t1.template update<K>(L, ldl, U, ldu, r1, c1);
+    t1.store(C, n, r1, c1, mt, cw);
+    if (cur >= tiles) return;
+  }
+}
+
+// x <- L^{-1} x for 16 entries x[i] = xs[i * lds]; L unit lower, entry (i, k)
+// at l[k * ldl + i].
+template <typename T>
+__device__ __noinline__ void solve16(const T* l, int ldl, T* xs, int lds, int w) {
+  T x[kLeafW];
+#pragma unroll
+  for (int i = 0; i < kLeafW; ++i) x[i] = i < w ? xs[i * lds] : T(0);
+#pragma unroll
+  for (int k = 0; k < kLeafW - 1; ++k)
+#pragma unroll
+    for (int i = k + 1; i < kLeafW; ++i) x[i] = fma_t<T>(-l[k * ldl + i], x[k], x[i]);
+#pragma unroll
+  for (int i = 0; i < kLeafW; ++i)
+    if (i < w) xs[i * lds] = x[i];
+}
+
+// LU with partial pivoting of the n x n matrix a (global, leading dim n) in
+// place; ipiv (global, n ints): the sequential interchanges. rhs (may be null):
+// one more column of n entries, left as L^{-1} P rhs. perm (shared, may be
+// null): n ints, left as the row order. Returns 0 or 1 + the first column
+// with a zero pivot. NT threads, RPT rows each (n <= NT * RPT), panel PB.
+template <typename T, int NT, int RPT, int PB>
+__device__ int cta_getrf(T* a, int n, T* rhs, int* ipiv, int* perm, unsigned char* smem, int cap) {
+  using Rec = PivotRec<T, kLeafW>;
+  constexpr int NW = NT / 32;
+  constexpr int CH = chunk_cols<NT>();
+  constexpr int ldu = chunk_ld<T, NT>();
+  const int ldt = panel_ld(cap);
+  Rec(*rec)[NW] = reinterpret_cast<Rec(*)[NW]>(smem);
+  T* tile = reinterpret_cast<T*>(smem + 2 * NW * sizeof(Rec));  // [col][row]
+  T* us = tile + (size_t)PB * ldt;                              // [k][col], two buffers (16-byte aligned)
+  int* piv_slot = reinterpret_cast<int*>(us + 2 * PB * ldu);    // slot of each pivot row
+  int* disp = piv_slot + PB;  // where a top row that is no pivot went (-1: it is one)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int zero = INT_MAX;
+  if (perm != nullptr)
+    for (int i = tid; i < n; i += NT) perm[i] = i;
+  for (int k0 = 0; k0 < n; k0 += PB) {
+    const int w = min(PB, n - k0);
     const int m = n - k0;  // panel rows
     // ---- panel into shared memory --------------------------------------
-    for (int c = 0; c < w; ++c)
-      for (int r = threadIdx.x; r < m; r += blockDim.x) panel[c * kMaxN + r] = a[(size_t)(k0 + r) + (size_t)(k0 + c) * n];
-    // row labels for the interchanges of this panel
-    int* lab = reinterpret_cast<int*>(ct);  // m ints (ct is free during the panel)
-    for (int r = threadIdx.x; r < m; r += blockDim.x) lab[r] = r;
-    __syncthreads();
-    for (int j = 0; j < w; ++j) {
-      double key = -CUDART_INF;
-      int idx = INT_MAX;
-      for (int r = j + threadIdx.x; r < m; r += blockDim.x) {
-        const double kk = pkey((double)panel[j * kMaxN + r], r == j);
-        if (kk > key) { key = kk; idx = r; }
-      }
-      const int p = block_argmax(key, idx, red_k, red_i, j & 1);
-      const T d = panel[j * kMaxN + p];
-      if (threadIdx.x == 0) {
-        ipiv[k0 + j] = k0 + p;
-        if (fabs((double)d) <= 0.0 && *info_s == 0) *info_s = k0 + j + 1;
-      }
-      if (p != j) {
-        for (int c = threadIdx.x; c < w; c += blockDim.x) {
-          const T t = panel[c * kMaxN + j];
-          panel[c * kMaxN + j] = panel[c * kMaxN + p];
-          panel[c * kMaxN + p] = t;
-        }
-        if (threadIdx.x == 0) {
-          const int t = lab[j];
-          lab[j] = lab[p];
-          lab[p] = t;
-        }
-      }
-      __syncthreads();
-      // each row's multiplier and its rank-1 update by the same thread (the
-      // pivot row, read here, is not written in this phase: no barrier between)
-      for (int r = j + 1 + threadIdx.x; r < m; r += blockDim.x) {
-        const T l = panel[j * kMaxN + r] / d;
-        panel[j * kMaxN + r] = l;
-        for (int c = j + 1; c < w; ++c) panel[c * kMaxN + r] = fma_t<T>(-l, panel[c * kMaxN + j], panel[c * kMaxN + r]);
-      }
-      __syncthreads();
-    }
-    for (int c = 0; c < w; ++c)
-      for (int r = threadIdx.x; r < m; r += blockDim.x) a[(size_t)(k0 + r) + (size_t)(k0 + c) * n] = panel[c * kMaxN + r];
-    // ---- the panel's interchanges on the other columns: one gather ----------
-    if (threadIdx.x == 0) *cnt = 0;
-    __syncthreads();
-    for (int r = threadIdx.x; r < m; r += blockDim.x) {
-      if (lab[r] != r) {
-        const int s = atomicAdd(cnt, 1);
-        if (s < 2 * kPB) { mv[s] = r; mv[2 * kPB + s] = lab[r]; }
+    int pos[RPT];
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int r = tid + k * NT;
+      pos[k] = r < m ? r : -1;
+      if (r < m) {
+        const T* src = a + (size_t)(k0 + r) + (size_t)k0 * n;
+#pragma unroll 8
+        for (int c = 0; c < w; ++c) tile[c * ldt + r] = src[(size_t)c * n];
       }
     }
-    __syncthreads();
-    const int moves = min(*cnt, 2 * kPB);
-    // stage the moved rows 64 columns at a time in shared memory (ut and ct,
-    // contiguous, hold 2 * kPB * kT entries): all reads of a chunk, then all writes
-    T* stage = ut;
-    for (int cb = 0; cb < n; cb += kT) {
-      const int cw = min(kT, n - cb);
-      for (int e = threadIdx.x; e < moves * cw; e += blockDim.x) {
-        const int sidx = e / cw, c = cb + e % cw;
-        if (c < k0 || c >= k0 + w) stage[e] = a[(size_t)(k0 + mv[2 * kPB + sidx]) + (size_t)c * n];
-      }
+    if (tid < PB) disp[tid] = -1;
+    // ---- its leaves (each thread reads its own rows: no barrier needed) ------
+    for (int cl0 = 0; cl0 < w; cl0 += kLeafW) {
+      const int wl = min(kLeafW, w - cl0), tc = w - cl0 - wl;
+      const int z = cta_leaf<T, kLeafW, NT, RPT, false, false>(tile, ldt, m, cl0, wl, pos, rec, piv_slot, ipiv + k0);
+      if (z != INT_MAX && zero == INT_MAX) zero = k0 + z;
       __syncthreads();
-      for (int e = threadIdx.x; e < moves * cw; e += blockDim.x) {
-        const int sidx = e / cw, c = cb + e % cw;
-        if (c < k0 || c >= k0 + w) a[(size_t)(k0 + mv[sidx]) + (size_t)c * n] = stage[e];
-      }
-      __syncthreads();
-    }
-    const int kr = k0 + w;
-    if (kr < n) {
-      // ---- U12 = L11^{-1} A12, 64 columns at a time through shared memory ---
-      for (int cb = kr; cb < n; cb += kT) {
-        const int cw = min(kT, n - cb);
-        for (int e = threadIdx.x; e < w * cw; e += blockDim.x) {
-          const int i = e % w, c = e / w;
-          stage[c * kPB + i] = a[(size_t)(k0 + i) + (size_t)(cb + c) * n];
-        }
-        __syncthreads();
-        if (threadIdx.x < cw) {
-          T* x = stage + threadIdx.x * kPB;
-          for (int i = 1; i < w; ++i) {
-            T acc = x[i];
-            for (int kk = 0; kk < i; ++kk) acc = fma_t<T>(-panel[kk * kMaxN + i], x[kk], acc);
-            x[i] = acc;
+      if (tc > 0) {
+        if (tid < tc) {  // U of the leaf's pivot rows in the panel's other columns
+          T x[kLeafW];
+          T* tcol = tile + (cl0 + kLeafW + tid) * ldt;
+#pragma unroll
+          for (int i = 0; i < kLeafW; ++i) x[i] = tcol[piv_slot[cl0 + i]];
+#pragma unroll
+          for (int i = 1; i < kLeafW; ++i) {
+            const T* lrow = tile + cl0 * ldt + piv_slot[cl0 + i];
+#pragma unroll
+            for (int k = 0; k < i; ++k) x[i] = fma_t<T>(-lrow[k * ldt], x[k], x[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < kLeafW; ++i) {
+            us[tid * kLeafW + i] = x[i];
+            tcol[piv_slot[cl0 + i]] = x[i];
           }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < w * cw; e += blockDim.x) {
-          const int i = e % w, c = e / w;
-          a[(size_t)(k0 + i) + (size_t)(cb + c) * n] = stage[c * kPB + i];
-        }
-        __syncthreads();
-      }
-      // ---- A22 -= L21 U12 in 64 x 64 tiles ----------------------------------
-      const int mt = n - kr;
-      const int tiles = (mt + kT - 1) / kT;
-      for (int tj = 0; tj < tiles; ++tj) {
-        const int c0 = kr + tj * kT, cw = min(kT, n - c0);
-        for (int idx2 = threadIdx.x; idx2 < w * kT; idx2 += blockDim.x) {
-          const int kk = idx2 % kPB, c = idx2 / kPB;
-          if (kk < w) ut[c * kPB + kk] = c < cw ? a[(size_t)(k0 + kk) + (size_t)(c0 + c) * n] : T(0);
-        }
-        __syncthreads();
-        // register micro-tile per thread: kTR rows (tr + 16 i) x kTC columns
-        // (tc + kCG j) of the 64 x 64 tile; each entry's terms are still
-        // accumulated in increasing kk, one fused multiply-add each
-        constexpr int kRG = kT / kTR, kCG = NT / kRG, kTC = kT / kCG;
-        static_assert(kRG * kCG == NT && kCG * kTC == kT, "micro-tile covers the tile");
-        const int tr = threadIdx.x % kRG, tc = threadIdx.x / kRG;
-        for (int ti = 0; ti < tiles; ++ti) {
-          const int r0 = kr + ti * kT, rw = min(kT, n - r0);
-          T acc[kTR][kTC];
 #pragma unroll
-          for (int i = 0; i < kTR; ++i)
+        for (int k = 0; k < RPT; ++k)
+          if (pos[k] >= cl0 + kLeafW) {
+            T* trow = tile + tid + k * NT;
+            T l[kLeafW];
 #pragma unroll
-            for (int j = 0; j < kTC; ++j) {
-              const int r = tr + kRG * i, c = tc + kCG * j;
-              acc[i][j] = (r < rw && c < cw) ? a[(size_t)(r0 + r) + (size_t)(c0 + c) * n] : T(0);
+            for (int i = 0; i < kLeafW; ++i) l[i] = trow[(cl0 + i) * ldt];
+#pragma unroll 4
+            for (int c = 0; c < tc; ++c) {
+              T acc = trow[(cl0 + kLeafW + c) * ldt];
+              const T* uc = static_cast<const T*>(__builtin_assume_aligned(us + c * kLeafW, 16));
+#pragma unroll
+              for (int i = 0; i < kLeafW; ++i) acc = fma_t<T>(-l[i], uc[i], acc);
+              trow[(cl0 + kLeafW + c) * ldt] = acc;
             }
-          const T* lcol = panel + (r0 - k0);
-          for (int kk = 0; kk < w; ++kk) {
-            T l[kTR], u[kTC];
-#pragma unroll
-            for (int i = 0; i < kTR; ++i) {
-              const int r = tr + kRG * i;
-              l[i] = r < rw ? lcol[kk * kMaxN + r] : T(0);
-            }
-#pragma unroll
-            for (int j = 0; j < kTC; ++j) u[j] = ut[(tc + kCG * j) * kPB + kk];
-#pragma unroll
-            for (int i = 0; i < kTR; ++i)
-#pragma unroll
-              for (int j = 0; j < kTC; ++j) acc[i][j] = fma_t<T>(-l[i], u[j], acc[i][j]);
           }
-#pragma unroll
-          for (int i = 0; i < kTR; ++i)
-#pragma unroll
-            for (int j = 0; j < kTC; ++j) {
-              const int r = tr + kRG * i, c = tc + kCG * j;
-              if (r < rw && c < cw) a[(size_t)(r0 + r) + (size_t)(c0 + c) * n] = acc[i][j];
-            }
-        }
-        __syncthreads();
       }
     }
-    __syncthreads();
+    // ---- rows into position order: pivots first, displaced top rows last ----
+#pragma unroll
+    for (int k = 0; k < RPT; ++k)
+      if (tid + k * NT < w && pos[k] >= w) disp[tid + k * NT] = pos[k];
+    const bool moved = __syncthreads_or(tid < w && piv_slot[tid] != tid);
+    if (moved) {
+      constexpr int kIt = (PB * PB + NT - 1) / NT;
+      T pv[kIt], dv[kIt];
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < w) {
+          pv[it] = tile[c * ldt + piv_slot[i]];
+          dv[it] = tile[c * ldt + i];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < w) {
+          tile[c * ldt + i] = pv[it];
+          if (disp[i] >= 0) tile[c * ldt + disp[i]] = dv[it];
+        }
+      }
+      // the same interchanges on the columns left of the panel, a warp each
+      for (int c = warp; c < k0 + (perm != nullptr ? 1 : 0); c += NW) {
+        if (c < k0) {
+          T* cp = a + (size_t)c * n + k0;
+          T p0 = T(0), d0 = T(0);
+          if (lane < w) {
+            p0 = cp[piv_slot[lane]];
+            d0 = cp[lane];
+          }
+          __syncwarp();
+          if (lane < w) {
+            cp[lane] = p0;
+            if (disp[lane] >= 0) cp[disp[lane]] = d0;
+          }
+        } else {
+          int p0 = 0, d0 = 0;
+          if (lane < w) {
+            p0 = perm[k0 + piv_slot[lane]];
+            d0 = perm[k0 + lane];
+          }
+          __syncwarp();
+          if (lane < w) {
+            perm[k0 + lane] = p0;
+            if (disp[lane] >= 0) perm[k0 + disp[lane]] = d0;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    // sequential interchanges from positions within the panel to rows
+    if (tid < w) ipiv[k0 + tid] += k0;
+    for (int r = tid; r < m; r += NT) {
+      T* dst = a + (size_t)(k0 + r) + (size_t)k0 * n;
+#pragma unroll 8
+      for (int c = 0; c < w; ++c) dst[(size_t)c * n] = tile[c * ldt + r];
+    }
+    // ---- the columns right of the panel (and the right-hand side) -----------
+    const int kr = k0 + w, mt = n - kr;
+    const int nright = mt + (rhs != nullptr ? 1 : 0);
+    // (a chunk's rows of U12, in pivot order, are fetched while the chunk
+    // before it is updated)
+    auto fetch = [&](int cb, T* u) {
+      const int cw = min(CH, nright - cb);
+#pragma unroll
+      for (int it = 0; it < PB * CH / NT; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < cw)
+          cp_async_entry(u + i * ldu + c, (cb + c < mt ? a + (size_t)(kr + cb + c) * n : rhs) + k0 + piv_slot[i]);
+      }
+      cp_async_commit();
+    };
+    if (nright > 0) fetch(0, us);
+    for (int cb = 0, buf = 0; cb < nright; cb += CH, buf ^= 1) {
+      T* u = us + buf * PB * ldu;
+      const int cw = min(CH, nright - cb);
+      auto col = [&](int c) { return cb + c < mt ? a + (size_t)(kr + cb + c) * n : rhs; };
+      constexpr int kIt = PB * CH / NT;
+      T dv[kIt];
+      if (moved) {
+#pragma unroll
+        for (int it = 0; it < kIt; ++it) {
+          const int e = tid + it * NT, i = e % PB, c = e / PB;
+          if (i < w && c < cw) dv[it] = col(c)[k0 + i];
+        }
+      }
+      cp_async_wait_all();
+      __syncthreads();
+      if (cb + CH < nright) fetch(cb + CH, us + (buf ^ 1) * PB * ldu);
+      if (moved) {
+#pragma unroll
+        for (int it = 0; it < kIt; ++it) {
+          const int e = tid + it * NT, i = e % PB, c = e / PB;
+          if (i < w && c < cw && disp[i] >= 0) col(c)[k0 + disp[i]] = dv[it];
+        }
+      }
+      if (tid < cw) solve16(tile, ldt, u + tid, ldu, min(w, kLeafW));
+      __syncthreads();
+      if (PB > kLeafW && w > kLeafW) {
+        for (int e = tid; e < kLeafW * cw; e += NT) {
+          const int i = kLeafW + e % kLeafW, c = e / kLeafW;
+          if (i < w) {
+            T acc = u[i * ldu + c];
+#pragma unroll
+            for (int k = 0; k < kLeafW; ++k) acc = fma_t<T>(-tile[k * ldt + i], u[k * ldu + c], acc);
+            u[i * ldu + c] = acc;
+          }
+        }
+        __syncthreads();
+        if (tid < cw) solve16(tile + kLeafW * ldt + kLeafW, ldt, u + kLeafW * ldu + tid, ldu, w - kLeafW);
+        __syncthreads();
+      }
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < cw) col(c)[k0 + i] = u[i * ldu + c];
+      }
+      if (mt > 0) {  // (then w == PB)
+        const int cm = min(cw, mt - cb);  // the chunk's matrix columns
+        cta_update<PB, NW>(tile + PB, ldt, u, ldu, a + (size_t)(kr + cb) * n + kr, n, mt, cm);
+        if (cm < cw)  // and the right-hand side
+          for (int r = tid; r < mt; r += NT) {
+            T acc = rhs[kr + r];
+#pragma unroll
+            for (int k = 0; k < PB; ++k) acc = fma_t<T>(-tile[k * ldt + PB + r], u[k * ldu + cm], acc);
+            rhs[kr + r] = acc;
+          }
+      }
+      __syncthreads();
+    }
   }
-  const int info = *info_s;
   __syncthreads();
-  return info;
+  return zero == INT_MAX ? 0 : zero + 1;
 }
 
-// x <- (LU)^{-1} P x for one vector (global), LU n x n in global, x staged in shared memory.
-template <typename T, typename V>
-__device__ void cta_getrs(const T* lu, int n, const int* ipiv, V* x, V* xs) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = x[i];
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < n; ++k) {
-      const int p = ipiv[k];
-      if (p != k) { const V t = xs[k]; xs[k] = xs[p]; xs[p] = t; }
+constexpr int kSB = 32;  // rows of a block of the triangular sweeps
+
+// xs (shared, n) <- U^{-1} xs, or with UNIT_LOWER L^{-1} xs, for the factors
+// lu (global, n x n). By blocks of 32 rows: one warp solves the diagonal
+// block (its rows in registers, one shuffle per step; quotients correctly
+// rounded from reciprocals formed beforehand), then every thread subtracts
+// the block's 32 terms from a row of the rest, its 32 loads in flight at once.
+template <bool UNIT_LOWER, typename T, int NT>
+__device__ __noinline__ void cta_sweep(const T* lu, int n, double* xs) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int nb = (n + kSB - 1) / kSB;
+  for (int b = 0; b < nb; ++b) {
+    const int k0 = (UNIT_LOWER ? b : nb - 1 - b) * kSB, w = min(kSB, n - k0);
+    const T* blk = lu + (size_t)k0 * n;  // the block's columns
+    if (tid < 32) {
+      double u[kSB];
+#pragma unroll
+      for (int j = 0; j < kSB; ++j) u[j] = (lane < w && j < w) ? (double)blk[(size_t)(k0 + lane) + (size_t)j * n] : 0.0;
+      double x = lane < w ? xs[k0 + lane] : 0.0;
+      if (UNIT_LOWER) {
+#pragma unroll
+        for (int j = 0; j < kSB; ++j) {
+          const double xj = __shfl_sync(0xffffffffu, x, j);
+          if (lane > j) x = __fma_rn(-u[j], xj, x);
+        }
+      } else {
+        double d = 1.0;
+#pragma unroll
+        for (int j = 0; j < kSB; ++j)
+          if (lane == j && j < w) d = u[j];
+        const bool fast = exp_fast_ok(d);
+        const double y = fast ? rcp_rn(d) : 1.0;
+#pragma unroll
+        for (int j = kSB - 1; j >= 0; --j) {
+          if (lane == j) x = quotient<double>(x, d, y, fast);
+          const double xj = __shfl_sync(0xffffffffu, x, j);
+          if (lane < j) x = __fma_rn(-u[j], xj, x);
+        }
+      }
+      if (lane < w) xs[k0 + lane] = x;
     }
-  __syncthreads();
-  // forward (unit lower), column sweep
-  for (int j = 0; j < n; ++j) {
-    const V xj = xs[j];
-    for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) xs[i] -= (V)lu[(size_t)i + (size_t)j * n] * xj;
+    __syncthreads();
+    const int r0 = UNIT_LOWER ? k0 + w : 0, r1 = UNIT_LOWER ? n : k0;
+    for (int i = r0 + tid; i < r1; i += NT) {
+      const T* row = blk + i;
+      double acc = xs[i];
+      if (w == kSB) {
+        T v[kSB];
+#pragma unroll
+        for (int j = 0; j < kSB; ++j) v[j] = row[(size_t)j * n];
+#pragma unroll
+        for (int j = 0; j < kSB; ++j) acc = __fma_rn(-(double)v[j], xs[k0 + j], acc);
+      } else {
+        for (int j = 0; j < w; ++j) acc = __fma_rn(-(double)row[(size_t)j * n], xs[k0 + j], acc);
+      }
+      xs[i] = acc;
+    }
     __syncthreads();
   }
-  // backward (upper), column sweep
-  for (int j = n - 1; j >= 0; --j) {
-    if (threadIdx.x == 0) xs[j] = xs[j] / (V)lu[(size_t)j + (size_t)j * n];
-    __syncthreads();
-    const V xj = xs[j];
-    for (int i = threadIdx.x; i < j; i += blockDim.x) xs[i] -= (V)lu[(size_t)i + (size_t)j * n] * xj;
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = xs[i];
+}
+
+// xs (shared) <- (LU)^{-1} P x for one vector x (global).
+template <typename T, int NT>
+__device__ void cta_getrs(const T* lu, int n, const int* perm, const double* x, double* xs) {
+  for (int i = threadIdx.x; i < n; i += NT) xs[i] = x[perm[i]];
   __syncthreads();
+  cta_sweep<true, T, NT>(lu, n, xs);
+  cta_sweep<false, T, NT>(lu, n, xs);
 }
 
 // Normwise backward error of x for A x = b (FP64, A n x n in global).
-__device__ double cta_backward_error(const double* a, int n, const double* x, const double* b, double* rs,
+__device__ __noinline__ double cta_backward_error(const double* a, int n, const double* x, const double* b, double* rs,
                                      double* red) {
   double rmax = 0.0, amax = 0.0, xmax = 0.0, bmax = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     double s = 0.0, ra = 0.0;
+#pragma unroll 16
     for (int j = 0; j < n; ++j) {
       const double aij = a[(size_t)i + (size_t)j * n];
       s = __fma_rn(aij, x[j], s);
@@ -344,13 +576,20 @@ struct BatchArgs {
   double tol_scale;        // tol = tol_scale * n * 2^-53
 };
 
-template <int NT, int PB>
-__global__ void __launch_bounds__(NT) batched_gesv_kernel(BatchArgs p) {
+// RPT rows per thread: systems of up to NT * RPT rows. Bound by the column
+// chain (latency) and, for the largest orders, by the trailing matrix's
+// passes through L2 and HBM (n^3 / PB bytes of it per system and direction);
+// 20 000 systems of order 8..512, FP64: 81 ms before (panel columns with three
+// barriers each in shared memory, the update on the CUDA cores, sweeps of two
+// barriers a column), 29 ms now; 3 000 in the mixed form 11.1 and 6.0 ms.
+template <int NT, int RPT, int PB>
+__global__ void __launch_bounds__(NT, RPT == 4 ? 2 : 512 / NT) batched_gesv_kernel(BatchArgs p) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int next;
   __shared__ double red[4 * (NT / 32)];
-  double* vs = reinterpret_cast<double*>(smem);   // cap doubles for vectors
-  unsigned char* lus = smem + sizeof(double) * p.cap;
+  double* vs = reinterpret_cast<double*>(smem);  // cap doubles for vectors
+  int* perm = reinterpret_cast<int*>(vs + p.cap);  // cap ints: the row order (mixed form)
+  unsigned char* lus = reinterpret_cast<unsigned char*>(perm + ((p.cap + 3) & ~3));
   for (;;) {
     if (threadIdx.x == 0) next = atomicAdd(p.queue, 1);
     __syncthreads();
@@ -363,36 +602,53 @@ __global__ void __launch_bounds__(NT) batched_gesv_kernel(BatchArgs p) {
     double* b = p.b + p.b_off[s];
     int* ipiv = p.ipiv + p.b_off[s];
     if (!p.mixed) {
-      const int info = cta_getrf<double, NT, PB>(a, n, ipiv, lus, p.cap);
+      double* y = p.work + p.b_off[s];  // b stays as it is when the system is singular
+      for (int i = threadIdx.x; i < n; i += NT) y[i] = b[i];
+      __syncthreads();
+      const int info = cta_getrf<double, NT, RPT, PB>(a, n, y, ipiv, nullptr, lus, p.cap);
       if (threadIdx.x == 0) p.info[s] = info;
-      if (info == 0) cta_getrs<double, double>(a, n, ipiv, b, vs);
+      if (info == 0) {  // y = L^{-1} P b
+        for (int i = threadIdx.x; i < n; i += NT) vs[i] = y[i];
+        __syncthreads();
+        cta_sweep<false, double, NT>(a, n, vs);
+        for (int i = threadIdx.x; i < n; i += NT) b[i] = vs[i];
+      }
       continue;
     }
     // ---- mixed: FP32 LU, FP64 refinement against the FP64 matrix ------------
     float* a32 = p.a32 + p.a_off[s];
-    for (size_t e = threadIdx.x; e < (size_t)n * n; e += NT) a32[e] = __double2float_rn(a[e]);
+    {
+      const size_t nn = (size_t)n * n;
+      size_t e = threadIdx.x;
+      for (; e + 7 * NT < nn; e += 8 * NT) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = a[e + u * NT];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a32[e + u * NT] = __double2float_rn(v[u]);
+      }
+      for (; e < nn; e += NT) a32[e] = __double2float_rn(a[e]);
+    }
     __syncthreads();
-    const int info = cta_getrf<float, NT, PB>(a32, n, ipiv, lus, p.cap);
+    const int info = cta_getrf<float, NT, RPT, PB>(a32, n, nullptr, ipiv, perm, lus, p.cap);
     if (info != 0) {
       if (threadIdx.x == 0) p.info[s] = info;
       continue;
     }
-    double* x = p.work + p.b_off[s];               // correction / residual (global)
+    double* res = p.work + p.b_off[s];             // residual (global)
     double* sol = vs;                              // solution (shared)
     double* r = reinterpret_cast<double*>(lus);    // solve staging (the panel area is free now)
-    for (int i = threadIdx.x; i < n; i += NT) x[i] = b[i];
-    __syncthreads();
-    cta_getrs<float, double>(a32, n, ipiv, x, r);
-    for (int i = threadIdx.x; i < n; i += NT) sol[i] = x[i];
+    cta_getrs<float, NT>(a32, n, perm, b, r);
+    for (int i = threadIdx.x; i < n; i += NT) sol[i] = r[i];
     __syncthreads();
     const double tol = p.tol_scale * n * 0x1p-53;
     int it = 0;
     double e = 0.0;
     for (;;) {
-      e = cta_backward_error(a, n, sol, b, x, red);  // also x = b - A sol
+      e = cta_backward_error(a, n, sol, b, res, red);  // also res = b - A sol
       if (e <= tol || it >= p.max_ir || !(e == e)) break;
-      cta_getrs<float, double>(a32, n, ipiv, x, r);
-      for (int i = threadIdx.x; i < n; i += NT) sol[i] += x[i];
+      cta_getrs<float, NT>(a32, n, perm, res, r);
+      for (int i = threadIdx.x; i < n; i += NT) sol[i] += r[i];
       __syncthreads();
       ++it;
     }
@@ -405,34 +661,63 @@ __global__ void __launch_bounds__(NT) batched_gesv_kernel(BatchArgs p) {
   }
 }
 
-size_t kernel_smem(int cap, bool mixed, int pb) {
-  const size_t g = mixed ? getrf_smem<float>(cap, pb) : getrf_smem<double>(cap, pb);
-  return sizeof(double) * (size_t)cap + std::max(g, sizeof(double) * (size_t)cap) + 64;
+// Every launch shape: NT threads, the rows per thread that cover the bucket's
+// cap, the panel width.
+using BatchKernel = void (*)(BatchArgs);
+template <int NT, int PB>
+BatchKernel batch_kernel_rpt(int cap) {
+  if (cap <= NT) return batched_gesv_kernel<NT, 1, PB>;
+  if constexpr (2 * NT <= kMaxN)
+    if (cap <= 2 * NT) return batched_gesv_kernel<NT, 2, PB>;
+  if constexpr (4 * NT <= kMaxN) return batched_gesv_kernel<NT, 4, PB>;
+  return nullptr;
 }
-// one limit for every bucket sharing an instantiation: the largest any asks for
-size_t kernel_smem_max() {
-  return std::max(kernel_smem(kMaxN, false, 32), kernel_smem(kMaxN, true, 32));
+BatchKernel batch_kernel(int cap, int threads, int panel) {
+  const bool narrow = panel == 16;
+  switch (threads) {
+    case 128: return narrow ? batch_kernel_rpt<128, 16>(cap) : batch_kernel_rpt<128, 32>(cap);
+    case 512: return narrow ? batch_kernel_rpt<512, 16>(cap) : batch_kernel_rpt<512, 32>(cap);
+    default: return narrow ? batch_kernel_rpt<256, 16>(cap) : batch_kernel_rpt<256, 32>(cap);
+  }
 }
 
-// Host-side configuration (not stream work, so never inside a graph capture).
-template <int NT, int PB>
-int configure_bucket(alg_ctx* ctx, int cap, bool mixed, int count, int* grid) {
-  const size_t smem = kernel_smem(cap, mixed, PB);
-  ALG_CUDA_TRY(cudaFuncSetAttribute(batched_gesv_kernel<NT, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kernel_smem_max()));
-  int per_sm = 0;
-  ALG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_gesv_kernel<NT, PB>, NT, smem));
-  *grid = std::max(1, std::min(std::max(1, per_sm) * ctx->sm_count, count));
-  return ALG_OK;
+// The launch shape of a bucket when no autotuner chose one. With more systems
+// than SMs throughput counts: small CTAs, several to an SM, so that one
+// system's column chain runs beside another's update (1 500 systems of order
+// 257..512 in FP64: 128 x 16 11.2 ms, 256 x 16 11.9 ms, 512 x 32 11.8 ms; 3 000
+// of 129..256: 256 x 16 4.3 ms, 128 x 16 4.6 ms, 256 x 32 4.9 ms; 4 000 of
+// 65..128: 128 x 16 1.2 ms, 128 x 32 1.5 ms). The mixed form's longest systems
+// prefer the wide panel (128 x 32 12.0 ms, 128 x 16 12.8 ms). A few systems
+// run one to an SM: a thread per row and the wide panel's fewer sweeps.
+void default_batch_shape(int cap, bool mixed, bool few, int* threads, int* panel) {
+  if (few) {
+    *threads = std::max(128, std::min(512, cap));
+    *panel = 32;
+  } else {
+    *threads = cap == 256 && !mixed ? 256 : 128;
+    *panel = mixed && cap >= 512 ? 32 : 16;
+  }
 }
 
-template <int NT, int PB>
-int launch_bucket(alg_ctx* ctx, const BatchArgs& p, int grid) {
-  const size_t smem = kernel_smem(p.cap, p.mixed != 0, PB);
-  batched_gesv_kernel<NT, PB><<<grid, NT, smem, ctx->stream>>>(p);
-  count_launches();
-  ALG_CUDA_TRY(cudaGetLastError());
-  return ALG_OK;
+template <int NT>
+size_t kernel_smem_nt(int cap, bool mixed, int pb) {
+  const size_t g = mixed ? getrf_smem<float, NT>(cap, pb) : getrf_smem<double, NT>(cap, pb);
+  return sizeof(double) * (size_t)cap + sizeof(int) * (size_t)((cap + 3) & ~3) +
+         std::max(g, sizeof(double) * (size_t)cap) + 64;
+}
+size_t kernel_smem(int cap, bool mixed, int threads, int pb) {
+  switch (threads) {
+    case 128: return kernel_smem_nt<128>(cap, mixed, pb);
+    case 512: return kernel_smem_nt<512>(cap, mixed, pb);
+    default: return kernel_smem_nt<256>(cap, mixed, pb);
+  }
+}
+
+// Lifts a kernel's shared-memory limit: one limit for every bucket sharing an
+// instantiation, the largest any asks for.
+cudaError_t allow_smem(BatchKernel k, int threads, int pb) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)std::max(kernel_smem(kMaxN, false, threads, pb), kernel_smem(kMaxN, true, threads, pb)));
 }
 
 }  // namespace
@@ -457,29 +742,24 @@ int batch_launch_bucket(alg_ctx* ctx, const BatchSpec& sp, const BucketLaunch& b
   p.max_ir = sp.max_ir > 0 ? sp.max_ir : 10;
   p.tol_scale = sp.tol_scale > 0 ? sp.tol_scale : 10.0;
   ALG_CUDA_TRY(cudaMemsetAsync(bl.d_queue, 0, sizeof(int), ctx->stream));
-  const bool narrow = bl.panel == 16;
-  switch (bl.threads) {
-    case 128: return narrow ? launch_bucket<128, 16>(ctx, p, bl.grid) : launch_bucket<128, 32>(ctx, p, bl.grid);
-    case 512: return narrow ? launch_bucket<512, 16>(ctx, p, bl.grid) : launch_bucket<512, 32>(ctx, p, bl.grid);
-    default: return narrow ? launch_bucket<256, 16>(ctx, p, bl.grid) : launch_bucket<256, 32>(ctx, p, bl.grid);
-  }
+  const BatchKernel k = batch_kernel(bl.cap, bl.threads, bl.panel);
+  k<<<bl.grid, bl.threads, kernel_smem(bl.cap, sp.mixed != 0, bl.threads, bl.panel), ctx->stream>>>(p);
+  count_launches();
+  ALG_CUDA_TRY(cudaGetLastError());
+  return ALG_OK;
 }
 
+// Host-side configuration (not stream work, so never inside a graph capture).
 int batch_configure_bucket(alg_ctx* ctx, bool mixed, BucketLaunch* bl) {
   if (bl->panel != 16) bl->panel = 32;
-  const bool narrow = bl->panel == 16;
-  switch (bl->threads) {
-    case 128:
-      return narrow ? configure_bucket<128, 16>(ctx, bl->cap, mixed, bl->count, &bl->grid)
-                    : configure_bucket<128, 32>(ctx, bl->cap, mixed, bl->count, &bl->grid);
-    case 512:
-      return narrow ? configure_bucket<512, 16>(ctx, bl->cap, mixed, bl->count, &bl->grid)
-                    : configure_bucket<512, 32>(ctx, bl->cap, mixed, bl->count, &bl->grid);
-    default:
-      bl->threads = 256;
-      return narrow ? configure_bucket<256, 16>(ctx, bl->cap, mixed, bl->count, &bl->grid)
-                    : configure_bucket<256, 32>(ctx, bl->cap, mixed, bl->count, &bl->grid);
-  }
+  if (bl->threads != 128 && bl->threads != 512) bl->threads = 256;
+  const BatchKernel k = batch_kernel(bl->cap, bl->threads, bl->panel);
+  ALG_CUDA_TRY(allow_smem(k, bl->threads, bl->panel));
+  int per_sm = 0;
+  ALG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bl->threads,
+                                                             kernel_smem(bl->cap, mixed, bl->threads, bl->panel)));
+  bl->grid = std::max(1, std::min(std::max(1, per_sm) * ctx->sm_count, bl->count));
+  return ALG_OK;
 }
 
 int batch_max_order() { return kMaxN; }
@@ -605,7 +885,7 @@ int alg_batch_create(alg_ctx* ctx, int count, const int* n_host, int mixed, alg_
       alg::BucketLaunch bl;
       bl.count = end - pos;
       bl.cap = kBucketCaps[bi];
-      bl.threads = kBucketCaps[bi] >= 256 ? 512 : (kBucketCaps[bi] >= 64 ? 256 : 128);
+      alg::default_batch_shape(bl.cap, b->mixed != 0, bl.count <= ctx->sm_count, &bl.threads, &bl.panel);
       bl.d_order = b->d_order + pos;
       bl.d_queue = b->d_queues + qi++;
       const int rc = alg::batch_configure_bucket(ctx, b->mixed != 0, &bl);
@@ -675,9 +955,8 @@ int alg_batch_solve_graph(alg_batch* b, double* d_a, double* d_b, int* d_info) {
 
 // Tries every launch shape for each bucket on the given batch (which it
 // solves several times: pass scratch copies) and keeps the fastest: 128 / 256
-// / 512 threads per CTA (with the trailing update's micro-tile 4 x 8, 4 x 4
-// or 4 x 2 per thread) times a 16- or 32-column panel (the split between the
-// column-serial panel and the register-tiled update).
+// / 512 threads per CTA times a 16- or 32-column panel (the split between the
+// column-serial panel and the tiled update).
 int alg_batch_autotune(alg_batch* b, double* d_a, double* d_b, int* d_info, const double* d_a_src,
                        const double* d_b_src, int* threads_out) {
   if (b == nullptr) return ALG_INVALID_ARGUMENT;
@@ -897,25 +1176,15 @@ int noalloc_setup(int dev, unsigned char** out) {
     ALG_TRY(current_context_id(&id));
     cudaFuncAttributes fa;
     ALG_CUDA_TRY(cudaFuncGetAttributes(&fa, noalloc_header_kernel));
-    const int smem_max = (int)kernel_smem_max();
-    ALG_CUDA_TRY(cudaFuncSetAttribute(batched_gesv_kernel<128, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem_max));
-    ALG_CUDA_TRY(cudaFuncSetAttribute(batched_gesv_kernel<256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem_max));
-    ALG_CUDA_TRY(cudaFuncSetAttribute(batched_gesv_kernel<512, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem_max));
+    for (int cap = 32; cap <= kNoAllocMaxN; cap *= 2) {
+      int threads, panel;
+      default_batch_shape(cap, true, true, &threads, &panel);
+      ALG_CUDA_TRY(allow_smem(batch_kernel(cap, threads, panel), threads, panel));
+    }
     g_noalloc_ptr[dev] = p;
     g_noalloc_ctx[dev] = id;
   }
   *out = static_cast<unsigned char*>(g_noalloc_ptr[dev]);
-  return ALG_OK;
-}
-
-template <int NT>
-int noalloc_launch(cudaStream_t s, const BatchArgs& p) {
-  batched_gesv_kernel<NT, 32><<<1, NT, kernel_smem(p.cap, true, 32), s>>>(p);
-  count_launches();
-  ALG_CUDA_TRY(cudaGetLastError());
   return ALG_OK;
 }
 
@@ -948,7 +1217,8 @@ extern "C" int alg_dgesv_mixed_noalloc(void* stream, const double* d_a, double* 
   // the size bucket and CTA size a one-system plan of this order uses
   int cap = 32;
   while (cap < n) cap *= 2;
-  const int threads = cap >= 256 ? 512 : (cap >= 64 ? 256 : 128);
+  int threads, panel;
+  default_batch_shape(cap, true, true, &threads, &panel);
   BatchArgs p;
   p.count = 1;
   p.order = &hdr->order;
@@ -970,9 +1240,8 @@ extern "C" int alg_dgesv_mixed_noalloc(void* stream, const double* d_a, double* 
   noalloc_header_kernel<<<1, 1, 0, s>>>(hdr, n);
   count_launches();
   ALG_CUDA_TRY(cudaGetLastError());
-  switch (threads) {
-    case 128: return noalloc_launch<128>(s, p);
-    case 512: return noalloc_launch<512>(s, p);
-    default: return noalloc_launch<256>(s, p);
-  }
+  batch_kernel(cap, threads, panel)<<<1, threads, kernel_smem(cap, true, threads, panel), s>>>(p);
+  count_launches();
+  ALG_CUDA_TRY(cudaGetLastError());
+  return ALG_OK;
 }

@@ -15,9 +15,8 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
-#include <type_traits>
-
 #include "common.cuh"
+#include "pivot.cuh"
 
 namespace alg {
 namespace cg = cooperative_groups;
@@ -189,33 +188,6 @@ __device__ __forceinline__ T rec_entry(const unsigned long long* words, int c) {
     const unsigned long long wv = words[c >> 1];
     return static_cast<T>(__uint_as_float((unsigned)(c & 1 ? (wv >> 32) : wv)));
   }
-}
-
-template <typename T>
-__device__ __forceinline__ bool div_fast_ok(T x) {
-  const double ax = fabs(static_cast<double>(x));
-  if constexpr (sizeof(T) == 8) {
-    return ax >= 0x1p-500 && ax <= 0x1p500;
-  } else {
-    return ax >= 0x1p-60f && ax <= 0x1p60f;
-  }
-}
-__device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
-__device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-
-// a / d correctly rounded; y = RN(1/d), fast = d passed div_fast_ok.
-template <typename T>
-__device__ __forceinline__ T quotient(T a, T d, T y, bool fast) {
-  if (fast && div_fast_ok(a)) {
-    const T q = mul_rn(a, y);
-    const T r = fma_rn(-q, d, a);
-    return fma_rn(r, y, q);
-  }
-  return div_rn(a, d);
 }
 
 template <typename T, int W, bool EXACT>
@@ -533,69 +505,6 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(PanelAr
 // values take the plain IEEE division instead.
 // ---------------------------------------------------------------------------
 
-// A pivot candidate: |v|'s bits as an ordered integer and the row's position;
-// (0, INT_MAX) is no candidate (a zero entry is (0, its position), which wins
-// over it). The reference's NaN rule (mod.rs:123-134): +inf on the diagonal,
-// never chosen elsewhere.
-__device__ __forceinline__ void pivot_candidate(double v, int pos, int J, unsigned long long& key, int& kpos) {
-  key = pos >= J ? (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull : 0ull;
-  kpos = pos >= J ? pos : INT_MAX;
-  if (v != v) {
-    key = pos == J ? 0x7ff0000000000000ull : 0ull;
-    kpos = pos == J ? J : INT_MAX;
-  }
-}
-__device__ __forceinline__ void pivot_candidate(float v, int pos, int J, unsigned& key, int& kpos) {
-  key = pos >= J ? __float_as_uint(v) & 0x7fffffffu : 0u;
-  kpos = pos >= J ? pos : INT_MAX;
-  if (v != v) {
-    key = pos == J ? 0x7f800000u : 0u;
-    kpos = pos == J ? J : INT_MAX;
-  }
-}
-// Warp-wide: the largest key, and among its lanes the smallest tag; true on
-// the lanes that hold both.
-__device__ __forceinline__ bool warp_pivot(unsigned long long key, int tag, unsigned long long& mk, int& mt) {
-  const unsigned hi = (unsigned)(key >> 32);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)key : 0u);
-  const bool eq = hi == mh && (unsigned)key == ml;
-  mt = __reduce_min_sync(0xffffffffu, eq ? tag : INT_MAX);
-  mk = ((unsigned long long)mh << 32) | ml;
-  return eq && tag == mt;
-}
-__device__ __forceinline__ bool warp_pivot(unsigned key, int tag, unsigned& mk, int& mt) {
-  mk = __reduce_max_sync(0xffffffffu, key);
-  const bool eq = key == mk;
-  mt = __reduce_min_sync(0xffffffffu, eq ? tag : INT_MAX);
-  return eq && tag == mt;
-}
-// The same over the records rec[0 .. count) (one lane each): the winner's
-// index; its position in mp. Positions are below 2^20 (longer panels take
-// another kernel), so position and index share one reduction.
-template <typename Rec>
-__device__ __forceinline__ int warp_pick(const Rec* rec, int count, int lane, int& mp) {
-  typename Rec::Key k = 0, mk;
-  int t = INT_MAX, mt;
-  if (lane < count) {
-    const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(&rec[lane]);  // key; position and slot
-    k = (typename Rec::Key)h.x;
-    const unsigned pos = (unsigned)h.y;
-    t = pos < (1u << 20) ? (int)(pos << 5 | (unsigned)lane) : INT_MAX - 31 + lane;
-  }
-  warp_pivot(k, t, mk, mt);
-  mp = mt >> 5;
-  return mt & 31;
-}
-// div_fast_ok on the exponent bits (also false for zero, infinity and NaN)
-__device__ __forceinline__ bool exp_fast_ok(double v) {
-  const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
-  return e - (1023u - 500u) < 1000u;  // [2^-500, 2^500)
-}
-__device__ __forceinline__ bool exp_fast_ok(float v) {
-  const unsigned e = (__float_as_uint(v) >> 23) & 0xffu;
-  return e - (127u - 60u) < 120u;  // [2^-60, 2^60)
-}
 __device__ __forceinline__ void st_async_v2(uint32_t remote, ulonglong2 v, uint32_t remote_bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];"
                :: "r"(remote), "l"(v.x), "l"(v.y), "r"(remote_bar) : "memory");
@@ -606,18 +515,6 @@ __device__ __forceinline__ void ld_cluster(double& v, uint32_t a) {
 __device__ __forceinline__ void ld_cluster(float& v, uint32_t a) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
 }
-
-// A pivot record, in 16-byte chunks: (key; position and the row's slot in its
-// CTA), (reciprocal, unused), then the leaf's row, rotated as in registers.
-template <typename T, int W>
-struct alignas(16) PivotRec {
-  using Key = std::conditional_t<sizeof(T) == 8, unsigned long long, unsigned>;
-  unsigned long long key;
-  unsigned pos, slot;
-  T recip;
-  alignas(16) T row[W];
-  static constexpr int kChunks = 2 + W * (int)sizeof(T) / 16;
-};
 
 constexpr int kBlockMaxW = 64;  // columns of a block that one launch factors
 

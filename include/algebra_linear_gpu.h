@@ -298,8 +298,8 @@ int alg_batch_solve(alg_batch* batch, double* d_a, double* d_b, int* d_info);
 int alg_batch_solve_graph(alg_batch* batch, double* d_a, double* d_b, int* d_info);
 /* Autotuner: for every size bucket, times each launch shape on this batch
  * (restoring the inputs from d_a_src/d_b_src before each trial): 128, 256 or
- * 512 threads per CTA (the trailing update's register micro-tile 4 x 8, 4 x 4
- * or 4 x 2 per thread) times a 16- or 32-column panel, and keeps the fastest;
+ * 512 threads per CTA (a panel row per thread, or two or four) times a 16- or
+ * 32-column panel, and keeps the fastest;
  * threads_out (may be NULL) receives one value per bucket, alg_batch_panels
  * the panel widths. Shapes from an earlier run can be set directly with
  * alg_batch_set_config (host-side; not inside a stream capture). */
