@@ -29,24 +29,13 @@
 #include <math_constants.h>
 
 #include "batched.cuh"
-#include "pivot.cuh"
+#include "cta_lu.cuh"
 
 namespace alg {
 namespace {
 
 constexpr int kMaxN = 512;    // largest order a CTA handles
-constexpr int kLeafW = 16;    // columns a leaf keeps in registers
 
-template <typename T>
-__device__ __forceinline__ T fma_t(T a, T b, T c);
-template <>
-__device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
-template <>
-__device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-
-// Column strides in shared memory: 4 mod 16 entries, so that a half-warp's
-// DMMA fragment loads (4 k x 4 rows or columns) fall in distinct banks.
-__host__ __device__ constexpr int panel_ld(int cap) { return ((cap + 15) & ~15) + 4; }
 // Columns of the trailing matrix taken at a time.
 template <int NT>
 __host__ __device__ constexpr int chunk_cols() {
@@ -55,172 +44,10 @@ __host__ __device__ constexpr int chunk_cols() {
 
 // Shared memory of cta_getrf for panels of up to `cap` rows: the leaf's
 // records, the panel [col][row], two U12 chunks [k][col] and 2 pb + 4 ints.
-// A chunk's row stride is odd in FP64: its columns arrive 32 k at a time
-// (cp.async, a row of U each), and an even stride made those stores 8-way
-// bank conflicts; the FP32 tiles need rows of whole 16 bytes.
-template <typename T, int NT>
-__host__ __device__ constexpr int chunk_ld() {
-  return chunk_cols<NT>() + (sizeof(T) == 8 ? 5 : 4);
-}
 template <typename T, int NT>
 __host__ __device__ constexpr size_t getrf_smem(int cap, int pb) {
   return 2 * (NT / 32) * sizeof(PivotRec<T, kLeafW>) + sizeof(T) * (size_t)panel_ld(cap) * pb +
-         2 * sizeof(T) * (size_t)chunk_ld<T, NT>() * pb + (2 * pb + 4) * 4;
-}
-
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
-// An entry copied asynchronously from global to shared memory.
-template <typename T>
-__device__ __forceinline__ void cp_async_entry(T* dst, const T* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
-               "n"(sizeof(T))
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// A 32 x 16 tile at (r0, c0) of C (mt x cw) -= L U held by one warp: L[k][row]
-// (stride ldl) and U[k][col] (stride ldu) in shared memory, C global (leading
-// dimension n). K terms in increasing k, each one fused multiply-add.
-// Rows and columns past the edge read padding and are not stored.
-struct TileF64 {  // FP64 tensor cores; U is negated, so a load is not touched before its tile's turn
-  double acc[4][2][2];
-  __device__ __forceinline__ void load(const double* C, int n, int r0, int c0, int mt, int cw) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int c = c0 + 8 * j + 2 * t + e;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = r0 + 8 * i + g;
-          acc[i][j][e] = (c < cw && r < mt) ? C[c * n + r] : 0.0;
-        }
-      }
-  }
-  template <int K>
-  __device__ __forceinline__ void update(const double* L, int ldl, const double* U, int ldu, int r0, int c0) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int k = 0; k < K; k += 4) {
-      double av[4], bv[2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = L[(k + t) * ldl + r0 + 8 * i + g];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) bv[j] = -U[(k + t) * ldu + c0 + 8 * j + g];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], av[i], bv[j]);
-    }
-  }
-  __device__ __forceinline__ void store(double* C, int n, int r0, int c0, int mt, int cw) const {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int c = c0 + 8 * j + 2 * t + e;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = r0 + 8 * i + g;
-          if (c < cw && r < mt) C[c * n + r] = acc[i][j][e];
-        }
-      }
-  }
-};
-struct TileF32 {  // CUDA cores; a lane has rows 4 rg .. 4 rg + 3 and columns 4 cg .. 4 cg + 3
-  float acc[4][4];
-  __device__ __forceinline__ void load(const float* C, int n, int r0, int c0, int mt, int cw) {
-    const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = c0 + 4 * cg + j;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = r0 + 4 * rg + i;
-        acc[i][j] = (c < cw && r < mt) ? C[c * n + r] : 0.f;
-      }
-    }
-  }
-  template <int K>
-  __device__ __forceinline__ void update(const float* L, int ldl, const float* U, int ldu, int r0, int c0) {
-    const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
-#pragma unroll 8
-    for (int k = 0; k < K; ++k) {
-      const float4 l = *reinterpret_cast<const float4*>(L + k * ldl + r0 + 4 * rg);
-      const float4 u = *reinterpret_cast<const float4*>(U + k * ldu + c0 + 4 * cg);
-      const float lv[4] = {l.x, l.y, l.z, l.w}, uv[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i][j] = __fmaf_rn(-lv[i], uv[j], acc[i][j]);
-    }
-  }
-  __device__ __forceinline__ void store(float* C, int n, int r0, int c0, int mt, int cw) const {
-    const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = c0 + 4 * cg + j;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = r0 + 4 * rg + i;
-        if (c < cw && r < mt) C[c * n + r] = acc[i][j];
-      }
-    }
-  }
-};
-
-// All tiles of C (mt x cw) -= L U, dealt to the CTA's NW warps; a warp loads
-// its next tile while it updates one (the loads' latency was most of the
-// update's time: n = 400, 670 us per system without).
-template <int K, int NW, typename T>
-__device__ __noinline__ void cta_update(const T* L, int ldl, const T* U, int ldu, T* C, int n, int mt, int cw) {
-  using Tile = std::conditional_t<sizeof(T) == 8, TileF64, TileF32>;
-  const int tr = (mt + 31) / 32, tiles = tr * ((cw + 15) / 16);
-  int cur = threadIdx.x >> 5;
-  if (cur >= tiles) return;
-  Tile t0, t1;
-  int r0 = 32 * (cur % tr), c0 = 16 * (cur / tr), r1 = 0, c1 = 0;
-  t0.load(C, n, r0, c0, mt, cw);
-  for (;;) {
-    if ((cur += NW) < tiles) {
-      r1 = 32 * (cur % tr), c1 = 16 * (cur / tr);
-      t1.load(C, n, r1, c1, mt, cw);
-    }
-    t0.template update<K>(L, ldl, U, ldu, r0, c0);
-    t0.store(C, n, r0, c0, mt, cw);
-    if (cur >= tiles) return;
-    if ((cur += NW) < tiles) {
-      r0 = 32 * (cur % tr), c0 = 16 * (cur / tr);
-      t0.load(C, n, r0, c0, mt, cw);
-    }
-    t1.template update<K>(L, ldl, U, ldu, r1, c1);
-    t1.store(C, n, r1, c1, mt, cw);
-    if (cur >= tiles) return;
-  }
-}
-
-// x <- L^{-1} x for 16 entries x[i] = xs[i * lds]; L unit lower, entry (i, k)
-// at l[k * ldl + i].
-template <typename T>
-__device__ __noinline__ void solve16(const T* l, int ldl, T* xs, int lds, int w) {
-  T x[kLeafW];
-#pragma unroll
-  for (int i = 0; i < kLeafW; ++i) x[i] = i < w ? xs[i * lds] : T(0);
-#pragma unroll
-  for (int k = 0; k < kLeafW - 1; ++k)
-#pragma unroll
-    for (int i = k + 1; i < kLeafW; ++i) x[i] = fma_t<T>(-l[k * ldl + i], x[k], x[i]);
-#pragma unroll
-  for (int i = 0; i < kLeafW; ++i)
-    if (i < w) xs[i * lds] = x[i];
+         2 * sizeof(T) * (size_t)chunk_ld<T>(chunk_cols<NT>()) * pb + (2 * pb + 4) * 4;
 }
 
 // LU with partial pivoting of the n x n matrix a (global, leading dim n) in
@@ -233,7 +60,7 @@ __device__ int cta_getrf(T* a, int n, T* rhs, int* ipiv, int* perm, unsigned cha
   using Rec = PivotRec<T, kLeafW>;
   constexpr int NW = NT / 32;
   constexpr int CH = chunk_cols<NT>();
-  constexpr int ldu = chunk_ld<T, NT>();
+  constexpr int ldu = chunk_ld<T>(chunk_cols<NT>());
   const int ldt = panel_ld(cap);
   Rec(*rec)[NW] = reinterpret_cast<Rec(*)[NW]>(smem);
   T* tile = reinterpret_cast<T*>(smem + 2 * NW * sizeof(Rec));  // [col][row]
@@ -426,7 +253,7 @@ __device__ int cta_getrf(T* a, int n, T* rhs, int* ipiv, int* perm, unsigned cha
       }
       if (mt > 0) {  // (then w == PB)
         const int cm = min(cw, mt - cb);  // the chunk's matrix columns
-        cta_update<PB, NW>(tile + PB, ldt, u, ldu, a + (size_t)(kr + cb) * n + kr, n, mt, cm);
+        cta_update<PB, NW, true>(tile + PB, ldt, u, ldu, a + (size_t)(kr + cb) * n + kr, n, mt, cm);
         if (cm < cw)  // and the right-hand side
           for (int r = tid; r < mt; r += NT) {
             T acc = rhs[kr + r];

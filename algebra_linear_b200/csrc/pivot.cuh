@@ -41,20 +41,22 @@ __device__ __forceinline__ T quotient(T a, T d, T y, bool fast) {
 // (0, INT_MAX) is no candidate (a zero entry is (0, its position), which wins
 // over it). The reference's NaN rule (mod.rs:123-134): +inf on the diagonal,
 // never chosen elsewhere.
+template <bool DIAG_NAN = true>
 __device__ __forceinline__ void pivot_candidate(double v, int pos, int J, unsigned long long& key, int& kpos) {
   key = pos >= J ? (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull : 0ull;
   kpos = pos >= J ? pos : INT_MAX;
   if (v != v) {
-    key = pos == J ? 0x7ff0000000000000ull : 0ull;
-    kpos = pos == J ? J : INT_MAX;
+    key = DIAG_NAN && pos == J ? 0x7ff0000000000000ull : 0ull;
+    kpos = DIAG_NAN && pos == J ? J : INT_MAX;
   }
 }
+template <bool DIAG_NAN = true>
 __device__ __forceinline__ void pivot_candidate(float v, int pos, int J, unsigned& key, int& kpos) {
   key = pos >= J ? __float_as_uint(v) & 0x7fffffffu : 0u;
   kpos = pos >= J ? pos : INT_MAX;
   if (v != v) {
-    key = pos == J ? 0x7f800000u : 0u;
-    kpos = pos == J ? J : INT_MAX;
+    key = DIAG_NAN && pos == J ? 0x7f800000u : 0u;
+    kpos = DIAG_NAN && pos == J ? J : INT_MAX;
   }
 }
 // Warp-wide: the largest key, and among its lanes the smallest tag; true on
@@ -122,6 +124,7 @@ __device__ __forceinline__ int warp_pick(const Rec* rec, int count, int lane, in
 // piv_slot[J] receives the slot of column J's pivot row and ipiv[J] its
 // position at that step. RECIP: multipliers by the reciprocal (else the
 // correctly rounded quotient, see panel_reg_kernel).
+// With RECIP a NaN is never chosen, on the diagonal either (lu_front's rule).
 // Warps without rows (late panels of a CTA sized for the first) only keep the
 // barriers. Returns the first column of the leaf whose pivot is zero (INT_MAX:
 // none); with RECIP the leaf stops there (a column without any number counts
@@ -142,7 +145,7 @@ __device__ __noinline__ int cta_leaf(T* tile, int ldt, int m, int cl0, int w, in
       const int par = (cl0 + j) & 1;
       const T d = rec[par][warp_pick(&rec[par][0], nw, lane, mp)].row[0];
       if (RECIP) {
-        if (!(fabs((double)d) > 0.0)) return cl0 + j;
+        if (!(fabs((double)d) > 0.0) || mp >= (1 << 20)) return cl0 + j;
       } else if (d == T(0) && zero == INT_MAX) {
         zero = cl0 + j;
       }
@@ -165,12 +168,12 @@ __device__ __noinline__ int cta_leaf(T* tile, int ldt, int m, int cl0, int w, in
     Key key, mk;
     int kpos, kslot = tid;
     T cand = v[0][0];
-    pivot_candidate(v[0][0], pos[0], J, key, kpos);
+    pivot_candidate<!RECIP>(v[0][0], pos[0], J, key, kpos);
 #pragma unroll
     for (int k = 1; k < RPT; ++k) {
       Key kk;
       int kp;
-      pivot_candidate(v[k][0], pos[k], J, kk, kp);
+      pivot_candidate<!RECIP>(v[k][0], pos[k], J, kk, kp);
       if (kk > key || (kk == key && kp < kpos)) {
         key = kk;
         kpos = kp;
@@ -178,7 +181,7 @@ __device__ __noinline__ int cta_leaf(T* tile, int ldt, int m, int cl0, int w, in
         cand = v[k][0];
       }
     }
-    const T crecip = RECIP ? T(1) / cand : rcp_rn(exp_fast_ok(cand) ? cand : T(1));
+    const T crecip = rcp_rn(RECIP || exp_fast_ok(cand) ? cand : T(1));
     if (warp_pivot(key, kpos, mk, mp)) {  // (no candidate at all: any lanes, an empty record)
       PivotRec<T, W>& s = rec[par][warp];
       s.key = mk;
@@ -198,7 +201,7 @@ __device__ __noinline__ int cta_leaf(T* tile, int ldt, int m, int cl0, int w, in
     const T d = wr.row[0];
     const T y = wr.recip;
     if (RECIP) {
-      if (!(fabs((double)d) > 0.0)) return J;  // uniform
+      if (!(fabs((double)d) > 0.0) || mp >= (1 << 20)) return J;  // uniform
     } else if (d == T(0) && zero == INT_MAX) {
       zero = J;
     }

@@ -22,6 +22,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cta_lu.cuh"
 #include "dense.cuh"
 #include "sparse_numeric.cuh"
 
@@ -30,13 +31,6 @@ namespace sp {
 namespace {
 
 constexpr int kSmallThreads = 256;
-
-template <typename T>
-__device__ __forceinline__ T fma_t(T a, T b, T c);
-template <>
-__device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
-template <>
-__device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 // The scalar of SparseLu<Complex64> (num_complex::Complex<f64>; lu.rs:61-82),
 // stored interleaved (re, im) as the host's arrays: num-complex's product
@@ -58,9 +52,13 @@ __device__ __forceinline__ zc& operator+=(zc& a, zc b) { return a = a + b; }
 __device__ __forceinline__ zc& operator-=(zc& a, zc b) { return a = a - b; }
 __device__ __forceinline__ zc& operator*=(zc& a, zc b) { return a = a * b; }
 __device__ __forceinline__ bool operator!=(zc a, zc b) { return a.re != b.re || a.im != b.im; }
-template <>
-__device__ __forceinline__ zc fma_t<zc>(zc a, zc b, zc c) {
+__device__ __forceinline__ zc fma_z(zc a, zc b, zc c) {
   return zc(__fma_rn(a.re, b.re, __fma_rn(-a.im, b.im, c.re)), __fma_rn(a.re, b.im, __fma_rn(a.im, b.re, c.im)));
+}
+template <typename T>
+__device__ __forceinline__ T fma_s(T a, T b, T c) {
+  if constexpr (std::is_same<T, zc>::value) return fma_z(a, b, c);
+  else return fma_t<T>(a, b, c);
 }
 
 // |x| as the pivot search compares it (SparseScalar::abs)
@@ -149,7 +147,7 @@ __device__ __forceinline__ void cta_gemm_tile(T* C, const T* A, const T* B, int 
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fma_t(av[r], bv[c], acc[r][c]);
+        for (int c = 0; c < 4; ++c) acc[r][c] = fma_s(av[r], bv[c], acc[r][c]);
     }
   }
 #pragma unroll
@@ -169,41 +167,55 @@ __device__ void cta_gemm_sub(T* C, const T* A, const T* B, int ld, int mr, int n
   __syncthreads();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSmallThreads) small_front_kernel(SmallArgs<T> a) {
-  const int s = a.level_fronts[blockIdx.x];
-  const FrontDesc d = a.fronts[s];
-  const int rows = d.rows, size = d.size, cols = d.size + d.ncb;
+// Zeroes a front's block, lists its rows (the children's unpivoted ones, then
+// those entering here) and assembles its values: the entering rows of A and
+// the children's contribution blocks, a warp per column of one (rows of
+// different children have their own slots, so nothing is added up).
+template <typename T, int NT>
+__device__ __forceinline__ void assemble_small(const SmallArgs<T>& a, const FrontDesc& d) {
+  const int rows = d.rows, cols = d.size + d.ncb;
   T* f = a.block + d.block_off;
   int32_t* rid = a.rowid + d.rowid_off;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t total = (int64_t)rows * cols;
-  for (int64_t e = tid; e < total; e += kSmallThreads) f[e] = T(0);
-  // slots: the children's unpivoted rows, then the rows entering here
+  for (int64_t e = tid; e < total; e += NT) f[e] = T(0);
   for (int k = d.child_begin; k < d.child_end; ++k) {
     const FrontDesc c = a.fronts[a.child_idx[k]];
     const int slot0 = a.child_slot[k];
-    for (int i = tid; i < c.rows - c.size; i += kSmallThreads) rid[slot0 + i] = a.rowid[c.rowid_off + c.size + i];
+    for (int i = tid; i < c.rows - c.size; i += NT) rid[slot0 + i] = a.rowid[c.rowid_off + c.size + i];
   }
   {
     const int slot0 = rows - (d.new_end - d.new_begin);
-    for (int i = tid; i < d.new_end - d.new_begin; i += kSmallThreads) rid[slot0 + i] = a.new_rows[d.new_begin + i];
+    for (int i = tid; i < d.new_end - d.new_begin; i += NT) rid[slot0 + i] = a.new_rows[d.new_begin + i];
   }
   __syncthreads();
-  for (int q = d.anew_begin + tid; q < d.anew_end; q += kSmallThreads)
+  for (int q = d.anew_begin + tid; q < d.anew_end; q += NT)
     f[a.anew_slot[q] + (int64_t)a.anew_col[q] * rows] = load_value<T>(a.values, a.anew_q[q]);
   for (int k = d.child_begin; k < d.child_end; ++k) {
     const FrontDesc c = a.fronts[a.child_idx[k]];
     const int slot0 = a.child_slot[k];
     const int crows = c.rows - c.size;
     const T* cb = a.block + c.cb_off;
-    for (int t = 0; t < c.ncb; ++t) {
-      T* dst = f + slot0 + a.cb_colmap[c.struct_begin + t] * rows;
-      const T* src = cb + t * c.cb_ld;
-      for (int i = tid; i < crows; i += kSmallThreads) dst[i] = src[i];
+#pragma unroll 2
+    for (int t = warp; t < c.ncb; t += NT / 32) {
+      T* dst = f + slot0 + (int64_t)a.cb_colmap[c.struct_begin + t] * rows;
+      const T* src = cb + (int64_t)t * c.cb_ld;
+      for (int i = lane; i < crows; i += 32) dst[i] = src[i];
     }
   }
   __syncthreads();
+}
+
+// Complex small fronts (real ones: small_front_kernel below).
+template <typename T>
+__global__ void __launch_bounds__(kSmallThreads) small_front_z_kernel(SmallArgs<T> a) {
+  const int s = a.level_fronts[blockIdx.x];
+  const FrontDesc d = a.fronts[s];
+  const int rows = d.rows, size = d.size, cols = d.size + d.ncb;
+  T* f = a.block + d.block_off;
+  int32_t* rid = a.rowid + d.rowid_off;
+  const int tid = threadIdx.x;
+  assemble_small<T, kSmallThreads>(a, d);
   // Three barriers per column: (1) the previous column's multipliers are
   // scaled and this column's pivot is searched, each warp posting its
   // candidate in a mailbox double-buffered by column parity that every
@@ -270,7 +282,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_front_kernel(SmallArgs<T>
     const int mr = rows - k - 1, mc = size - k - 1;
     for (int e = tid; e < mr * mc; e += kSmallThreads) {
       const int i = k + 1 + e % mr, j = k + 1 + e / mr;
-      f[i + j * rows] = fma_t(-f[k + j * rows], f[i + k * rows] * inv, f[i + j * rows]);
+      f[i + j * rows] = fma_s(-f[k + j * rows], f[i + k * rows] * inv, f[i + j * rows]);
     }
     inv_prev = inv;
     __syncthreads();
@@ -288,7 +300,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_front_kernel(SmallArgs<T>
       T* col = f + (int64_t)c * rows;
       for (int k = kb; k < ke; ++k) {
         const T uk = col[k];
-        for (int i = k + 1; i < ke; ++i) col[i] = fma_t(-f[i + (int64_t)k * rows], uk, col[i]);
+        for (int i = k + 1; i < ke; ++i) col[i] = fma_s(-f[i + (int64_t)k * rows], uk, col[i]);
       }
     }
     __syncthreads();
@@ -304,6 +316,177 @@ __global__ void __launch_bounds__(kSmallThreads) small_front_kernel(SmallArgs<T>
   T* up = a.U + d.u_off;
   for (int t = 0; t < d.ncb; ++t)
     for (int kk = tid; kk < size; kk += kSmallThreads) up[kk + t * size] = f[kk + (size + t) * rows];
+}
+
+// Small fronts (at most NT rows): one CTA factors a front in its block (global,
+// ld = rows) with a right-looking blocked LU: 16-column panels in shared
+// memory with a row per thread in registers (cta_leaf: first largest |x|,
+// multipliers by the reciprocal, lu_front supernodal_lu.rs:490-533), the
+// interchanges as one gather per panel, and the columns right of it in
+// chunks: U12 by a unit-lower solve, the rest by warp tiles (FP64 tensor
+// cores / FP32 register tiles). Bound by the column chain of the level's
+// largest front (about 0.8 us a column) where a level has few fronts. The
+// 192-dof lattice (one front of 192 x 192): 2.90 ms with rank-1 updates in
+// global memory and three barriers a column, 0.37 ms now; the 300 x 300
+// grid's 27 levels, FP32: 18.6 ms before, 8.9 ms now (twice as many columns
+// per chunk changes neither). CTAs of 64, 128 and 256 threads for fronts of as
+// many rows: idle warps would lengthen every barrier.
+template <int NT>
+__host__ __device__ constexpr int front_chunk() {  // columns right of a panel taken at a time
+  return NT / 4;
+}
+template <typename T, int NT>
+__host__ __device__ constexpr size_t small_front_smem() {
+  return 2 * (NT / 32) * sizeof(PivotRec<T, kLeafW>) +
+         sizeof(T) * (size_t)(panel_ld(NT) + 2 * chunk_ld<T>(front_chunk<NT>())) * kLeafW + 2 * kLeafW * 4 + kLeafW * 4;
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) small_front_kernel(SmallArgs<T> a) {
+  using Rec = PivotRec<T, kLeafW>;
+  constexpr int NW = NT / 32, PB = kLeafW;
+  constexpr int CH = front_chunk<NT>(), ldu = chunk_ld<T>(CH), ldt = panel_ld(NT);
+  extern __shared__ __align__(16) unsigned char smem[];
+  Rec(*rec)[NW] = reinterpret_cast<Rec(*)[NW]>(smem);
+  T* tile = reinterpret_cast<T*>(smem + 2 * NW * sizeof(Rec));  // [col][row]
+  T* us = tile + PB * ldt;                                      // [k][col], two buffers
+  int* piv_slot = reinterpret_cast<int*>(us + 2 * PB * ldu);
+  int* disp = piv_slot + PB;  // where a top row that is no pivot went (-1: it is one)
+  int* piv = disp + PB;
+  const int s = a.level_fronts[blockIdx.x];
+  const FrontDesc d = a.fronts[s];
+  const int rows = d.rows, size = d.size, cols = d.size + d.ncb;
+  T* f = a.block + d.block_off;
+  int32_t* rid = a.rowid + d.rowid_off;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  assemble_small<T, NT>(a, d);
+  for (int k0 = 0; k0 < size; k0 += PB) {
+    const int w = min(PB, size - k0), m = rows - k0, kr = k0 + w, mt = rows - kr;
+    int pos[1] = {tid < m ? tid : -1};
+    {
+      const T* src = f + (k0 + tid) + (int64_t)k0 * rows;
+#pragma unroll
+      for (int c = 0; c < PB; ++c) tile[c * ldt + tid] = (tid < m && c < w) ? src[(int64_t)c * rows] : T(0);
+    }
+    if (tid < PB) disp[tid] = -1;
+    if (cta_leaf<T, kLeafW, NT, 1, false, true>(tile, ldt, m, 0, w, pos, rec, piv_slot, piv) != INT_MAX) {
+      if (tid == 0) atomicExch(a.singular, 1);
+      return;  // uniform: every thread saw the same record
+    }
+    __syncthreads();
+    if (tid < w && pos[0] >= w) disp[tid] = pos[0];
+    const bool moved = __syncthreads_or(tid < w && piv_slot[tid] != tid);
+    if (moved) {  // rows into position order; the same on the left columns and the row list
+      constexpr int kIt = (PB * PB + NT - 1) / NT;
+      T pv[kIt], dv[kIt];
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < w) {
+          pv[it] = tile[c * ldt + piv_slot[i]];
+          dv[it] = tile[c * ldt + i];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < w) {
+          tile[c * ldt + i] = pv[it];
+          if (disp[i] >= 0) tile[c * ldt + disp[i]] = dv[it];
+        }
+      }
+      for (int c = warp; c < k0 + 1; c += NW) {
+        if (c < k0) {
+          T* cp = f + (int64_t)c * rows + k0;
+          T p0 = T(0), d0 = T(0);
+          if (lane < w) {
+            p0 = cp[piv_slot[lane]];
+            d0 = cp[lane];
+          }
+          __syncwarp();
+          if (lane < w) {
+            cp[lane] = p0;
+            if (disp[lane] >= 0) cp[disp[lane]] = d0;
+          }
+        } else {
+          int32_t p0 = 0, d0 = 0;
+          if (lane < w) {
+            p0 = rid[k0 + piv_slot[lane]];
+            d0 = rid[k0 + lane];
+          }
+          __syncwarp();
+          if (lane < w) {
+            rid[k0 + lane] = p0;
+            if (disp[lane] >= 0) rid[k0 + disp[lane]] = d0;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (tid < m) {
+      T* dst = f + (k0 + tid) + (int64_t)k0 * rows;
+#pragma unroll
+      for (int c = 0; c < PB; ++c)
+        if (c < w) dst[(int64_t)c * rows] = tile[c * ldt + tid];
+    }
+    // ---- the columns right of the panel (a chunk's rows of U12 are fetched
+    // while the chunk before it is updated) -----------------------------------
+    const int nright = cols - kr;
+    constexpr int kIt = PB * CH / NT;
+    auto fetch = [&](int cb, T* u) {
+      const int cw = min(CH, nright - cb);
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < cw) cp_async_entry(u + i * ldu + c, f + (k0 + piv_slot[i]) + (int64_t)(kr + cb + c) * rows);
+        else u[i * ldu + c] = T(0);  // a narrow panel's update runs over zeros
+      }
+      cp_async_commit();
+    };
+    if (nright > 0) fetch(0, us);
+    for (int cb = 0, buf = 0; cb < nright; cb += CH, buf ^= 1) {
+      T* u = us + buf * PB * ldu;
+      const int cw = min(CH, nright - cb);
+      T* fc = f + (int64_t)(kr + cb) * rows;
+      T dv[kIt];
+      if (moved) {
+#pragma unroll
+        for (int it = 0; it < kIt; ++it) {
+          const int e = tid + it * NT, i = e % PB, c = e / PB;
+          if (i < w && c < cw) dv[it] = fc[(k0 + i) + (int64_t)c * rows];
+        }
+      }
+      cp_async_wait_all();
+      __syncthreads();
+      if (cb + CH < nright) fetch(cb + CH, us + (buf ^ 1) * PB * ldu);
+      if (moved) {
+#pragma unroll
+        for (int it = 0; it < kIt; ++it) {
+          const int e = tid + it * NT, i = e % PB, c = e / PB;
+          if (i < w && c < cw && disp[i] >= 0) fc[(k0 + disp[i]) + (int64_t)c * rows] = dv[it];
+        }
+      }
+      if (tid < cw) solve16(tile, ldt, u + tid, ldu, w);
+      __syncthreads();
+#pragma unroll
+      for (int it = 0; it < kIt; ++it) {
+        const int e = tid + it * NT, i = e % PB, c = e / PB;
+        if (i < w && c < cw) fc[(k0 + i) + (int64_t)c * rows] = u[i * ldu + c];
+      }
+      if (mt > 0) {
+        if (w == PB) cta_update<PB, NW, true>(tile + PB, ldt, u, ldu, fc + kr, rows, mt, cw);
+        else cta_update<PB, NW, false>(tile + w, ldt, u, ldu, fc + kr, rows, mt, cw);
+      }
+      __syncthreads();
+    }
+  }
+  T* lp = a.L + d.l_off;
+#pragma unroll 4
+  for (int e = tid; e < rows * size; e += NT) lp[e] = f[e];
+  T* up = a.U + d.u_off;
+  for (int t = warp; t < d.ncb; t += NW)
+    for (int kk = lane; kk < size; kk += 32) up[kk + (int64_t)t * size] = f[kk + (int64_t)(size + t) * rows];
 }
 
 // ---- large fronts ----------------------------------------------------------
@@ -457,7 +640,7 @@ __global__ void __launch_bounds__(kZPanelThreads) zfront_panel_kernel(zc* f, int
     const int mr = rows - k - 1, mc = k1 - k - 1;
     for (int e = tid; e < mr * mc; e += kZPanelThreads) {
       const int i = k + 1 + e % mr, j = k + 1 + e / mr;
-      f[i + (int64_t)j * rows] = fma_t(-f[k + (int64_t)j * rows], f[i + (int64_t)k * rows] * inv,
+      f[i + (int64_t)j * rows] = fma_s(-f[k + (int64_t)j * rows], f[i + (int64_t)k * rows] * inv,
                                        f[i + (int64_t)j * rows]);
     }
     inv_prev = inv;
@@ -503,7 +686,7 @@ __global__ void __launch_bounds__(256) zfront_trsm_kernel(zc* f, int rows, int c
 #pragma unroll
     for (int k = 0; k < kZnb; ++k)
 #pragma unroll
-      for (int i = k + 1; i < kZnb; ++i) x[i] = fma_t(-l11[k][i], x[k], x[i]);  // zero outside the block
+      for (int i = k + 1; i < kZnb; ++i) x[i] = fma_s(-l11[k][i], x[k], x[i]);  // zero outside the block
 #pragma unroll
     for (int r = 0; r < kZnb; ++r)
       if (r < w) col[r] = x[r];
@@ -638,9 +821,9 @@ __global__ void __launch_bounds__(kSolveThreads) fwd_diag_kernel(const FrontDesc
       T acc = T(0);
       if (w == 32) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) acc = fma_t(row[(int64_t)k * rows], yb[k], acc);
+        for (int k = 0; k < 32; ++k) acc = fma_s(row[(int64_t)k * rows], yb[k], acc);
       } else {
-        for (int k = 0; k < w; ++k) acc = fma_t(row[(int64_t)k * rows], yb[k], acc);
+        for (int k = 0; k < w; ++k) acc = fma_s(row[(int64_t)k * rows], yb[k], acc);
       }
       ys[i] -= acc;
     }
@@ -671,9 +854,9 @@ __global__ void __launch_bounds__(kSolveThreads) fwd_l21_kernel(const FrontDesc*
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = row[(int64_t)(k + u) * d.rows];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc = fma_t(v[u], ys[k + u], acc);
+    for (int u = 0; u < 8; ++u) acc = fma_s(v[u], ys[k + u], acc);
   }
-  for (; k < k1; ++k) acc = fma_t(row[(int64_t)k * d.rows], ys[k], acc);
+  for (; k < k1; ++k) acc = fma_s(row[(int64_t)k * d.rows], ys[k], acc);
   if (d.size <= kKChunk)
     y[pos_of_row[rowid[d.rowid_off + i]]] -= acc;
   else
@@ -717,9 +900,9 @@ __global__ void __launch_bounds__(kSolveThreads) bwd_u12_kernel(const FrontDesc*
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = up[(int64_t)(t + u) * d.size];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc = fma_t(v[u], x[st[t + u]], acc);
+    for (int u = 0; u < 8; ++u) acc = fma_s(v[u], x[st[t + u]], acc);
   }
-  for (; t < t1; ++t) acc = fma_t(up[(int64_t)t * d.size], x[st[t]], acc);
+  for (; t < t1; ++t) acc = fma_s(up[(int64_t)t * d.size], x[st[t]], acc);
   partial[part_off[it.front] + (int64_t)it.tchunk * d.size + kk] = acc;
 }
 
@@ -775,9 +958,9 @@ __global__ void __launch_bounds__(kSolveThreads) bwd_diag_kernel(const FrontDesc
       T acc = T(0);
       if (w == 32) {
 #pragma unroll
-        for (int l = 0; l < 32; ++l) acc = fma_t(row[(int64_t)l * rows], xb[l], acc);
+        for (int l = 0; l < 32; ++l) acc = fma_s(row[(int64_t)l * rows], xb[l], acc);
       } else {
-        for (int l = 0; l < w; ++l) acc = fma_t(row[(int64_t)l * rows], xb[l], acc);
+        for (int l = 0; l < w; ++l) acc = fma_s(row[(int64_t)l * rows], xb[l], acc);
       }
       xs[i] -= acc;
     }
@@ -867,6 +1050,16 @@ int grid_for(alg_ctx* ctx, int64_t work, int threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, 8LL * ctx->sm_count));
 }
 
+template <typename T, int NT>
+int launch_small(const SmallArgs<T>& sa, int count, cudaStream_t st) {
+  static const cudaError_t configured = cudaFuncSetAttribute(
+      small_front_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_front_smem<T, NT>());
+  ALG_CUDA_TRY(configured);
+  small_front_kernel<T, NT><<<count, NT, small_front_smem<T, NT>(), st>>>(sa);
+  count_launches();
+  return ALG_OK;
+}
+
 // The complex front's partial LU (kernels above) on lane context lc.
 // Stream-ordered; a zero pivot lands in lc's status (singular_col).
 int zfront_lu(alg_ctx* lc, zc* f, int rows, int size, int cols, int* ipiv, int* perm, double* ah) {
@@ -917,7 +1110,23 @@ int DeviceLu::init(alg_ctx* c, const FrontPlan* p, int w) {
   ALG_TRY(upload(F.anew_slot, &d_anew_slot));
   ALG_TRY(upload(F.anew_col, &d_anew_col));
   ALG_TRY(upload(F.new_rows, &d_new_rows));
-  ALG_TRY(upload(F.small_level_fronts, &d_small_levels));
+  {
+    // each level's small fronts by row class (the CTA sizes of small_front_kernel)
+    std::vector<int32_t> order = F.small_level_fronts;
+    const size_t levels = F.small_level_ptr.empty() ? 0 : F.small_level_ptr.size() - 1;
+    small_le64.assign(levels, 0);
+    small_le128.assign(levels, 0);
+    auto cls = [&](int32_t s) { return F.fronts[s].rows <= 64 ? 0 : (F.fronts[s].rows <= 128 ? 1 : 2); };
+    for (size_t h = 0; h < levels; ++h) {
+      auto b = order.begin() + F.small_level_ptr[h], e = order.begin() + F.small_level_ptr[h + 1];
+      std::stable_sort(b, e, [&](int32_t x, int32_t y) { return cls(x) < cls(y); });
+      for (auto it = b; it != e; ++it) {
+        small_le64[h] += cls(*it) == 0;
+        small_le128[h] += cls(*it) == 1;
+      }
+    }
+    ALG_TRY(upload(order, &d_small_levels));
+  }
   ALG_TRY(upload(F.col_perm, &d_col_perm));
   const size_t n = (size_t)std::max<idx>(F.n, 1);
   ALG_TRY(dmalloc((void**)&d_values, sizeof(double) * words * std::max<idx>(F.nnz, 1)));
@@ -1105,8 +1314,18 @@ int DeviceLu::factor_t(int b, const double* values, int tc_prec) {
     const int cnt = F.small_level_ptr[h + 1] - F.small_level_ptr[h];
     if (cnt == 0) continue;
     sa.level_fronts = d_small_levels + F.small_level_ptr[h];
-    small_front_kernel<T><<<cnt, kSmallThreads, 0, st>>>(sa);
-    count_launches();
+    if constexpr (std::is_same<T, zc>::value) {
+      small_front_z_kernel<T><<<cnt, kSmallThreads, 0, st>>>(sa);
+      count_launches();
+    } else {
+      // the level's fronts by rows: at most 64, at most 128, the rest
+      const int n64 = small_le64[h], n128 = small_le128[h];
+      if (n64 > 0) ALG_TRY((launch_small<T, 64>(sa, n64, st)));
+      sa.level_fronts += n64;
+      if (n128 > 0) ALG_TRY((launch_small<T, 128>(sa, n128, st)));
+      sa.level_fronts += n128;
+      if (cnt - n64 - n128 > 0) ALG_TRY((launch_small<T, 256>(sa, cnt - n64 - n128, st)));
+    }
     ALG_CUDA_TRY(cudaGetLastError());
   }
   prof_end(ctx, tok_small, 0.0, 0.0);

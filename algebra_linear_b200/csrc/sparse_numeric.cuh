@@ -52,6 +52,7 @@ struct DeviceLu {
   int64_t* d_anew_q = nullptr;
   int32_t *d_anew_slot = nullptr, *d_anew_col = nullptr, *d_new_rows = nullptr;
   int32_t *d_small_levels = nullptr, *d_col_perm = nullptr;
+  std::vector<int> small_le64, small_le128;  // per level: small fronts of at most 64, of 65..128 rows
   double* d_values = nullptr;  // A's values (CSC order) of the next factorization
   // arenas sized in doubles (times words); the FP32 form uses their first halves as floats
   double* d_block = nullptr;   // small fronts' blocks
