@@ -368,8 +368,12 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
   // the leaf panels of block [k0, k0 + kb), with their in-block updates
   auto factor_block = [&](int k0, int kb, int* lb) -> int {
     for (int c0 = k0, w = 0; c0 < k0 + kb; c0 += w) {
-      // a whole block per launch where it fits on the chip, else leaf by leaf
-      const bool whole = !tslu_ws && nbl == panel_leaf_w<T>() && block_panel_fits<T>(m - c0);
+      // a whole block per launch where it fits on the chip, else leaf by leaf.
+      // With tournament pivoting too: a panel that one cluster holds is a
+      // tree of one node, whose partial-pivoting LU is the panel's (FP32, 64
+      // columns of 5 000 rows: 105 us against 2 x 64 us for the three levels
+      // plus the update between; of 2 000 rows 70 us).
+      const bool whole = nbl == panel_leaf_w<T>() && block_panel_fits<T>(m - c0);
       w = std::min(whole ? kBlockMaxW : nbl, k0 + kb - c0);
       PanelArgs<T> pa;
       pa.a = a;
@@ -386,7 +390,7 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
       int prc = ALG_NOT_IMPLEMENTED;
       bool u12_done = false;  // the tournament's apply step also forms U12 of the block's trailing columns
       if constexpr (std::is_same<T, float>::value) {
-        if (tslu_ws) {
+        if (tslu_ws && !whole) {
           prc = tslu_panel(ctx, TsluArgs{a, lda, m, c0, w, k0, k0 + kb, ipiv, lb, pa.first_leaf, ctx->d_status},
                            tslu_ws);
           u12_done = prc == ALG_OK;

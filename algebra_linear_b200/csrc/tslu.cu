@@ -18,6 +18,9 @@
 //      row gets its multipliers l = a U11^-1, the labels of the moved rows
 //      and the block panel's other columns follow the interchanges, and the
 //      top rows of the block panel's trailing columns become U12.
+// Panels that one cluster holds in shared memory (up to about 8 000 FP32 rows) do
+// not come here: their tree would be one node, and the cluster's
+// partial-pivoting LU (panel_reg_kernel) is that node's, 64 columns a launch.
 // The factorization differs from partial pivoting's (other pivots); the
 // mixed form's refinement in FP64 then brings the solution to the FP64
 // backward error, which is its contract. In the single-launch form every CTA
