@@ -242,15 +242,25 @@ bool dmma_disabled() {
   return off;
 }
 
-// ALG_GEMM_WIDE=1: the CUDA-core update's former 128 x 128 tiles (one CTA
-// per SM) instead of 128 x 64 tiles two to an SM (for comparison).
-bool gemm_wide_tiles() {
-  static const bool v = [] {
-    const char* e = std::getenv("ALG_GEMM_WIDE");
-    return e != nullptr && e[0] == '1';
-  }();
-  return v;
+template <typename T, bool EXACT, int NJ, bool VEC>
+int launch_gemm_sub(alg_ctx* ctx, int M, int N, int K, const T* A, int lda, const T* B, int ldb, T* C, int ldc) {
+  using Cfg = SubCfg<T, NJ>;
+  static const cudaError_t configured = cudaFuncSetAttribute(
+      gemm_sub_kernel<T, EXACT, NJ, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
+  ALG_CUDA_TRY(configured);
+  dim3 grid((M + Cfg::kBM - 1) / Cfg::kBM, (N + Cfg::kBN - 1) / Cfg::kBN);
+  gemm_sub_kernel<T, EXACT, NJ, VEC><<<grid, Cfg::kThreads, Cfg::kSmem, ctx->stream>>>(
+      M, N, K, A, lda, B, ldb, C, ldc, Cfg::kCtas * ctx->sm_count);
+  return ALG_OK;
 }
+
+// C -= A B on the CUDA cores, in 64 x 64 tiles, or 64 x 32 while there are few
+// (as the tensor-core update: shorter last waves and half the latency of the
+// look-ahead chain's narrow updates). Against 128 x 64 tiles of 8 x 8 entries
+// per thread with strided C accesses, two CTAs per SM: the exact update's
+// kernels of an n = 5001 LU 8.1 ms (11.1 ms before), the FP32 in-block updates
+// of n = 16384 11.9 us each (21.2 us before).
+constexpr long long kGemmNarrowTiles = 1024;  // 64 x 64 tiles
 
 template <typename T, bool EXACT>
 int gemm_sub_dev(alg_ctx* ctx, int M, int N, int K, const T* A, int lda, const T* B, int ldb,
@@ -261,24 +271,16 @@ int gemm_sub_dev(alg_ctx* ctx, int M, int N, int K, const T* A, int lda, const T
     if (!dmma_disabled()) return gemm_dmma_sub_dev(ctx, M, N, K, A, lda, B, ldb, C, ldc);
   }
   const int tok = prof_begin(ctx, ALG_K_GEMM);
-  // FP64 (the exact form's update) stages its operands by cp.async:
-  // fp64_exact 296.2 ms against 308.7 ms at n = 16384; FP32 keeps the
-  // register-prefetch form (mixed_fp32 133.8 ms against 138.3 ms).
-  // ALG_GEMM_SYNC=1: the register-prefetch form for FP64 too (measurement switch)
-  static const bool sync_env = [] {
-    const char* e = std::getenv("ALG_GEMM_SYNC");
-    return e != nullptr && e[0] == '1';
-  }();
-  const bool sync_form = sizeof(T) == 4 || sync_env;
-  if (gemm_wide_tiles()) {
-    dim3 grid((M + kGemmBM - 1) / kGemmBM, (N + 127) / 128);
-    gemm_sub_kernel<T, EXACT, 128><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
-  } else if (!sync_form) {
-    dim3 grid((M + kGemmBM - 1) / kGemmBM, (N + 63) / 64);
-    gemm_sub_async_kernel<T, EXACT><<<grid, 128, 0, ctx->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  const int align = 16 / (int)sizeof(T);
+  const bool vec = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) == 0 && lda % align == 0 &&
+                   ldb % align == 0;
+  const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64);
+  if (tiles <= kGemmNarrowTiles) {
+    ALG_TRY(vec ? (launch_gemm_sub<T, EXACT, 4, true>(ctx, M, N, K, A, lda, B, ldb, C, ldc))
+                : (launch_gemm_sub<T, EXACT, 4, false>(ctx, M, N, K, A, lda, B, ldb, C, ldc)));
   } else {
-    dim3 grid((M + kGemmBM - 1) / kGemmBM, (N + 63) / 64);
-    gemm_sub_kernel<T, EXACT, 64><<<grid, 128, 0, ctx->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
+    ALG_TRY(vec ? (launch_gemm_sub<T, EXACT, 8, true>(ctx, M, N, K, A, lda, B, ldb, C, ldc))
+                : (launch_gemm_sub<T, EXACT, 8, false>(ctx, M, N, K, A, lda, B, ldb, C, ldc)));
   }
   count_launches();
   prof_end(ctx, tok, 2.0 * M * N * K, sizeof(T) * (2.0 * M * N + double(M) * K + double(K) * N));

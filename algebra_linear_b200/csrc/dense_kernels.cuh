@@ -1214,210 +1214,140 @@ __global__ void gather_perm_rows_kernel(const T* __restrict__ b, int ldb, const 
 }
 
 // ---------------------------------------------------------------------------
-// K4 (CUDA-core form): C -= A * B with C M x N, A M x K, B K x N, all
-// column-major. Each thread owns an 8 x 8 block of C in registers, loads it
-// once, applies the K terms in increasing k (EXACT: rounded product then
-// rounded difference, the reference's per-entry sequence), and stores it once.
-// 128 x BN CTA tile (BN = 128: 256 threads, one CTA per SM; BN = 64: 128
-// threads, two CTAs per SM, so one tile's C load and store overlap the
-// other's arithmetic), K staged through shared memory 8 at a time with
-// register double buffering. Out-of-range A rows / B columns / k are zero,
-// which leaves every in-range entry unchanged bit for bit (x - 0*0 = x).
+// K4: C -= A B on the CUDA cores (the exact FP64 update and the FP32 one).
+// Every entry takes its terms in increasing k, each a rounded multiply-
+// subtract (EXACT: rounded product, then rounded difference), so it equals
+// the rank-1 order of the reference's loop bit for bit.
+//
+// 128 threads per 64 x (8 NJ) tile: thread (tx, ty) has rows tx + 16 r and
+// columns ty + 8 c, so a warp's C accesses are whole 128-byte lines and its
+// shared-memory reads are free of bank conflicts; A [k][m] and B [n][k] in
+// chunks of 16 k through a three-stage cp.async ring (16-byte copies when the
+// operands allow, else element by element; out-of-range elements are
+// zero-filled, which leaves every in-range entry unchanged bit for bit). A CTA
+// also asks L2 for the C tile its slot takes next. Bound by the FP64 (FP32)
+// pipe. Measured: see the table at gemm_sub_dev.
 // ---------------------------------------------------------------------------
-constexpr int kGemmBM = 128, kGemmBK = 8;
-
-template <typename T, bool EXACT, int BN>
-__global__ void __launch_bounds__(2 * BN, BN == 64 ? 2 : 1) gemm_sub_kernel(
-    int M, int N, int K, const T* __restrict__ A, int lda, const T* __restrict__ B, int ldb,
-    T* __restrict__ Cm, int ldc) {
-  constexpr int kThreads = 2 * BN, kHalf = BN / 2, kAPer = kGemmBK * kGemmBM / kThreads,
-                kBPer = kGemmBK * BN / kThreads;
-  __shared__ __align__(16) T As[2][kGemmBK][kGemmBM];
-  __shared__ __align__(16) T Bs[2][kGemmBK][BN + 2];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.x * kGemmBM, n0 = blockIdx.y * BN;
-
-  T acc[8][8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int mi = m0 + (r >> 2) * 64 + tx * 4 + (r & 3);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int nj = n0 + (c >> 2) * kHalf + ty * 4 + (c & 3);
-      acc[r][c] = (mi < M && nj < N) ? Cm[(size_t)mi + (size_t)nj * ldc] : T(0);
-    }
-  }
-
-  // loader mapping: the A chunk is kGemmBK x 128 (k-major in smem), the B
-  // chunk kGemmBK x BN
-  T ra[kAPer], rb[kBPer];
-  auto load_chunk = [&](int k0) {
-#pragma unroll
-    for (int t = 0; t < kAPer; ++t) {
-      const int idx = tid + t * kThreads;
-      const int mm = idx & 127, kk = idx >> 7;
-      const int gm = m0 + mm, gk = k0 + kk;
-      ra[t] = (gm < M && gk < K) ? A[(size_t)gm + (size_t)gk * lda] : T(0);
-    }
-#pragma unroll
-    for (int t = 0; t < kBPer; ++t) {
-      const int idx = tid + t * kThreads;
-      const int bk = idx & 7, bn = idx >> 3;
-      const int gn = n0 + bn, gk2 = k0 + bk;
-      rb[t] = (gn < N && gk2 < K) ? B[(size_t)gk2 + (size_t)gn * ldb] : T(0);
-    }
-  };
-  auto store_chunk = [&](int buf) {
-#pragma unroll
-    for (int t = 0; t < kAPer; ++t) {
-      const int idx = tid + t * kThreads;
-      As[buf][idx >> 7][idx & 127] = ra[t];
-    }
-#pragma unroll
-    for (int t = 0; t < kBPer; ++t) {
-      const int idx = tid + t * kThreads;
-      Bs[buf][idx & 7][idx >> 3] = rb[t];
-    }
-  };
-
-  const int nchunks = (K + kGemmBK - 1) / kGemmBK;
-  if (nchunks > 0) {
-    load_chunk(0);
-    store_chunk(0);
-  }
-  __syncthreads();
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const int buf = ch & 1;
-    if (ch + 1 < nchunks) load_chunk((ch + 1) * kGemmBK);
-#pragma unroll
-    for (int kk = 0; kk < kGemmBK; ++kk) {
-      T af[8], bf[8];
-#pragma unroll
-      for (int r = 0; r < 8; ++r) af[r] = As[buf][kk][(r >> 2) * 64 + tx * 4 + (r & 3)];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) bf[c] = Bs[buf][kk][(c >> 2) * kHalf + ty * 4 + (c & 3)];
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = msub<EXACT>(acc[r][c], af[r], bf[c]);
-    }
-    if (ch + 1 < nchunks) store_chunk(buf ^ 1);
-    __syncthreads();
-  }
-
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int mi = m0 + (r >> 2) * 64 + tx * 4 + (r & 3);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int nj = n0 + (c >> 2) * kHalf + ty * 4 + (c & 3);
-      if (mi < M && nj < N) Cm[(size_t)mi + (size_t)nj * ldc] = acc[r][c];
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// K4a: the same update (128 x 64 tile, 128 threads, 8 x 8 per thread, each
-// entry's terms in increasing k) with A and B staged by cp.async through a
-// three-stage shared-memory ring instead of registers: no prefetch registers,
-// and the loads of chunk c + 2 run while chunk c is multiplied. Element-wise
-// copies (any leading dimension and offset); out-of-range elements are
-// zero-filled, which leaves every in-range entry unchanged bit for bit.
-// ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void cp_async_elem_zfill(T* dst, const T* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 8) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
-  }
-}
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-constexpr int kGemmAsyncStages = 3;
+template <typename T, int NJ>
+struct SubCfg {
+  static constexpr int kBM = 64, kBN = 8 * NJ, kBK = 16, kThreads = 128, kStages = 3;
+  static constexpr int kV = 16 / (int)sizeof(T);
+  static constexpr int kBS = kBK + kV;  // B's row stride
+  static constexpr int kStage = kBK * kBM + kBN * kBS;
+  static constexpr size_t kSmem = sizeof(T) * kStages * kStage;
+  static constexpr int kCtas = sizeof(T) == 8 && NJ == 8 ? 4 : 5;  // per SM
+};
 
-template <typename T, bool EXACT>
-__global__ void __launch_bounds__(128, 2) gemm_sub_async_kernel(int M, int N, int K, const T* __restrict__ A, int lda,
-                                                                const T* __restrict__ B, int ldb, T* __restrict__ Cm,
-                                                                int ldc) {
-  constexpr int kBN = 64, kHalf = kBN / 2, kThreads = 128, kBS = kBN + 2;
-  constexpr int kStage = kGemmBK * kGemmBM + kGemmBK * kBS;
-  __shared__ __align__(16) T smem[kGemmAsyncStages * kStage];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.x * kGemmBM, n0 = blockIdx.y * kBN;
+template <typename T, bool EXACT, int NJ, bool VEC>
+__global__ void __launch_bounds__(128, SubCfg<T, NJ>::kCtas)
+    gemm_sub_kernel(int M, int N, int K, const T* __restrict__ A, int lda, const T* __restrict__ B, int ldb,
+                    T* __restrict__ Cm, int ldc, int ahead) {
+  using Cfg = SubCfg<T, NJ>;
+  constexpr int kBM = Cfg::kBM, kBN = Cfg::kBN, kBK = Cfg::kBK, kThreads = Cfg::kThreads, kStages = Cfg::kStages;
+  constexpr int kV = Cfg::kV, kBS = Cfg::kBS, kStage = Cfg::kStage;
+  struct alignas(16) Vec {
+    T e[kV];
+  };
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* smem = reinterpret_cast<T*>(smem_raw);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
 
   auto load_stage = [&](int stage, int k0) {
     T* As = smem + stage * kStage;  // [k][m]
-    T* Bs = As + kGemmBK * kGemmBM;  // [k][n], padded rows
+    T* Bs = As + kBK * kBM;         // [n][k]
+    constexpr int P = VEC ? kV : 1;  // entries per copy
+    auto copy = [&](T* dst, const T* src, int count) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+      if constexpr (VEC)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src),
+                     "r"(max(0, min(kV, count)) * (int)sizeof(T)) : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(sizeof(T)),
+                     "r"(count > 0 ? (int)sizeof(T) : 0) : "memory");
+    };
 #pragma unroll
-    for (int r = 0; r < kGemmBK * kGemmBM / kThreads; ++r) {
+    for (int r = 0; r < kBK * kBM / (P * kThreads); ++r) {
       const int e = tid + r * kThreads;
-      const int mm = e & (kGemmBM - 1), kk = e / kGemmBM;
+      const int mm = P * (e % (kBM / P)), kk = e / (kBM / P);
       const int gm = m0 + mm, gk = k0 + kk;
-      const bool ok = gm < M && gk < K;
-      cp_async_elem_zfill(As + kk * kGemmBM + mm, ok ? A + (size_t)gm + (size_t)gk * lda : A, ok);
+      const int cnt = gk < K ? M - gm : 0;
+      copy(As + kk * kBM + mm, cnt > 0 ? A + (size_t)gm + (size_t)gk * lda : A, cnt);
     }
 #pragma unroll
-    for (int r = 0; r < kGemmBK * kBN / kThreads; ++r) {
+    for (int r = 0; r < kBK * kBN / (P * kThreads); ++r) {
       const int e = tid + r * kThreads;
-      const int kk = e % kGemmBK, nn = e / kGemmBK;
+      const int kk = P * (e % (kBK / P)), nn = e / (kBK / P);
       const int gn = n0 + nn, gk = k0 + kk;
-      const bool ok = gn < N && gk < K;
-      cp_async_elem_zfill(Bs + kk * kBS + nn, ok ? B + (size_t)gk + (size_t)gn * ldb : B, ok);
+      const int cnt = gn < N ? K - gk : 0;
+      copy(Bs + nn * kBS + kk, cnt > 0 ? B + (size_t)gk + (size_t)gn * ldb : B, cnt);
     }
   };
 
-  const int nch = (K + kGemmBK - 1) / kGemmBK;
+  const int nch = (K + kBK - 1) / kBK;
 #pragma unroll
-  for (int st = 0; st < kGemmAsyncStages - 1; ++st) {
-    if (st < nch) load_stage(st, st * kGemmBK);
+  for (int st = 0; st < kStages - 1; ++st) {
+    if (st < nch) load_stage(st, st * kBK);
     cp_async_commit_group();
   }
-  T acc[8][8];
+  T acc[4][NJ];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int mi = m0 + (r >> 2) * 64 + tx * 4 + (r & 3);
+  for (int c = 0; c < NJ; ++c) {
+    const int nj = n0 + ty + 8 * c;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int nj = n0 + (c >> 2) * kHalf + ty * 4 + (c & 3);
+    for (int r = 0; r < 4; ++r) {
+      const int mi = m0 + tx + 16 * r;
       acc[r][c] = (mi < M && nj < N) ? Cm[(size_t)mi + (size_t)nj * ldc] : T(0);
     }
   }
+  {
+    constexpr int kLine = 128 / (int)sizeof(T);
+    const int nxt = (int)(blockIdx.x + blockIdx.y * gridDim.x) + ahead;
+    if (nxt < (int)(gridDim.x * gridDim.y)) {
+      const int pm = (nxt % (int)gridDim.x) * kBM, pn = (nxt / (int)gridDim.x) * kBN;
+      for (int e = tid; e < kBN * (kBM / kLine); e += kThreads) {
+        const int r = pm + kLine * (e % (kBM / kLine)), c = pn + e / (kBM / kLine);
+        if (r < M && c < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(Cm + (size_t)r + (size_t)c * ldc));
+      }
+    }
+  }
   for (int ch = 0; ch < nch; ++ch) {
-    cp_async_wait_group<kGemmAsyncStages - 2>();  // chunk ch has landed
-    __syncthreads();  // ... for every thread, and chunk ch - 1's stage is free
-    if (ch + kGemmAsyncStages - 1 < nch)
-      load_stage((ch + kGemmAsyncStages - 1) % kGemmAsyncStages, (ch + kGemmAsyncStages - 1) * kGemmBK);
+    cp_async_wait_group<kStages - 2>();  // chunk ch has landed
+    __syncthreads();                     // ... for every thread, and chunk ch - 1's stage is free
+    if (ch + kStages - 1 < nch) load_stage((ch + kStages - 1) % kStages, (ch + kStages - 1) * kBK);
     cp_async_commit_group();
-    const T* As = smem + (ch % kGemmAsyncStages) * kStage;
-    const T* Bs = As + kGemmBK * kGemmBM;
+    const T* As = smem + (ch % kStages) * kStage;
+    const T* Bs = As + kBK * kBM;
 #pragma unroll
-    for (int kk = 0; kk < kGemmBK; ++kk) {
-      T af[8], bf[8];
+    for (int k0 = 0; k0 < kBK; k0 += kV) {
+      Vec bv[NJ];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) af[r] = As[kk * kGemmBM + (r >> 2) * 64 + tx * 4 + (r & 3)];
+      for (int c = 0; c < NJ; ++c) bv[c] = *reinterpret_cast<const Vec*>(Bs + (ty + 8 * c) * kBS + k0);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) bf[c] = Bs[kk * kBS + (c >> 2) * kHalf + ty * 4 + (c & 3)];
+      for (int q = 0; q < kV; ++q) {
+        T av[4];
 #pragma unroll
-      for (int r = 0; r < 8; ++r)
+        for (int r = 0; r < 4; ++r) av[r] = As[(k0 + q) * kBM + tx + 16 * r];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = msub<EXACT>(acc[r][c], af[r], bf[c]);
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int c = 0; c < NJ; ++c) acc[r][c] = msub<EXACT>(acc[r][c], av[r], bv[c].e[q]);
+      }
     }
   }
   cp_async_wait_group<0>();
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int mi = m0 + (r >> 2) * 64 + tx * 4 + (r & 3);
+  for (int c = 0; c < NJ; ++c) {
+    const int nj = n0 + ty + 8 * c;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int nj = n0 + (c >> 2) * kHalf + ty * 4 + (c & 3);
+    for (int r = 0; r < 4; ++r) {
+      const int mi = m0 + tx + 16 * r;
       if (mi < M && nj < N) Cm[(size_t)mi + (size_t)nj * ldc] = acc[r][c];
     }
   }

@@ -2,14 +2,16 @@
 // fused (non bit-exact) forms: the FP64 LU with fused updates and the sparse
 // fronts' Schur complements.
 //
-// CTA tile 128 x 64 (four warps in a 2 x 2 grid, two CTAs per SM), each warp
-// a 64 x 32 tile = 8 x 4 m8n8 accumulators (two doubles per lane each); K in
-// chunks of 16 staged in shared memory by cp.async through a three-stage
-// ring: 16-byte copies of two consecutive doubles when the operands allow,
-// 8-byte copies otherwise (any leading dimension and offset); out-of-range
-// elements are zero-filled. The accumulators start as -C and each MMA adds
-// A B (the store negates back), so every partial sum is one fused
-// multiply-add chain into C, as the CUDA-core fused kernel does.
+// CTA tile 64 x 64 or 64 x 32 (four warps in a 2 x 2 grid, three or four CTAs
+// per SM), each warp 4 x 4 or 4 x 2 m8n8 accumulators (two doubles per lane
+// each); K in chunks of 16 staged in shared memory by cp.async through a
+// three-stage ring: 16-byte copies of two consecutive doubles when the
+// operands allow, 8-byte copies otherwise (any leading dimension and offset);
+// out-of-range elements are zero-filled. The accumulators start as C and each
+// MMA subtracts A B, so every partial sum is one fused multiply-add chain into
+// C, as the CUDA-core fused kernel does. Bound by the FP64 tensor cores for
+// K >= 128 (30.1 of cuBLAS's 35.4 TFLOP/s on a square GEMM), by C's traffic
+// beside them for K = 64.
 // Shared-memory rows are padded by 4 doubles so that a half-warp's fragment
 // loads (4 k-rows x 4 m-columns) fall in 32 distinct banks.
 #include <algorithm>
@@ -46,31 +48,34 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// Tile shape: 128 x (32 WN) per CTA, warps in a 2 x WN grid, each warp 64 x 32
-// (8 x 4 m8n8 accumulators, two doubles per lane each). K in chunks of 16
-// through a STAGES-deep cp.async ring. VEC: 16-byte copies of two
-// consecutive doubles (A's rows / B's k entries), when both operands and
-// their leading dimensions allow it; 8-byte copies otherwise.
-template <int WN, int STAGES, bool VEC>
+// Tile shape: four warps in a 2 x 2 grid, each warp 8 MI x 8 NJ (MI x NJ m8n8
+// accumulators, two doubles per lane each). K in chunks of 16 through a
+// three-stage cp.async ring. VEC: 16-byte copies of two consecutive doubles
+// (A's rows / B's k entries), when both operands and their leading dimensions
+// allow it; 8-byte copies otherwise.
+template <int MI, int NJ>
 struct DmmaCfg {
-  static constexpr int kBM = 128, kBN = 32 * WN, kBK = 16, kThreads = 64 * WN;
+  static constexpr int kBM = 16 * MI, kBN = 16 * NJ, kBK = 16, kThreads = 128, kStages = 3;
   static constexpr int kAS = kBM + 4;  // As[k][m] row stride (doubles)
   static constexpr int kBS = kBK + 4;  // Bs[n][k] row stride
   static constexpr int kStage = kBK * kAS + kBN * kBS;
-  static constexpr size_t kSmem = sizeof(double) * STAGES * kStage;
+  static constexpr size_t kSmem = sizeof(double) * kStages * kStage;
 };
 
-template <int WN, int STAGES, bool VEC>
-__global__ void __launch_bounds__(64 * WN, WN == 2 ? 2 : 1)
+// `ahead`: a CTA also asks L2 for the C tile that its slot takes next (linear
+// tile index + ahead), so that DRAM works during the MMAs instead of between
+// them.
+template <int MI, int NJ, bool VEC>
+__global__ void __launch_bounds__(128, NJ == 4 ? 3 : 4)
     dmma_gemm_sub_kernel(int M, int N, int K, const double* __restrict__ A, int lda, const double* __restrict__ B,
-                         int ldb, double* __restrict__ C, int ldc) {
-  using Cfg = DmmaCfg<WN, STAGES, VEC>;
-  constexpr int kBM = Cfg::kBM, kBN = Cfg::kBN, kBK = Cfg::kBK, kThreads = Cfg::kThreads;
+                         int ldb, double* __restrict__ C, int ldc, int ahead) {
+  using Cfg = DmmaCfg<MI, NJ>;
+  constexpr int kBM = Cfg::kBM, kBN = Cfg::kBN, kBK = Cfg::kBK, kThreads = Cfg::kThreads, STAGES = Cfg::kStages;
   constexpr int kAS = Cfg::kAS, kBS = Cfg::kBS, kStage = Cfg::kStage;
   extern __shared__ __align__(16) double smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = (warp & 1) * 64, wn = (warp >> 1) * 32;
+  const int wm = (warp & 1) * (kBM / 2), wn = (warp >> 1) * (kBN / 2);
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
 
   auto load_stage = [&](int stage, int k0) {
@@ -121,20 +126,30 @@ __global__ void __launch_bounds__(64 * WN, WN == 2 ? 2 : 1)
     cp_async_commit();
   }
 
-  // accumulators = -C (fragment layout: row g, columns 2t and 2t + 1 of each
-  // m8n8 tile); the MMAs add A B and the store writes -acc: rounding is
-  // symmetric, so -(-C + A B) equals C - A B term by term, and the operands
-  // need no negation
-  double acc[8][4][2];
+  // accumulators = C (fragment layout: row g, columns 2t and 2t + 1 of each
+  // m8n8 tile); B's fragments are negated, so no instruction waits for a C
+  // entry before the first MMA that takes it
+  double acc[MI][NJ][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int gm = m0 + wm + i * 8 + g, gn = n0 + wn + j * 8 + 2 * t + h;
-        acc[i][j][h] = (gm < M && gn < N) ? -C[(size_t)gm + (size_t)gn * ldc] : 0.0;
+        acc[i][j][h] = (gm < M && gn < N) ? C[(size_t)gm + (size_t)gn * ldc] : 0.0;
       }
+  {
+    const int nxt = (int)(blockIdx.x + blockIdx.y * gridDim.x) + ahead;
+    if (nxt < (int)(gridDim.x * gridDim.y)) {
+      const int pm = (nxt % (int)gridDim.x) * kBM, pn = (nxt / (int)gridDim.x) * kBN;
+#pragma unroll
+      for (int e = tid; e < kBN * (kBM / 16); e += kThreads) {  // a 128-byte line each
+        const int r = pm + 16 * (e % (kBM / 16)), c = pn + e / (kBM / 16);
+        if (r < M && c < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (size_t)r + (size_t)c * ldc));
+      }
+    }
+  }
 
   for (int ch = 0; ch < nch; ++ch) {
     cp_async_wait<STAGES - 2>();  // chunk ch has landed
@@ -146,58 +161,59 @@ __global__ void __launch_bounds__(64 * WN, WN == 2 ? 2 : 1)
     const double* Bs = As + kBK * kAS;
 #pragma unroll
     for (int k4 = 0; k4 < kBK; k4 += 4) {
-      double af[8], bf[4];
+      double af[MI], bf[NJ];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) af[i] = As[(k4 + t) * kAS + wm + i * 8 + g];
+      for (int i = 0; i < MI; ++i) af[i] = As[(k4 + t) * kAS + wm + i * 8 + g];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bf[j] = Bs[(wn + j * 8 + g) * kBS + k4 + t];
+      for (int j = 0; j < NJ; ++j) bf[j] = -Bs[(wn + j * 8 + g) * kBS + k4 + t];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
     }
   }
   cp_async_wait<0>();
 
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int gm = m0 + wm + i * 8 + g, gn = n0 + wn + j * 8 + 2 * t + h;
-        if (gm < M && gn < N) C[(size_t)gm + (size_t)gn * ldc] = -acc[i][j][h];
+        if (gm < M && gn < N) C[(size_t)gm + (size_t)gn * ldc] = acc[i][j][h];
       }
 }
 
-template <int WN, int STAGES, bool VEC>
+template <int MI, int NJ, bool VEC>
 int launch_dmma(alg_ctx* ctx, int M, int N, int K, const double* A, int lda, const double* B, int ldb, double* C,
                 int ldc) {
-  using Cfg = DmmaCfg<WN, STAGES, VEC>;
+  using Cfg = DmmaCfg<MI, NJ>;
   static const cudaError_t configured = cudaFuncSetAttribute(
-      dmma_gemm_sub_kernel<WN, STAGES, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
+      dmma_gemm_sub_kernel<MI, NJ, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
   ALG_CUDA_TRY(configured);
   dim3 grid((M + Cfg::kBM - 1) / Cfg::kBM, (N + Cfg::kBN - 1) / Cfg::kBN);
-  dmma_gemm_sub_kernel<WN, STAGES, VEC><<<grid, Cfg::kThreads, Cfg::kSmem, ctx->stream>>>(M, N, K, A, lda, B, ldb,
-                                                                                          C, ldc);
+  dmma_gemm_sub_kernel<MI, NJ, VEC><<<grid, Cfg::kThreads, Cfg::kSmem, ctx->stream>>>(
+      M, N, K, A, lda, B, ldb, C, ldc, (NJ == 4 ? 3 : 4) * ctx->sm_count);
   return ALG_OK;
-}
-
-// ALG_DMMA_SHAPE=1: the former shape (128 x 128 tile, 8 warps, one CTA per
-// SM, two stages of 8-byte copies), for comparison.
-bool dmma_old_shape() {
-  static const bool v = [] {
-    const char* e = std::getenv("ALG_DMMA_SHAPE");
-    return e != nullptr && e[0] == '1';
-  }();
-  return v;
 }
 
 }  // namespace
 
-// Default: 128 x 64 tiles of 4 warps, two CTAs per SM (one tile's C load
-// and store overlap the other's MMAs), a three-stage ring; 16-byte copies
-// when A, B are 16-byte aligned with even leading dimensions.
+// 64 x 64 tiles, three CTAs per SM (one tile's C load and store overlap the
+// others' MMAs); 64 x 32 tiles, four per SM, while there are few tiles: the
+// last wave is shorter and a tile's own latency, which the look-ahead chain's
+// narrow updates wait for, is halved. 16-byte copies when A, B are 16-byte
+// aligned with even leading dimensions. Measured (M x N x K, us; 128 x 64
+// tiles two to an SM before, 64 x 32, 64 x 64):
+//   8192 x 8192 x 128    642   600   570  (cuBLAS's C - A B: 577)
+//   4096 x 4096 x 64     106    92    91
+//   2000 x 2000 x 64      30    25    25
+//   1000 x 1000 x 64      10.5   8.5   8.8
+//   16000 x 128 x 128     26    23    26
+//   3000 x 64 x 64        10.2   4.0   5.9
+constexpr long long kNarrowTiles = 1024;  // 64 x 64 tiles
+
 int gemm_dmma_sub_dev(alg_ctx* ctx, int M, int N, int K, const double* A, int lda, const double* B, int ldb,
                       double* C, int ldc) {
   if (M <= 0 || N <= 0 || K <= 0) return ALG_OK;
@@ -205,9 +221,14 @@ int gemm_dmma_sub_dev(alg_ctx* ctx, int M, int N, int K, const double* A, int ld
                    (lda % 2) == 0 && (ldb % 2) == 0;
   const int tok = prof_begin(ctx, ALG_K_GEMM);
   int rc;
-  if (dmma_old_shape()) rc = launch_dmma<4, 2, false>(ctx, M, N, K, A, lda, B, ldb, C, ldc);
-  else if (vec) rc = launch_dmma<2, 3, true>(ctx, M, N, K, A, lda, B, ldb, C, ldc);
-  else rc = launch_dmma<2, 3, false>(ctx, M, N, K, A, lda, B, ldb, C, ldc);
+  const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64);
+  if (tiles <= kNarrowTiles) {
+    rc = vec ? launch_dmma<4, 2, true>(ctx, M, N, K, A, lda, B, ldb, C, ldc)
+             : launch_dmma<4, 2, false>(ctx, M, N, K, A, lda, B, ldb, C, ldc);
+  } else {
+    rc = vec ? launch_dmma<4, 4, true>(ctx, M, N, K, A, lda, B, ldb, C, ldc)
+             : launch_dmma<4, 4, false>(ctx, M, N, K, A, lda, B, ldb, C, ldc);
+  }
   count_launches();
   prof_end(ctx, tok, 2.0 * M * N * K, 8.0 * (2.0 * M * N + double(M) * K + double(K) * N));
   ALG_TRY(rc);

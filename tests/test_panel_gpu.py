@@ -58,3 +58,56 @@ def test_blocks_wider_and_narrower_than_a_launch(gpu, oracle, monkeypatch, nb):
     rows = cols = 523
     a = np.random.default_rng(nb).uniform(-1.0, 1.0, rows * cols)
     check(oracle, a, rows, cols)
+
+
+@pytest.mark.parametrize("lda_off,a_off", [(0, 0), (1, 0), (0, 1)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 65, 15), (64, 32, 16), (65, 33, 17), (200, 130, 64), (2100, 2051, 40),
+                                   (4200, 1100, 129)])
+def test_fused_update_edges(gpu, m, n, k, lda_off, a_off):
+    """C -= A B at the tile edges of both tile shapes, with aligned operands
+    (16-byte copies) and not. Bound: k + 1 roundings of the entry's terms,
+    gamma_{k+1} (|C| + |A| |B|)."""
+    import torch
+
+    from algebra_linear_b200 import _lib
+    from algebra_linear_b200.device import Context
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    lda = m + (m & 1) + lda_off
+    ldb = k + (k & 1) + lda_off
+    u = lambda cnt: torch.rand(cnt, generator=g, dtype=torch.float64, device="cuda") * 2 - 1  # noqa: E731
+    A, B, Cm = u(lda * k + a_off), u(ldb * n + a_off), u(m * n)
+    ref_a = A[a_off:].as_strided((k, m), (lda, 1))
+    ref_b = B[a_off:].as_strided((n, k), (ldb, 1))
+    C0 = Cm.view(n, m).clone()
+    with Context() as ctx:
+        rc = _lib.load().alg_gemm_dmma_sub_dev(ctx.handle, m, n, k, A.data_ptr() + 8 * a_off, lda,
+                                               B.data_ptr() + 8 * a_off, ldb, Cm.data_ptr(), m)
+        assert rc == 0
+    gamma = (k + 2) * 2.0**-53
+    bound = 2 * gamma * (C0.abs() + ref_b.abs() @ ref_a.abs())
+    assert ((Cm.view(n, m) - (C0 - ref_b @ ref_a)).abs() <= bound + 1e-300).all()
+
+
+@pytest.mark.parametrize("n", [130, 1999])
+def test_exact_update_with_odd_strides_bit_identical(gpu, oracle, n):
+    """The exact update's element-wise copies (odd leading dimension) and its
+    16-byte ones (even) give the oracle's bits; n = 1999 has both tile shapes."""
+    import torch
+
+    from algebra_linear_b200 import _lib
+    from algebra_linear_b200.device import Context
+
+    a = np.random.default_rng(n).uniform(-1.0, 1.0, n * n)
+    ra = a.copy()
+    rc, rpiv, _, _ = oracle.dgetrf(ra, n)
+    assert rc == 0
+    for lda in (n, n + 1):
+        A = torch.zeros(lda * n, dtype=torch.float64, device="cuda")
+        A.view(n, lda)[:, :n] = torch.from_numpy(a).cuda().view(n, n)
+        ipiv = torch.empty(n, dtype=torch.int32, device="cuda")
+        with Context() as ctx:
+            assert _lib.load().alg_dgetrf_dev(ctx.handle, 0, A.data_ptr(), n, lda, ipiv.data_ptr(), None) == 0
+        assert ipiv.cpu().tolist() == list(rpiv)
+        got = A.view(n, lda)[:, :n].contiguous().view(-1).cpu().numpy()
+        assert same_bits(got, ra)
