@@ -20,6 +20,12 @@ struct DevStatus {
   int pad[5];
 };
 
+// Whether the factorization that wrote this block met a zero pivot or gave up.
+__device__ __forceinline__ bool factor_failed(const DevStatus* s) {
+  const volatile DevStatus* v = s;
+  return v->singular_col != INT_MAX || v->timeout != 0;
+}
+
 // Arithmetic of one multiply-subtract `acc - l * u`.
 //  EXACT = true : rounded product, then rounded difference (two roundings),
 //                 the operation order of the reference's scalar loop

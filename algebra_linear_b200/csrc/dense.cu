@@ -454,7 +454,9 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
                                   a + (size_t)k0 + (size_t)cb * lda, lda, a + (size_t)kr + (size_t)cb * lda, lda);
   };
 
-  const bool la = lookahead_enabled() && nc > nb;
+  // (with two blocks there is nothing beside the chain: one stream saves the
+  // events and a swap launch, n = 96: 174 us against 180 us)
+  const bool la = lookahead_enabled() && nc > 2 * nb;
   if (!la) {
     for (int k0 = 0; k0 < nc; k0 += nb) {
       const int kb = std::min(nb, nc - k0);
@@ -523,7 +525,8 @@ constexpr int kBlockedSolveRhs = 16;
 // reads x1 and writes y into x2; the backward sweep reads x2 and writes x
 // into x1.
 template <typename T>
-int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb) {
+int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb,
+                         const DevStatus* guard) {
   if (n == 0 || nrhs == 0) return ALG_OK;
   constexpr int kb = kSolveKb;
   const int nblk = (n + kb - 1) / kb;
@@ -558,7 +561,7 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
     tri_block_inverse_kernel<T, true, 4, 2><<<ig, kTrsmThreads, kInvSmem, ctx->stream>>>(lu, lda, n, kb, uinv);
     const size_t cnt = (size_t)n * nrhs;
     const int g = (int)std::max<size_t>(1, std::min<size_t>((cnt + 255) / 256, (size_t)ctx->sm_count * 8));
-    gather_perm_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x1, n);
+    gather_perm_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x1, n, guard);
     count_launches(3);
     ALG_CUDA_TRY(cudaGetLastError());
   }
@@ -579,20 +582,19 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
     count_launches();
   }
   ALG_CUDA_TRY(cudaGetLastError());
-  ALG_CUDA_TRY(cudaMemcpy2DAsync(b, sizeof(T) * (size_t)ldb, x1, sizeof(T) * (size_t)n, sizeof(T) * (size_t)n, nrhs,
-                                 cudaMemcpyDeviceToDevice, ctx->stream));
+  ALG_TRY(store_solution_dev<T>(ctx, x1, n, nrhs, b, ldb, guard));
   prof_end(ctx, tok, 2.0 * n * n * nrhs, sizeof(T) * (double(n) * n + 4.0 * n * nrhs));
   return ALG_OK;
 }
 
 template <typename T, bool EXACT>
 int lu_solve_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs,
-                 int ldb) {
+                 int ldb, const DevStatus* guard) {
   if (nrhs > 65535) return ALG_BAD_SHAPE;
   // the exact form keeps the reference's per-entry order (the dataflow
   // sweeps); the fused forms solve many right-hand sides blocked
-  if (!EXACT && nrhs >= kBlockedSolveRhs) return lu_solve_blocked_dev<T>(ctx, lu, n, lda, perm, b, nrhs, ldb);
-  return lu_solve_dataflow_dev<T, EXACT>(ctx, lu, n, lda, perm, b, nrhs, ldb);
+  if (!EXACT && nrhs >= kBlockedSolveRhs) return lu_solve_blocked_dev<T>(ctx, lu, n, lda, perm, b, nrhs, ldb, guard);
+  return lu_solve_dataflow_dev<T, EXACT>(ctx, lu, n, lda, perm, b, nrhs, ldb, guard);
 }
 
 int trsm_lower_unit_f32(alg_ctx* ctx, float* a, int lda, int r0, int kb, int cb, int ce) {
@@ -603,7 +605,7 @@ int trsm_lower_unit_f32(alg_ctx* ctx, float* a, int lda, int r0, int kb, int cb,
 #define ALG_INST(T, E)                                                                          \
   template int lu_factor_dev<T, E>(alg_ctx*, T*, int, int, int, int*, int*, const LuPlan&);   \
   template int lu_factor_partial_dev<T, E>(alg_ctx*, T*, int, int, int, int, int*, int*, const LuPlan&); \
-  template int lu_solve_dev<T, E>(alg_ctx*, const T*, int, int, const int*, T*, int, int);    \
+  template int lu_solve_dev<T, E>(alg_ctx*, const T*, int, int, const int*, T*, int, int, const DevStatus*); \
   template int gemm_sub_dev<T, E>(alg_ctx*, int, int, int, const T*, int, const T*, int, T*, int);
 ALG_INST(double, true)
 ALG_INST(double, false)
@@ -629,11 +631,13 @@ int factor_any(alg_ctx* ctx, int update, double* d_a, int m, int nc, int lda, in
   return ALG_INVALID_ARGUMENT;
 }
 
+// guard: see lu_solve_dev. With it a solve follows its factorization without
+// the host looking at the status in between (one synchronisation a dgesv).
 int solve_any(alg_ctx* ctx, int update, const double* d_lu, int n, int lda, const int* d_perm,
-              double* d_b, int nrhs, int ldb) {
+              double* d_b, int nrhs, int ldb, const alg::DevStatus* guard) {
   if (update == ALG_UPDATE_EXACT)
-    return alg::lu_solve_dev<double, true>(ctx, d_lu, n, lda, d_perm, d_b, nrhs, ldb);
-  return alg::lu_solve_dev<double, false>(ctx, d_lu, n, lda, d_perm, d_b, nrhs, ldb);
+    return alg::lu_solve_dev<double, true>(ctx, d_lu, n, lda, d_perm, d_b, nrhs, ldb, guard);
+  return alg::lu_solve_dev<double, false>(ctx, d_lu, n, lda, d_perm, d_b, nrhs, ldb, guard);
 }
 
 // Sizes accepted by the int32-indexed kernels.
@@ -670,13 +674,11 @@ int host_lu(int update, double* a, size_t m, size_t nc, size_t* ipiv, double* de
   if (d_b) ALG_CUDA_TRY(cudaMemcpyAsync(d_b, b, sizeof(double) * m * nrhs, cudaMemcpyHostToDevice, ctx->stream));
   ALG_TRY(alg::status_reset(ctx));
   ALG_TRY(factor_any(ctx, update, d_a, M, N, M, d_ipiv, d_perm));
-  ALG_TRY(alg::status_fetch(ctx));
+  if (d_b) ALG_TRY(solve_any(ctx, update, d_a, M, M, d_perm, d_b, R, M, ctx->d_status));
+  ALG_TRY(alg::status_fetch(ctx));  // a timed-out sweep is an error, not a result
   const bool singular = ctx->h_status->singular_col != INT_MAX;
-  if (!singular && d_b) {
-    ALG_TRY(solve_any(ctx, update, d_a, M, M, d_perm, d_b, R, M));
-    ALG_TRY(alg::status_fetch(ctx));  // a timed-out sweep is an error, not a result
+  if (!singular && d_b)
     ALG_CUDA_TRY(cudaMemcpyAsync(b, d_b, sizeof(double) * m * nrhs, cudaMemcpyDeviceToHost, ctx->stream));
-  }
   ALG_CUDA_TRY(cudaMemcpyAsync(a, d_a, sizeof(double) * m * nc, cudaMemcpyDeviceToHost, ctx->stream));
   std::vector<int> h_ipiv(nc);
   ALG_CUDA_TRY(cudaMemcpyAsync(h_ipiv.data(), d_ipiv, sizeof(int) * nc, cudaMemcpyDeviceToHost, ctx->stream));
@@ -864,7 +866,7 @@ int alg_dgetrs_dev(alg_ctx* ctx, const double* d_lu, int n, int lda, const int32
   if (ctx == nullptr || d_perm == nullptr) return ALG_INVALID_ARGUMENT;
   if (n < 0 || nrhs < 0 || lda < std::max(1, n) || ldb < std::max(1, n)) return ALG_BAD_SHAPE;
   ALG_TRY(alg::status_reset(ctx));
-  ALG_TRY(solve_any(ctx, ALG_UPDATE_EXACT, d_lu, n, lda, d_perm, d_b, nrhs, ldb));
+  ALG_TRY(solve_any(ctx, ALG_UPDATE_EXACT, d_lu, n, lda, d_perm, d_b, nrhs, ldb, nullptr));
   return alg::status_fetch(ctx);  // synchronises; reports a timed-out sweep
 }
 
@@ -880,10 +882,9 @@ int alg_dgesv_dev(alg_ctx* ctx, int update, double* d_a, int n, int lda, double*
   ALG_TRY(alg::ws_get(ctx, alg::WS_PERM, sizeof(int) * n, reinterpret_cast<void**>(&perm)));
   ALG_TRY(alg::status_reset(ctx));
   ALG_TRY(factor_any(ctx, update, d_a, n, n, lda, ipiv, perm));
-  ALG_TRY(alg::status_fetch(ctx));
-  if (ctx->h_status->singular_col != INT_MAX) return ALG_SINGULAR;
-  ALG_TRY(solve_any(ctx, update, d_a, n, lda, perm, d_b, nrhs, ldb));
-  return alg::status_fetch(ctx);  // synchronises; reports a timed-out sweep
+  ALG_TRY(solve_any(ctx, update, d_a, n, lda, perm, d_b, nrhs, ldb, ctx->d_status));
+  ALG_TRY(alg::status_fetch(ctx));  // synchronises; reports a timed-out sweep
+  return ctx->h_status->singular_col != INT_MAX ? ALG_SINGULAR : ALG_OK;
 }
 
 }  // extern "C"

@@ -57,14 +57,21 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
                           const LuPlan& plan);
 
 // Solves with the packed factors: b (n x nrhs, ldb) becomes x. Stream-ordered.
+// guard (may be null): the status block of the factorization; when that failed,
+// b stays as it is.
 template <typename T, bool EXACT>
 int lu_solve_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs,
-                 int ldb);
+                 int ldb, const DevStatus* guard = nullptr);
 
 // Same contract as lu_solve_dev: gather by perm, then the forward and
 // backward sweeps as single dataflow launches (trsv.cu).
 template <typename T, bool EXACT>
-int lu_solve_dataflow_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb);
+int lu_solve_dataflow_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb,
+                          const DevStatus* guard = nullptr);
+
+// b (n x nrhs, ldb) <- x (n x nrhs, ld n); with a guard, only when its factorization succeeded.
+template <typename T>
+int store_solution_dev(alg_ctx* ctx, const T* x, int n, int nrhs, T* b, int ldb, const DevStatus* guard);
 
 // FP64 C -= A B on the FP64 tensor cores (mma.sync m8n8k4), fused arithmetic;
 // column-major, any leading dimensions, stream-ordered.

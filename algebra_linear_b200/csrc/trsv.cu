@@ -19,6 +19,7 @@
 #include <climits>
 
 #include "dense.cuh"
+#include "pivot.cuh"
 
 namespace alg {
 namespace {
@@ -28,9 +29,6 @@ constexpr int kTThreads = 256;  // 64 rows x 4 column quarters
 constexpr int kMaxRhs = 4;      // right-hand sides handled per pass
 template <typename T>
 constexpr size_t kTSmem = 4 * kTB * kTB * sizeof(T);  // two factor tiles, the diagonal block, its inverse
-
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
   int v;
@@ -66,13 +64,15 @@ __device__ __forceinline__ void prefetch_tile(T* tile, const T* lu, int lda, int
 // another CTA aborted or the limit ran out (then this CTA raises the abort
 // flag and the status block's timeout, so every CTA of the launch returns).
 __device__ __forceinline__ int wait_ready(const int* flag, int* abort_flag, DevStatus* status, uint64_t limit_ns) {
+  // (the abort flag and the timer are looked at every 16th poll only: a poll
+  // is a round trip to L2, and most waits end within a few)
   uint64_t t0 = 0;
-  for (int it = 0;; ++it) {
+  for (int it = 1;; ++it) {
     if (ld_acquire(flag) != 0) return 1;
-    if (ld_acquire(abort_flag) != 0) return 0;
-    if ((it & 255) == 0) {
+    if ((it & 15) == 0) {
+      if (ld_acquire(abort_flag) != 0) return 0;
       const uint64_t now = global_timer_ns();
-      if (it == 0) {
+      if (t0 == 0) {
         t0 = now;
       } else if (now - t0 > limit_ns) {
         atomicExch(abort_flag, 1);
@@ -80,6 +80,57 @@ __device__ __forceinline__ int wait_ready(const int* flag, int* abort_flag, DevS
         return 0;
       }
     }
+  }
+}
+
+// The diagonal block of an exact sweep by one warp: lane l holds rows l and
+// l + 32 of every right-hand side; step c's solved entry is broadcast by a
+// shuffle and subtracted as a rounded product from the rows that follow (the
+// reference's order, mod.rs:341-353), the upper sweep's quotient correctly
+// rounded from the reciprocal formed beforehand. About 50 (lower) and 75
+// (upper) cycles a step; through shared memory with a division per step it
+// was 150 and 330.
+template <typename T, bool UPPER>
+__device__ __forceinline__ void exact_diag(const T* dtile, const T* drec, T (*acc_s)[kMaxRhs], int rows, int nrhs) {
+  const int lane = threadIdx.x & 31;
+  for (int k = 0; k < nrhs; ++k) {
+    T v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) v[h] = lane + 32 * h < rows ? acc_s[lane + 32 * h][k] : T(0);
+    if constexpr (!UPPER) {
+#pragma unroll
+      for (int hc = 0; hc < 2; ++hc) {
+        const int ce = min(32, rows - 32 * hc);
+#pragma unroll 8
+        for (int c = 0; c < ce; ++c) {
+          const T* col = dtile + (32 * hc + c) * kTB + lane;
+          const T u = __shfl_sync(0xffffffffu, v[hc], c);
+          if (lane > c) v[hc] = msub<true>(v[hc], col[32 * hc], u);
+          if (hc == 0) v[1] = msub<true>(v[1], col[32], u);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int hc = 1; hc >= 0; --hc) {
+        const int ce = min(32, rows - 32 * hc);
+        const T y = 32 * hc + lane < rows ? drec[32 * hc + lane] : T(0);
+        const T d = 32 * hc + lane < rows ? dtile[(32 * hc + lane) * (kTB + 1)] : T(1);
+#pragma unroll 8
+        for (int c = ce - 1; c >= 0; --c) {
+          const T* col = dtile + (32 * hc + c) * kTB + lane;
+          const T qv = mul_rn(v[hc], y);
+          T q = fma_rn(fma_rn(-qv, d, v[hc]), y, qv);
+          if (lane == c && !(y != T(0) && exp_fast_ok(v[hc]))) q = div_rn(v[hc], d);
+          if (lane == c) v[hc] = q;
+          const T u = __shfl_sync(0xffffffffu, v[hc], c);
+          if (lane < c) v[hc] = msub<true>(v[hc], col[32 * hc], u);
+          if (hc == 1) v[0] = msub<true>(v[0], col[0], u);
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (lane + 32 * h < rows) acc_s[lane + 32 * h][k] = v[h];
   }
 }
 
@@ -98,6 +149,7 @@ __global__ void __launch_bounds__(kTThreads) trsv_dataflow_kernel(const T* __res
   __shared__ T xs[kTB][kMaxRhs];       // x of the block being consumed
   __shared__ T part[4][kTB][kMaxRhs];  // partial sums of the four column quarters
   __shared__ T acc_s[kTB][kMaxRhs];
+  __shared__ T drec[kTB];  // EXACT, upper: reciprocals of the diagonal (0: divide plainly)
   __shared__ int stop;
   const int nb = (n + kTB - 1) / kTB;
   const int r = threadIdx.x & (kTB - 1);  // row within the block
@@ -147,6 +199,14 @@ __global__ void __launch_bounds__(kTThreads) trsv_dataflow_kernel(const T* __res
             xcol[rr] = -div_rn(acc, dtile[rr * kTB + rr]);
           }
         }
+      }
+    }
+    if constexpr (EXACT && UPPER) {
+      cp_async_wait<1>();
+      __syncthreads();
+      if (threadIdx.x < rows) {
+        const T d = dtile[threadIdx.x * kTB + threadIdx.x];
+        drec[threadIdx.x] = exp_fast_ok(d) ? rcp_rn(d) : T(0);
       }
     }
     __syncthreads();
@@ -219,33 +279,19 @@ __global__ void __launch_bounds__(kTThreads) trsv_dataflow_kernel(const T* __res
       if (qt == 0 && r < rows)
         for (int k = 0; k < nrhs; ++k)
           acc_s[r][k] = (part[0][r][k] + part[1][r][k]) + (part[2][r][k] + part[3][r][k]);
-    } else if (threadIdx.x < 32) {
-      for (int k = 0; k < nrhs; ++k) {
-        if constexpr (!UPPER) {
-          for (int c = 0; c + 1 < rows; ++c) {
-            const T u = acc_s[c][k];
-            for (int ii = c + 1 + threadIdx.x; ii < rows; ii += 32)
-              acc_s[ii][k] = msub<EXACT>(acc_s[ii][k], dtile[c * kTB + ii], u);
-            __syncwarp();
-          }
-        } else {
-          for (int c = rows - 1; c >= 0; --c) {
-            if (threadIdx.x == 0) acc_s[c][k] = div_rn(acc_s[c][k], dtile[c * kTB + c]);
-            __syncwarp();
-            const T u = acc_s[c][k];
-            for (int ii = threadIdx.x; ii < c; ii += 32) acc_s[ii][k] = msub<EXACT>(acc_s[ii][k], dtile[c * kTB + ii], u);
-            __syncwarp();
-          }
-        }
-      }
+    }
+    if constexpr (EXACT) {
+      if (threadIdx.x < 32) exact_diag<T, UPPER>(dtile, drec, acc_s, rows, nrhs);
     }
     __syncthreads();
-    if (qt == 0 && r < rows)
-      for (int k = 0; k < nrhs; ++k) x[(size_t)k * ldx + i0 + r] = acc_s[r][k];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();  // cumulative: the block's stores, ordered by the barrier, before the flag
-      st_release(&flags[bi], 1);
+    if (threadIdx.x < 64) {  // two warps store the block, one of them releases it
+      if (r < rows)
+        for (int k = 0; k < nrhs; ++k) x[(size_t)k * ldx + i0 + r] = acc_s[r][k];
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+      if (threadIdx.x == 0) {
+        __threadfence();  // cumulative: the block's stores, ordered by the barrier, before the flag
+        st_release(&flags[bi], 1);
+      }
     }
   }
 }
@@ -263,7 +309,6 @@ int launch_trsv(alg_ctx* ctx, const T* lu, int lda, int n, T* x, int ldx, int nr
     max_blocks = std::max(1, per_sm) * ctx->sm_count;
   }
   int grid = std::min(nb, max_blocks);
-  ALG_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (nb + 1), ctx->stream));
   uint64_t limit = ctx->wait_limit_ns ? ctx->wait_limit_ns : kWaitLimitNs;
   int stuck = 0;
   if (ctx->stuck_waits > 0) {
@@ -278,16 +323,12 @@ int launch_trsv(alg_ctx* ctx, const T* lu, int lda, int n, T* x, int ldx, int nr
   return ALG_OK;
 }
 
-__global__ void gather_rows_kernel_d(const double* __restrict__ b, int ldb, const int* __restrict__ perm, int n,
-                                     int nrhs, double* __restrict__ x, int ldx) {
-  const size_t cnt = (size_t)n * nrhs;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += (size_t)gridDim.x * blockDim.x) {
-    const size_t k = idx / n, i = idx % n;
-    x[k * ldx + i] = b[k * ldb + perm[i]];
-  }
-}
-__global__ void gather_rows_kernel_f(const float* __restrict__ b, int ldb, const int* __restrict__ perm, int n,
-                                     int nrhs, float* __restrict__ x, int ldx) {
+// x[:, k] = b[perm, k]; with `guard`, nothing when the factorization it reports
+// on failed (a row order from a timed-out one is not used as an index).
+template <typename T>
+__global__ void gather_rows_kernel(const T* __restrict__ b, int ldb, const int* __restrict__ perm, int n, int nrhs,
+                                   T* __restrict__ x, int ldx, const DevStatus* guard) {
+  if (guard != nullptr && factor_failed(guard)) return;
   const size_t cnt = (size_t)n * nrhs;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += (size_t)gridDim.x * blockDim.x) {
     const size_t k = idx / n, i = idx % n;
@@ -296,20 +337,49 @@ __global__ void gather_rows_kernel_f(const float* __restrict__ b, int ldb, const
 }
 
 template <typename T>
-void gather_rows(alg_ctx* ctx, const T* b, int ldb, const int* perm, int n, int nrhs, T* x, int ldx) {
+void gather_rows(alg_ctx* ctx, const T* b, int ldb, const int* perm, int n, int nrhs, T* x, int ldx,
+                 const DevStatus* guard) {
   const size_t cnt = (size_t)n * nrhs;
   const int g = (int)std::max<size_t>(1, std::min<size_t>((cnt + 255) / 256, (size_t)ctx->sm_count * 8));
-  if constexpr (sizeof(T) == 8) gather_rows_kernel_d<<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x, ldx);
-  else gather_rows_kernel_f<<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x, ldx);
+  gather_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x, ldx, guard);
   count_launches();
+}
+
+template <typename T>
+__global__ void store_solution_kernel(const T* __restrict__ x, int n, int nrhs, T* __restrict__ b, int ldb,
+                                      const DevStatus* guard) {
+  if (factor_failed(guard)) return;
+  const size_t cnt = (size_t)n * nrhs;
+  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += (size_t)gridDim.x * blockDim.x)
+    b[(idx / n) * ldb + idx % n] = x[idx];
 }
 
 }  // namespace
 
+// b (n x nrhs, ldb) <- x (n x nrhs, ld n), with `guard` only when the
+// factorization it reports on succeeded.
+template <typename T>
+int store_solution_dev(alg_ctx* ctx, const T* x, int n, int nrhs, T* b, int ldb, const DevStatus* guard) {
+  if (guard == nullptr) {
+    ALG_CUDA_TRY(cudaMemcpy2DAsync(b, sizeof(T) * (size_t)ldb, x, sizeof(T) * (size_t)n, sizeof(T) * (size_t)n, nrhs,
+                                   cudaMemcpyDeviceToDevice, ctx->stream));
+    return ALG_OK;
+  }
+  const size_t cnt = (size_t)n * nrhs;
+  const int g = (int)std::max<size_t>(1, std::min<size_t>((cnt + 255) / 256, (size_t)ctx->sm_count * 8));
+  store_solution_kernel<T><<<g, 256, 0, ctx->stream>>>(x, n, nrhs, b, ldb, guard);
+  count_launches();
+  ALG_CUDA_TRY(cudaGetLastError());
+  return ALG_OK;
+}
+template int store_solution_dev<double>(alg_ctx*, const double*, int, int, double*, int, const DevStatus*);
+template int store_solution_dev<float>(alg_ctx*, const float*, int, int, float*, int, const DevStatus*);
+
 // b (n x nrhs, ldb) <- (LU)^{-1} P b, one gather + two dataflow launches per
 // group of up to kMaxRhs right-hand sides.
 template <typename T, bool EXACT>
-int lu_solve_dataflow_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb) {
+int lu_solve_dataflow_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb,
+                          const DevStatus* guard) {
   if (n == 0 || nrhs == 0) return ALG_OK;
   const int nb = (n + kTB - 1) / kTB;
   T* x = nullptr;
@@ -319,16 +389,16 @@ int lu_solve_dataflow_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* 
                  reinterpret_cast<void**>(&flags)));
   int* abort_flag = flags + 2 * nb + 2;
   const int tok = prof_begin(ctx, ALG_K_SOLVE);
-  gather_rows<T>(ctx, b, ldb, perm, n, nrhs, x, n);
-  ALG_CUDA_TRY(cudaMemsetAsync(abort_flag, 0, sizeof(int), ctx->stream));
+  gather_rows<T>(ctx, b, ldb, perm, n, nrhs, x, n, guard);
   for (int k0 = 0; k0 < nrhs; k0 += kMaxRhs) {
+    // both sweeps' flags, and before the first group the abort flag behind them
+    ALG_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)(2 * nb + 2 + (k0 == 0 ? 1 : 0)), ctx->stream));
     const int kr = std::min(kMaxRhs, nrhs - k0);
     T* xk = x + (size_t)k0 * n;
     ALG_TRY((launch_trsv<T, EXACT, false>(ctx, lu, lda, n, xk, n, kr, flags, abort_flag)));
     ALG_TRY((launch_trsv<T, EXACT, true>(ctx, lu, lda, n, xk, n, kr, flags + nb + 1, abort_flag)));
   }
-  ALG_CUDA_TRY(cudaMemcpy2DAsync(b, sizeof(T) * (size_t)ldb, x, sizeof(T) * (size_t)n, sizeof(T) * (size_t)n, nrhs,
-                                 cudaMemcpyDeviceToDevice, ctx->stream));
+  ALG_TRY(store_solution_dev<T>(ctx, x, n, nrhs, b, ldb, guard));
   prof_end(ctx, tok, 2.0 * n * n * nrhs, sizeof(T) * (double(n) * n + 4.0 * n * nrhs));
   return ALG_OK;
 }
@@ -339,15 +409,20 @@ int lu_solve_dataflow_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* 
 template <typename T>
 int tri_solve_dev(alg_ctx* ctx, const T* lu, int lda, int n, T* x, bool upper, int* flags, int* abort_flag) {
   if (n <= 0) return ALG_OK;
+  ALG_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * ((n + kTB - 1) / kTB + 1), ctx->stream));
   if (upper) return launch_trsv<T, false, true>(ctx, lu, lda, n, x, n, 1, flags, abort_flag);
   return launch_trsv<T, false, false>(ctx, lu, lda, n, x, n, 1, flags, abort_flag);
 }
 
 template int tri_solve_dev<double>(alg_ctx*, const double*, int, int, double*, bool, int*, int*);
 template int tri_solve_dev<float>(alg_ctx*, const float*, int, int, float*, bool, int*, int*);
-template int lu_solve_dataflow_dev<double, true>(alg_ctx*, const double*, int, int, const int*, double*, int, int);
-template int lu_solve_dataflow_dev<double, false>(alg_ctx*, const double*, int, int, const int*, double*, int, int);
-template int lu_solve_dataflow_dev<float, false>(alg_ctx*, const float*, int, int, const int*, float*, int, int);
-template int lu_solve_dataflow_dev<float, true>(alg_ctx*, const float*, int, int, const int*, float*, int, int);
+template int lu_solve_dataflow_dev<double, true>(alg_ctx*, const double*, int, int, const int*, double*, int, int,
+    const DevStatus*);
+template int lu_solve_dataflow_dev<double, false>(alg_ctx*, const double*, int, int, const int*, double*, int, int,
+    const DevStatus*);
+template int lu_solve_dataflow_dev<float, false>(alg_ctx*, const float*, int, int, const int*, float*, int, int,
+    const DevStatus*);
+template int lu_solve_dataflow_dev<float, true>(alg_ctx*, const float*, int, int, const int*, float*, int, int,
+    const DevStatus*);
 
 }  // namespace alg
