@@ -496,6 +496,162 @@ __global__ void __launch_bounds__(kSolveThreads) zbackward_kernel(const double2*
   }
 }
 
+// Orders up to this take the shared-memory sweeps below (b and two rows of
+// products on the chip); longer ones the sweeps over global memory.
+constexpr int kSweepMaxN = 4608;
+constexpr int kZsb = 32;  // rows of a block of the unit-lower sweep
+
+// zgesv's interchanges and unit-lower sweep (complex.rs:287-301), one CTA, b
+// in shared memory. Blocks of 32 rows: one warp solves the diagonal block (a
+// row per lane, the solved entry broadcast by a shuffle), then every other
+// row takes the block's 32 terms; each row's terms still arrive in increasing
+// j, each product and difference rounded on its own. The column pipeline it
+// replaces paid a barrier and a round trip to L2 per column, and one thread's
+// interchanges through global memory: n = 777 590 us, 206 us now.
+__global__ void __launch_bounds__(kSolveThreads) zforward_smem_kernel(const double2* __restrict__ lu, int lda, int n,
+                                                                      const int* __restrict__ ipiv, double2* b) {
+  extern __shared__ __align__(16) unsigned char zsm[];
+  double2* bs = reinterpret_cast<double2*>(zsm);  // n
+  double2* tri = bs + n;                          // the diagonal block, [col][row]
+  int* piv = reinterpret_cast<int*>(tri + kZsb * kZsb);
+  const int t = threadIdx.x, lane = t & 31;
+  for (int i = t; i < n; i += kSolveThreads) {
+    bs[i] = b[i];
+    piv[i] = ipiv[i];
+  }
+  __syncthreads();
+  if (t == 0)
+    for (int k = 0; k < n; ++k) {
+      const int p = piv[k];
+      if (p != k) {
+        const double2 x = bs[k];
+        bs[k] = bs[p];
+        bs[p] = x;
+      }
+    }
+  for (int k0 = 0; k0 < n; k0 += kZsb) {
+    const int w = min(kZsb, n - k0);
+    {
+      const int r = t % kZsb, c = t / kZsb;  // kSolveThreads == kZsb * kZsb
+      tri[t] = (r < w && c < w) ? lu[(k0 + r) + (size_t)(k0 + c) * lda] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    if (t < 32) {
+      double2 v = lane < w ? bs[k0 + lane] : make_double2(0.0, 0.0);
+#pragma unroll 8
+      for (int c = 0; c < w; ++c) {
+        const double2 u = make_double2(__shfl_sync(0xffffffffu, v.x, c), __shfl_sync(0xffffffffu, v.y, c));
+        if (lane > c) v = zsub(v, zmul(tri[c * kZsb + lane], u));
+      }
+      if (lane < w) bs[k0 + lane] = v;
+    }
+    __syncthreads();
+    for (int i = k0 + w + t; i < n; i += kSolveThreads) {
+      double2 acc = bs[i];
+      constexpr int kQ = 8;  // entries in flight
+#pragma unroll 1
+      for (int c0 = 0; c0 < w; c0 += kQ) {
+        double2 l[kQ];
+#pragma unroll
+        for (int c = 0; c < kQ; ++c)
+          if (c0 + c < w) l[c] = lu[i + (size_t)(k0 + c0 + c) * lda];
+#pragma unroll
+        for (int c = 0; c < kQ; ++c)
+          if (c0 + c < w) acc = zsub(acc, zmul(l[c], bs[k0 + c0 + c]));
+      }
+      bs[i] = acc;
+    }
+    __syncthreads();
+  }
+  for (int i = t; i < n; i += kSolveThreads) b[i] = bs[i];
+}
+
+// zgesv's upper sweep (complex.rs:304-311), one CTA, b in shared memory. Row
+// i's terms are subtracted in increasing j by one thread, from u_{i,i+1}
+// b_{i+1}, the entry solved last, on: a chain of n^2 / 2 dependent differences
+// (8 cycles each) that nothing shortens without changing the order. All else is
+// kept off it: the other warps form row i - 1's products with the entries
+// already solved while row i is folded, and the folding thread reads its
+// products a batch ahead. n = 777: 2 820 us with products, fold and division
+// in turn, 1 800 us now (the chain alone: 1 270 us).
+constexpr int kZbackThreads = 512;  // 128 registers: the folding thread holds two batches
+
+__global__ void __launch_bounds__(kZbackThreads) zbackward_smem_kernel(const double2* __restrict__ lu, int lda, int n,
+                                                                       double2* b) {
+  extern __shared__ __align__(16) unsigned char zsm[];
+  constexpr int kB = 8;  // products per batch
+  const int np = n + 2 * kB;
+  double2* bs = reinterpret_cast<double2*>(zsm);  // n
+  double2* prod = bs + n;                         // two rows: product j at [j]; raw u_ii at [i], u_{i,i+1} at [i + 1]
+  const int t = threadIdx.x;
+  for (int i = t; i < n; i += kZbackThreads) bs[i] = b[i];
+  for (int i = t; i < 2 * np; i += kZbackThreads) prod[i] = make_double2(0.0, 0.0);
+  __syncthreads();
+  auto products = [&](int i, int first, int step) {  // of row i, by threads first, first + step, ...
+    double2* p = prod + (i & 1) * np;
+#pragma unroll 4
+    for (int j = i + first; j < n; j += step) {
+      const double2 u = lu[i + (size_t)j * lda];
+      p[j] = j <= i + 1 ? u : zmul(u, bs[j]);
+    }
+  };
+  products(n - 1, t, kZbackThreads);
+  __syncthreads();
+  for (int i = n - 1; i >= 0; --i) {
+    if (t == 0) {
+      const double2* p = prod + (i & 1) * np;
+      double2 s = bs[i];
+      if (i + 1 < n) s = zsub(s, zmul(p[i + 1], bs[i + 1]));
+      int j = i + 2;
+      // two batches in turn, the next one's loads issued before this one's
+      // differences (reads past the row's end stay in the padding)
+      double2 q0[kB], q1[kB];
+#pragma unroll
+      for (int u = 0; u < kB; ++u) q0[u] = lds_f64x2(p + min(j, n) + u);
+      for (; j + 2 * kB <= n; j += 2 * kB) {
+#pragma unroll
+        for (int u = 0; u < kB; ++u) q1[u] = lds_f64x2(p + j + kB + u);
+#pragma unroll
+        for (int u = 0; u < kB; ++u) s = zsub(s, q0[u]);
+#pragma unroll
+        for (int u = 0; u < kB; ++u) q0[u] = lds_f64x2(p + j + 2 * kB + u);
+#pragma unroll
+        for (int u = 0; u < kB; ++u) s = zsub(s, q1[u]);
+      }
+#pragma unroll 4
+      for (; j < n; ++j) s = zsub(s, p[j]);
+      bs[i] = zdiv(s, p[i]);
+    } else if (t >= 32 && i > 0) {
+      products(i - 1, t - 32, kZbackThreads - 32);
+    }
+    __syncthreads();
+  }
+  for (int i = t; i < n; i += kZbackThreads) b[i] = bs[i];
+}
+
+int zsolve_dev(alg_ctx* ctx, const double2* lu, int lda, int n, const int* ipiv, double2* b) {
+  if (n <= kSweepMaxN) {
+    const size_t fs = sizeof(double2) * ((size_t)n + kZsb * kZsb) + sizeof(int) * (size_t)n;
+    const size_t bw = sizeof(double2) * ((size_t)n + 2 * ((size_t)n + 16));
+    static const cudaError_t configured = [] {
+      cudaError_t e = cudaFuncSetAttribute(zforward_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           225 * 1024);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(zbackward_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+      return e;
+    }();
+    ALG_CUDA_TRY(configured);
+    zforward_smem_kernel<<<1, kSolveThreads, fs, ctx->stream>>>(lu, lda, n, ipiv, b);
+    zbackward_smem_kernel<<<1, kZbackThreads, bw, ctx->stream>>>(lu, lda, n, b);
+  } else {
+    zforward_kernel<<<1, kSolveThreads, 0, ctx->stream>>>(lu, lda, n, ipiv, b);
+    zbackward_kernel<<<1, kSolveThreads, 0, ctx->stream>>>(lu, lda, n, b);
+  }
+  count_launches(2);
+  ALG_CUDA_TRY(cudaGetLastError());
+  return ALG_OK;
+}
+
 // zgetri (complex.rs:130-158 ztrti2 'Upper' 'Non-unit', then 217-271), in
 // three parts. U is inverted in place in one CTA, column after column: the
 // diagonal becomes 1/u_jj, and row i < j of the column becomes
@@ -640,10 +796,7 @@ int host_zlu(double* a, size_t m, size_t nc, size_t* ipiv, double* b) {
   ALG_TRY(status_fetch(ctx));
   const bool singular = ctx->h_status->singular_col != INT_MAX;
   if (!singular && d_b) {
-    zforward_kernel<<<1, kSolveThreads, 0, ctx->stream>>>(d_a, M, M, d_ipiv, d_b);
-    zbackward_kernel<<<1, kSolveThreads, 0, ctx->stream>>>(d_a, M, M, d_b);
-    count_launches(2);
-    ALG_CUDA_TRY(cudaGetLastError());
+    ALG_TRY(zsolve_dev(ctx, d_a, M, M, d_ipiv, d_b));
     ALG_CUDA_TRY(cudaMemcpyAsync(b, d_b, 2 * sizeof(double) * m, cudaMemcpyDeviceToHost, ctx->stream));
   }
   ALG_CUDA_TRY(cudaMemcpyAsync(a, d_a, abytes, cudaMemcpyDeviceToHost, ctx->stream));
