@@ -520,8 +520,8 @@ constexpr int kBlockedSolveRhs = 16;
 // b (n x nrhs, ldb) <- (LU)^{-1} P b for many right-hand sides (fused
 // arithmetic): the inverses of the 128 x 128 diagonal blocks of L and U
 // (K3i, two launches), the rows gathered by perm, then per block one K3b
-// launch per sweep: X_block <- T_bb^{-1} X_block by every CTA, the rows not
-// yet solved updated by the block's column of the factor. The forward sweep
+// launch per sweep: the rows not yet solved updated by the block's column of
+// the factor, and the next block multiplied by its inverse. The forward sweep
 // reads x1 and writes y into x2; the backward sweep reads x2 and writes x
 // into x1.
 template <typename T>
@@ -537,20 +537,17 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
   T* linv = x2 + (size_t)n * nrhs;
   T* uinv = linv + (size_t)nblk * kb * kb;
   constexpr size_t kInvSmem = sizeof(T) * kb * kb;
-  constexpr int kSolveCols = solve_cols<T>();
-  constexpr size_t kStepSmem = sizeof(T) * (kSolveKb * kSolveKb + kSolveKb * kSolveCols);
+  constexpr size_t kStepSmem = StepCfg<T>::kSmem;
   static const cudaError_t configured = [] {
     cudaError_t e = cudaFuncSetAttribute(tri_block_inverse_kernel<T, false, 4, 2>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(tri_block_inverse_kernel<T, true, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kInvSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(block_solve_step_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kStepSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(block_solve_step_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kStepSmem);
+    for (auto k : {block_solve_step_kernel<T, false, false>, block_solve_step_kernel<T, false, true>,
+                   block_solve_step_kernel<T, true, false>, block_solve_step_kernel<T, true, true>})
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem);
     return e;
   }();
   ALG_CUDA_TRY(configured);
@@ -566,21 +563,29 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
     ALG_CUDA_TRY(cudaGetLastError());
   }
   const int ctiles = (nrhs + kSolveCols - 1) / kSolveCols;
-  for (int k0 = 0; k0 < n; k0 += kb) {  // L y = P b: x1 -> y in x2
-    const int kbe = std::min(kb, n - k0);
-    const int rows = n - (k0 + kbe);
-    const dim3 grid(std::max(1, (rows + kSolveKb - 1) / kSolveKb), ctiles);
-    block_solve_step_kernel<T, false><<<grid, 256, kStepSmem, ctx->stream>>>(
-        lu, lda, n, k0, kbe, linv + (size_t)(k0 / kb) * kb * kb, x1, x2, nrhs);
-    count_launches();
+  // 16-byte copies when the factors' and the workspaces' columns allow them
+  constexpr int kV = 16 / (int)sizeof(T);
+  const bool vec = lda % kV == 0 && n % kV == 0 && (reinterpret_cast<uintptr_t>(lu) & 15) == 0;
+  auto lower = vec ? block_solve_step_kernel<T, false, true> : block_solve_step_kernel<T, false, false>;
+  auto upper = vec ? block_solve_step_kernel<T, true, true> : block_solve_step_kernel<T, true, false>;
+  // L y = P b: x1 -> y in x2 (the first launch forms block 0, launch b updates
+  // by block b and forms block b + 1)
+  lower<<<dim3(1, ctiles), 256, kStepSmem, ctx->stream>>>(lu, lda, n, 0, std::min(kb, n), linv, x1, x2, nrhs, 1);
+  for (int blk = 0; blk + 1 < nblk; ++blk) {
+    const int k0 = blk * kb;
+    const dim3 grid((n - k0 - kb + kb - 1) / kb, ctiles);
+    lower<<<grid, 256, kStepSmem, ctx->stream>>>(lu, lda, n, k0, kb, linv + (size_t)(blk + 1) * kb * kb, x1, x2, nrhs,
+                                                 0);
   }
-  for (int blk = nblk - 1; blk >= 0; --blk) {  // U x = y: x2 -> x in x1
-    const int k0 = blk * kb, kbe = std::min(kb, n - k0);
-    const dim3 grid(std::max(1, (k0 + kSolveKb - 1) / kSolveKb), ctiles);
-    block_solve_step_kernel<T, true><<<grid, 256, kStepSmem, ctx->stream>>>(
-        lu, lda, n, k0, kbe, uinv + (size_t)blk * kb * kb, x2, x1, nrhs);
-    count_launches();
+  // U x = y: x2 -> x in x1
+  upper<<<dim3(1, ctiles), 256, kStepSmem, ctx->stream>>>(lu, lda, n, (nblk - 1) * kb, n - (nblk - 1) * kb,
+                                                          uinv + (size_t)(nblk - 1) * kb * kb, x2, x1, nrhs, 1);
+  for (int blk = nblk - 1; blk > 0; --blk) {
+    const int k0 = blk * kb;
+    upper<<<dim3(blk, ctiles), 256, kStepSmem, ctx->stream>>>(lu, lda, n, k0, std::min(kb, n - k0),
+                                                              uinv + (size_t)(blk - 1) * kb * kb, x2, x1, nrhs, 0);
   }
+  count_launches(2 * nblk);
   ALG_CUDA_TRY(cudaGetLastError());
   ALG_TRY(store_solution_dev<T>(ctx, x1, n, nrhs, b, ldb, guard));
   prof_end(ctx, tok, 2.0 * n * n * nrhs, sizeof(T) * (double(n) * n + 4.0 * n * nrhs));

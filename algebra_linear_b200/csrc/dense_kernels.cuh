@@ -1105,100 +1105,157 @@ __global__ void __launch_bounds__(kTrsmThreads, 1) tri_block_inverse_kernel(cons
   }
 }
 
+__device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 // ---------------------------------------------------------------------------
-// K3b: one step of the blocked many-right-hand-side solve, for the block of
-// rows [k0, k0 + kbe): every CTA forms X_new = T_bb^{-1} X[k0:k0+kbe, tile]
-// (the block's inverse from K3i; CTA x = 0 stores it in Y), then updates its
-// 128 rows of the rows not yet solved, X[rows, tile] -= T[rows, k0:k0+kbe]
-// X_new (lower: the rows below the block; upper: the rows above). A tile of
-// 128 rows x solve_cols<T>() right-hand sides per CTA, the operands in
-// shared memory (kSolveKb x kSolveKb of the factor, the block rows of X).
-// Rows of X outside [k0, k0 + kbe) are touched only by the CTA that owns
-// them, and X[k0:k0+kbe] is only read in a step, so the CTAs need no sync.
+// K3b: one step of the blocked many-right-hand-side solve. Y[k0:k0+kbe] holds
+// the solved rows of a block; every CTA updates its 128 rows of the rows not
+// yet solved, X[rows, tile] -= T[rows, k0:k0+kbe] Y[k0:k0+kbe, tile] (lower:
+// the rows below the block; upper: the rows above), and the CTA whose rows
+// are the next block goes on to Y[rows, tile] = T_bb^{-1} X[rows, tile] (the
+// block's inverse from K3i). `first`: no update, the block [k0, k0 + kbe)
+// itself is formed. A tile of 128 rows x 32 right-hand sides per CTA, 4 x 4
+// entries per thread; both products read their 128-row operand in chunks of
+// K through one cp.async ring, so the inverse arrives during the update. (Every
+// CTA forming the block's solution for itself, operands whole in shared
+// memory: 33 us a step, FP32, 64 right-hand sides, n = 5 000; 16 us now.)
 // ---------------------------------------------------------------------------
 constexpr int kSolveKb = 128;
-// right-hand sides per CTA: 32 in FP32 (two CTAs per SM), 64 in FP64 (one);
-// a thread takes 8 rows x kSolveCols / 16 of them
-template <typename T>
-constexpr int solve_cols() { return sizeof(T) == 4 ? 32 : 64; }
+constexpr int kSolveCols = 32;  // right-hand sides per CTA
 
-template <typename T, bool UPPER>
+template <typename T>
+struct StepCfg {
+  static constexpr int kV = 16 / (int)sizeof(T);
+  static constexpr int kKC = 8 * kV, kStages = 3;  // K per chunk
+  static constexpr int kBS = kKC + kV;             // row stride of the Y chunk, [c][k]
+  static constexpr int kXS = kSolveKb + kV;        // row stride of the block's X, [c][k]
+  static constexpr int kStage = kKC * kSolveKb + kSolveCols * kBS;
+  static constexpr size_t kSmem = sizeof(T) * (kStages * kStage + kSolveCols * kXS);
+};
+
+template <typename T, bool UPPER, bool VEC>
 __global__ void __launch_bounds__(256) block_solve_step_kernel(const T* __restrict__ lu, int lda, int n, int k0,
-                                                               int kbe, const T* __restrict__ inv, T* x,
-                                                               T* __restrict__ y, int nrhs) {
-  constexpr int kSolveCols = solve_cols<T>(), kSolveTc = kSolveCols / 16;
+                                                               int kbe, const T* __restrict__ inv, T* __restrict__ x,
+                                                               T* __restrict__ y, int nrhs, int first) {
+  using Cfg = StepCfg<T>;
+  constexpr int kV = Cfg::kV, kKC = Cfg::kKC, kStages = Cfg::kStages, kBS = Cfg::kBS, kXS = Cfg::kXS;
+  struct alignas(16) Vec {
+    T e[kV];
+  };
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* As = reinterpret_cast<T*>(smem_raw);  // [k][i], kSolveKb x kSolveKb
-  T* Xs = As + kSolveKb * kSolveKb;        // [k][c], kSolveKb x kSolveCols
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  T* ring = reinterpret_cast<T*>(smem_raw);
+  T* Xs = ring + kStages * Cfg::kStage;
+  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
   const int c0 = blockIdx.y * kSolveCols;
   const int nc = min(kSolveCols, nrhs - c0);
-  const int ur0 = UPPER ? 0 : k0 + kbe, ur1 = UPPER ? k0 : n;
-  const int rt = ur0 + blockIdx.x * kSolveKb;  // this CTA's first update row
-  for (int e = tid; e < kSolveKb * kSolveKb; e += 256) {
-    const int i = e % kSolveKb, k = e / kSolveKb;
-    As[e] = (i < kbe && k < kbe) ? inv[i + (size_t)k * kSolveKb] : T(0);
+  // this CTA's rows; CTA x = 0 has the next block's
+  int r0, r1;
+  if (first) {
+    r0 = k0, r1 = k0 + kbe;
+  } else if (UPPER) {
+    r1 = k0 - blockIdx.x * kSolveKb, r0 = r1 - kSolveKb;
+  } else {
+    r0 = k0 + kbe + blockIdx.x * kSolveKb, r1 = min(n, r0 + kSolveKb);
   }
-  for (int e = tid; e < kSolveKb * kSolveCols; e += 256) {
-    const int c = e % kSolveCols, k = e / kSolveCols;
-    Xs[e] = (k < kbe && c < nc) ? x[(size_t)(k0 + k) + (size_t)(c0 + c) * n] : T(0);
-  }
-  __syncthreads();
-  T acc[8][kSolveTc];
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < kSolveTc; ++c) acc[r][c] = T(0);
-  for (int k = 0; k < kbe; ++k) {
-    T av[8], bv[kSolveTc];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) av[r] = As[k * kSolveKb + tx + 16 * r];
-#pragma unroll
-    for (int c = 0; c < kSolveTc; ++c) bv[c] = Xs[k * kSolveCols + ty * kSolveTc + c];
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-      for (int c = 0; c < kSolveTc; ++c) acc[r][c] = fma_rn(av[r], bv[c], acc[r][c]);
-  }
-  __syncthreads();  // every thread is done with X_old
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < kSolveTc; ++c) {
-      const int i = tx + 16 * r, cc = ty * kSolveTc + c;
-      Xs[i * kSolveCols + cc] = acc[r][c];
-      if (blockIdx.x == 0 && i < kbe && cc < nc) y[(size_t)(k0 + i) + (size_t)(c0 + cc) * n] = acc[r][c];
+  const int nr = r1 - r0;
+  const int nch1 = first ? 0 : (kbe + kKC - 1) / kKC;
+  const int nch = nch1 + (blockIdx.x == 0 ? (nr + kKC - 1) / kKC : 0);
+
+  auto copy = [&](T* dst, const T* src, int count) {  // kV entries (VEC) or one; count of them valid
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (VEC)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src),
+                   "r"(max(0, min(kV, count)) * (int)sizeof(T)) : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(sizeof(T)),
+                   "r"(count > 0 ? (int)sizeof(T) : 0) : "memory");
+  };
+  constexpr int P = VEC ? kV : 1;
+  auto load_chunk = [&](int ch) {
+    T* As = ring + (ch % kStages) * Cfg::kStage;  // [k][i]
+    T* Bs = As + kKC * kSolveKb;                  // [c][k]
+    const bool upd = ch < nch1;
+    const int kc = (upd ? ch : ch - nch1) * kKC;
+#pragma unroll 4
+    for (int e = tid; e < kKC * kSolveKb / P; e += 256) {
+      const int i = P * (e % (kSolveKb / P)), k = e / (kSolveKb / P);
+      if (upd) {
+        const int cnt = kc + k < kbe ? nr - i : 0;
+        copy(As + k * kSolveKb + i, cnt > 0 ? lu + (size_t)(r0 + i) + (size_t)(k0 + kc + k) * lda : lu, cnt);
+      } else {  // the inverse is padded with zeros to kSolveKb x kSolveKb
+        copy(As + k * kSolveKb + i, inv + i + (size_t)(kc + k) * kSolveKb, kV);
+      }
     }
-  if (rt >= ur1) return;  // no rows left to update (uniform over the CTA)
-  for (int e = tid; e < kSolveKb * kSolveKb; e += 256) {
-    const int i = e % kSolveKb, k = e / kSolveKb;
-    As[e] = (rt + i < ur1 && k < kbe) ? lu[(size_t)(rt + i) + (size_t)(k0 + k) * lda] : T(0);
+    if (upd)
+      for (int e = tid; e < kSolveCols * kKC / P; e += 256) {
+        const int k = P * (e % (kKC / P)), c = e / (kKC / P);
+        const int cnt = c < nc ? kbe - (kc + k) : 0;
+        copy(Bs + c * kBS + k, cnt > 0 ? y + (size_t)(k0 + kc + k) + (size_t)(c0 + c) * n : y, cnt);
+      }
+  };
+#pragma unroll
+  for (int st = 0; st < kStages - 1; ++st) {
+    if (st < nch) load_chunk(st);
+    cp_async_commit_group();
   }
+  T acc[4][4];
 #pragma unroll
-  for (int r = 0; r < 8; ++r)
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int c = 0; c < kSolveTc; ++c) {
-      const int i = rt + tx + 16 * r, cc = ty * kSolveTc + c;
-      acc[r][c] = (i < ur1 && cc < nc) ? x[(size_t)i + (size_t)(c0 + cc) * n] : T(0);
+    for (int r = 0; r < 4; ++r) {
+      const int i = tx + 32 * r, cc = ty * 4 + c;
+      acc[r][c] = (i < nr && cc < nc) ? x[(size_t)(r0 + i) + (size_t)(c0 + cc) * n] : T(0);
     }
-  __syncthreads();
-  for (int k = 0; k < kbe; ++k) {
-    T av[8], bv[kSolveTc];
+  for (int ch = 0; ch < nch; ++ch) {
+    cp_async_wait_group<kStages - 2>();
+    if (ch == nch1) {  // the block's rows are final: on to its inverse
 #pragma unroll
-    for (int r = 0; r < 8; ++r) av[r] = As[k * kSolveKb + tx + 16 * r];
+      for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int c = 0; c < kSolveTc; ++c) bv[c] = Xs[k * kSolveCols + ty * kSolveTc + c];
+        for (int r = 0; r < 4; ++r) {
+          Xs[(ty * 4 + c) * kXS + tx + 32 * r] = acc[r][c];
+          acc[r][c] = T(0);
+        }
+    }
+    __syncthreads();  // chunk ch is here for every thread, and chunk ch - 1's stage is free
+    if (ch + kStages - 1 < nch) load_chunk(ch + kStages - 1);
+    cp_async_commit_group();
+    const bool upd = ch < nch1;
+    const T* As = ring + (ch % kStages) * Cfg::kStage;
+    const T* Bs = upd ? As + kKC * kSolveKb : Xs + (ch - nch1) * kKC;
+    const int bs = upd ? kBS : kXS;
+#pragma unroll 2
+    for (int k = 0; k < kKC; k += kV) {
+      Vec bv[4];
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+      for (int c = 0; c < 4; ++c) bv[c] = *reinterpret_cast<const Vec*>(Bs + (ty * 4 + c) * bs + k);
 #pragma unroll
-      for (int c = 0; c < kSolveTc; ++c) acc[r][c] = msub<false>(acc[r][c], av[r], bv[c]);
+      for (int q = 0; q < kV; ++q) {
+        T av[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const T v = As[(k + q) * kSolveKb + tx + 32 * r];
+          av[r] = upd ? -v : v;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[r][c] = fma_rn(av[r], bv[c].e[q], acc[r][c]);
+      }
+    }
   }
+  cp_async_wait_group<0>();
+  T* out = blockIdx.x == 0 ? y : x;
 #pragma unroll
-  for (int r = 0; r < 8; ++r)
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int c = 0; c < kSolveTc; ++c) {
-      const int i = rt + tx + 16 * r, cc = ty * kSolveTc + c;
-      if (i < ur1 && cc < nc) x[(size_t)i + (size_t)(c0 + cc) * n] = acc[r][c];
+    for (int r = 0; r < 4; ++r) {
+      const int i = tx + 32 * r, cc = ty * 4 + c;
+      if (i < nr && cc < nc) out[(size_t)(r0 + i) + (size_t)(c0 + cc) * n] = acc[r][c];
     }
 }
 
@@ -1230,12 +1287,6 @@ __global__ void gather_perm_rows_kernel(const T* __restrict__ b, int ldb, const 
 // also asks L2 for the C tile its slot takes next. Bound by the FP64 (FP32)
 // pipe. Measured: see the table at gemm_sub_dev.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 template <typename T, int NJ>
 struct SubCfg {
   static constexpr int kBM = 64, kBN = 8 * NJ, kBK = 16, kThreads = 128, kStages = 3;
