@@ -11,6 +11,7 @@
 //       K3 trsm (w rows)          : U of its rows
 //       K4 gemm (k = w)           : the rows below
 //     K2 laswp_outside            : the block-panel's interchanges, all other columns
+//                                   (left of the block: at the end, K2c/K2p)
 //     K3 trsm (kb rows)           : U12 = L11^{-1} A12
 //     K4 gemm (k = kb)            : A22 -= L21 U12
 // Every entry sees its rank-1 terms in increasing pivot order, so with the
@@ -339,29 +340,58 @@ int tc_chain_ctas() {
   return v;
 }
 
+// Shared memory of permute_left_kernel: every FP64 column (a panel takes up to
+// 22 000 rows) and FP32 columns of up to 57 000 rows.
+constexpr size_t kPermSmem = 224 * 1024;
+bool left_at_end(int m, int nb, size_t elem_bytes) { return elem_bytes * (size_t)std::max(0, m - nb) <= kPermSmem; }
+
+size_t lu_label_bytes(int m, int nc, int nb, size_t elem_bytes) {
+  const size_t nblk = ((size_t)nc + nb - 1) / nb;
+  const bool at_end = lookahead_enabled() && nc > 2 * nb && left_at_end(m, nb, elem_bytes);
+  return sizeof(int) * (size_t)m * (at_end ? 2 * nblk - 1 : 2);
+}
+
 template <typename T, bool EXACT>
 int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, int* ipiv, int* perm,
                           const LuPlan& plan) {
   if (m < nc || nc < 0 || ntot < nc || lda < std::max(1, m)) return ALG_BAD_SHAPE;
   if (nc == 0) return ALG_OK;
-  int* lab = nullptr;  // two label buffers: block k's swaps are applied while block k + 1 is factored
+  // a block's interchanges move at most 2 nb rows, and the deferred-swap
+  // kernel holds kSwapMaxMoves of them: wider blocks are cut to that
+  const int nb = std::min(std::max(1, plan.nb), kSwapMaxMoves / 2);
+  const int nbl = std::max(1, std::min(plan.nbl, kPanelMaxW));
+  // (with two blocks there is nothing beside the chain: one stream saves the
+  // events and a swap launch, n = 96: 174 us against 180 us)
+  const bool la = lookahead_enabled() && nc > 2 * nb;
+  const int nblk = (nc + nb - 1) / nb;
+  // With look-ahead the columns left of the blocks are permuted once at the
+  // end, from every block's labels, when a column fits in shared memory and
+  // the labels (8 m bytes per block, 1/128 of an FP64 matrix) in memory
+  // (n = 16384: FP64 131.1 -> 126.2 ms, mixed 59.0 -> 56.0 ms; a block's
+  // swaps of the columns on its left took 55 us, their sum 7.3 ms, and the
+  // permutation at the end takes 0.8 ms).
+  // Otherwise, block by block: two label buffers, since block k's swaps are
+  // applied while block k + 1 is factored.
+  int* lab = nullptr;
+  bool at_end = la && left_at_end(m, nb, sizeof(T));
+  if (at_end) {
+    at_end = ws_get(ctx, WS_LAB, lu_label_bytes(m, nc, nb, sizeof(T)), reinterpret_cast<void**>(&lab)) == ALG_OK;
+    if (!at_end) cudaGetLastError();
+  }
+  if (!at_end) ALG_TRY(ws_get(ctx, WS_LAB, 2 * sizeof(int) * (size_t)m, reinterpret_cast<void**>(&lab)));
+  int* comp = lab + (size_t)nblk * m;  // (at_end)
   int* perm_tmp = nullptr;
-  ALG_TRY(ws_get(ctx, WS_LAB, 2 * sizeof(int) * (size_t)m, reinterpret_cast<void**>(&lab)));
   ALG_TRY(ws_get(ctx, WS_PERM_TMP, sizeof(int) * kSwapMaxMoves, reinterpret_cast<void**>(&perm_tmp)));
   void* tslu_ws = nullptr;
   if (std::is_same<T, float>::value && plan.tslu) {
     ALG_TRY(ws_get(ctx, WS_TSLU, tslu_scratch_bytes(), &tslu_ws));
     ALG_TRY(tslu_scratch_reset(ctx, tslu_ws));
   }
-  if (perm != nullptr) {
+  if (perm != nullptr && !at_end) {
     iota_kernel<<<std::min(1024, (m + 255) / 256), 256, 0, ctx->stream>>>(perm, m);
     count_launches();
     ALG_CUDA_TRY(cudaGetLastError());
   }
-  // a block's interchanges move at most 2 nb rows, and the deferred-swap
-  // kernel holds kSwapMaxMoves of them: wider blocks are cut to that
-  const int nb = std::min(std::max(1, plan.nb), kSwapMaxMoves / 2);
-  const int nbl = std::max(1, std::min(plan.nbl, kPanelMaxW));
   // persistent tensor-core grids: the wide update's cap (0: every SM) and the
   // look-ahead chain's (its launches must fit on the SMs the wide update
   // leaves free, or their extra CTAs wait for the wide update to retire)
@@ -454,9 +484,6 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
                                   a + (size_t)k0 + (size_t)cb * lda, lda, a + (size_t)kr + (size_t)cb * lda, lda);
   };
 
-  // (with two blocks there is nothing beside the chain: one stream saves the
-  // events and a swap launch, n = 96: 174 us against 180 us)
-  const bool la = lookahead_enabled() && nc > 2 * nb;
   if (!la) {
     for (int k0 = 0; k0 < nc; k0 += nb) {
       const int kb = std::min(nb, nc - k0);
@@ -485,8 +512,8 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
   for (int blk = 0, k0 = 0; rc == ALG_OK && k0 < nc; k0 += nb, ++blk) {
     const int kb = std::min(nb, nc - k0), kr = k0 + kb;
     const int kb1 = kr < nc ? std::min(nb, nc - kr) : 0;
-    int* lk = lab + (size_t)(blk & 1) * m;
-    int* ln = lab + (size_t)((blk + 1) & 1) * m;
+    int* lk = lab + (size_t)(at_end ? blk : blk & 1) * m;
+    int* ln = lab + (size_t)(at_end ? blk + 1 : (blk + 1) & 1) * m;
     // the rest of the update needs block k factored
     if ((rc = cudaEventRecord(ev_a, sa) == cudaSuccess ? ALG_OK : ALG_CUDA_ERROR) != ALG_OK) break;
     if ((rc = cudaStreamWaitEvent(sb, ev_a, 0) == cudaSuccess ? ALG_OK : ALG_CUDA_ERROR) != ALG_OK) break;
@@ -497,7 +524,7 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
       if ((rc = factor_block(kr, kb1, ln)) != ALG_OK) break;
     }
     ctx->stream = sb;
-    if ((rc = swaps(k0, kb, lk, 0, k0, perm)) != ALG_OK) break;
+    if (!at_end && (rc = swaps(k0, kb, lk, 0, k0, perm)) != ALG_OK) break;
     if ((rc = swaps(k0, kb, lk, kr + kb1, ntot, nullptr)) != ALG_OK) break;
     if ((rc = update(k0, kb, kr + kb1, ntot, true)) != ALG_OK) break;
     // block k + 1's swaps touch these columns next
@@ -510,6 +537,17 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
   cudaStreamWaitEvent(sa, ev_b, 0);
   cudaEventRecord(ev_a, sa);
   cudaStreamWaitEvent(user, ev_a, 0);
+  if (at_end && rc == ALG_OK) {
+    static const cudaError_t configured = cudaFuncSetAttribute(
+        permute_left_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPermSmem);
+    ALG_CUDA_TRY(configured);
+    const int tok = prof_begin(ctx, ALG_K_LASWP);
+    compose_swaps_kernel<<<(m + 63) / 64, 64, 0, user>>>(lab, m, nb, nblk, comp, perm);
+    permute_left_kernel<T><<<(nblk - 1) * nb, kPermThreads, sizeof(T) * (size_t)(m - nb), user>>>(a, lda, m, nb, comp);
+    count_launches(2);
+    prof_end(ctx, tok, 0.0, 0.0);
+    ALG_CUDA_TRY(cudaGetLastError());
+  }
   return rc;
 }
 

@@ -56,6 +56,11 @@ template <typename T, bool EXACT>
 int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, int* ipiv, int* perm,
                           const LuPlan& plan);
 
+// Workspace of the row labels of an m-row, nc-column factorization in blocks
+// of nb columns (WS_LAB): callers that factor matrices of growing size reserve
+// the largest first.
+size_t lu_label_bytes(int m, int nc, int nb, size_t elem_bytes);
+
 // Solves with the packed factors: b (n x nrhs, ldb) becomes x. Stream-ordered.
 // guard (may be null): the status block of the factorization; when that failed,
 // b stays as it is.

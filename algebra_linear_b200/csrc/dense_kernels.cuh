@@ -865,6 +865,7 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
 // ---------------------------------------------------------------------------
 constexpr int kSwapThreads = 256;
 constexpr int kSwapMaxMoves = 512;
+constexpr int kSwapScan = 16;  // labels a thread reads per round trip of the scan
 
 template <typename T>
 __global__ void __launch_bounds__(kSwapThreads) laswp_outside_kernel(
@@ -874,11 +875,20 @@ __global__ void __launch_bounds__(kSwapThreads) laswp_outside_kernel(
   __shared__ int mv_cnt;
   if (threadIdx.x == 0) mv_cnt = 0;
   __syncthreads();
-  for (int r = k0 + threadIdx.x; r < n; r += kSwapThreads) {
-    const int s = lab[r];
-    if (s != r) {
-      const int slot = atomicAdd(&mv_cnt, 1);
-      if (slot < kSwapMaxMoves) { mv_dst[slot] = r; mv_src[slot] = s; }
+  for (int r0 = k0 + threadIdx.x; r0 < n; r0 += kSwapScan * kSwapThreads) {
+    int src[kSwapScan];
+#pragma unroll
+    for (int i = 0; i < kSwapScan; ++i) {
+      const int r = r0 + i * kSwapThreads;
+      src[i] = r < n ? lab[r] : r;
+    }
+#pragma unroll
+    for (int i = 0; i < kSwapScan; ++i) {
+      const int r = r0 + i * kSwapThreads;
+      if (src[i] != r) {
+        const int slot = atomicAdd(&mv_cnt, 1);
+        if (slot < kSwapMaxMoves) { mv_dst[slot] = r; mv_src[slot] = src[i]; }
+      }
     }
   }
   __syncthreads();
@@ -912,6 +922,54 @@ __global__ void __launch_bounds__(kSwapThreads) laswp_outside_kernel(
     for (int s = threadIdx.x; s < moves; s += kSwapThreads) perm_tmp[s] = perm[mv_src[s]];
     __syncthreads();
     for (int s = threadIdx.x; s < moves; s += kSwapThreads) perm[mv_dst[s]] = perm_tmp[s];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// K2c / K2p: the interchanges of the columns left of each block, all at once
+// after the last block. Block b's labels lie at lab + b * n; the columns of
+// block b take the interchanges of the blocks b + 1, ..., nblk - 1 one after
+// the other: their row r takes the old content of row
+//   comp_b[r] = lab_{b+1}[... lab_{nblk-1}[r]],
+// which one thread per row follows backwards through the blocks (a block
+// moves rows from its own first one on, so row r starts at block r / nb).
+// comp_b lies at comp + b * n; the chain's last element is the net
+// permutation.
+// A move within a column costs 32 to 64 bytes of DRAM traffic for 4 or 8
+// bytes of data, and one block's interchanges move up to 2 nb rows of every
+// column. Here a column is read and written once, consecutively, with the
+// exchange in shared memory (bound by HBM).
+// ---------------------------------------------------------------------------
+__global__ void compose_swaps_kernel(const int* lab, int n, int nb, int nblk, int* comp, int* perm) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  int s = r;
+  for (int b = min(nblk - 1, r / nb); b >= 0; --b) {
+    const int t = lab[(size_t)b * n + s];
+    s = (unsigned)t < (unsigned)n ? t : s;  // (a panel that timed out may leave a label unset)
+    if (b > 0) comp[(size_t)(b - 1) * n + r] = s;
+  }
+  if (perm != nullptr) perm[r] = s;
+}
+
+constexpr int kPermThreads = 1024;
+
+// One CTA per column; dynamic shared memory: the longest column's moving rows.
+template <typename T>
+__global__ void __launch_bounds__(kPermThreads) permute_left_kernel(T* a, int lda, int n, int nb, const int* comp) {
+  extern __shared__ __align__(16) unsigned char perm_smem[];
+  T* old = reinterpret_cast<T*>(perm_smem);
+  const int c = blockIdx.x, b = c / nb;
+  const int base = (b + 1) * nb, cnt = n - base;
+  T* col = a + (size_t)c * lda + base;
+  const int* src = comp + (size_t)b * n + base;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < cnt; i += kPermThreads) old[i] = col[i];
+  __syncthreads();
+#pragma unroll 8
+  for (int i = threadIdx.x; i < cnt; i += kPermThreads) {
+    const int s = src[i] - base;
+    col[i] = old[(unsigned)s < (unsigned)cnt ? s : i];
   }
 }
 

@@ -1095,6 +1095,15 @@ int zfront_lu(alg_ctx* lc, zc* f, int rows, int size, int cols, int* ipiv, int* 
 
 }  // namespace
 
+// Block width of a large front's LU (ALG_SPLU_NB: measurement switch).
+static int splu_nb() {
+  static const int v = [] {
+    const char* e = std::getenv("ALG_SPLU_NB");
+    return e ? std::max(16, std::atoi(e)) : 64;
+  }();
+  return v;
+}
+
 // ---------------------------------------------------------------------------
 int DeviceLu::init(alg_ctx* c, const FrontPlan* p, int w) {
   ctx = c;
@@ -1147,6 +1156,17 @@ int DeviceLu::init(alg_ctx* c, const FrontPlan* p, int w) {
     ALG_TRY(dmalloc((void**)&d_ipiv[k], sizeof(int) * max_rows));
     ALG_TRY(dmalloc((void**)&d_perm[k], sizeof(int) * max_rows));
     ALG_TRY(dmalloc((void**)&d_rowtmp[k], sizeof(int32_t) * max_rows));
+    if (words == 1) {  // the row labels of the lane's largest front
+      size_t lab = 0;
+      auto front = [&](int32_t s) {
+        lab = std::max(lab, lu_label_bytes(F.fronts[s].rows, F.fronts[s].size, splu_nb(), sizeof(float)));
+      };
+      if (k + 1 < (int)F.lane_ptr.size())
+        std::for_each(F.lane_fronts.begin() + F.lane_ptr[k], F.lane_fronts.begin() + F.lane_ptr[k + 1], front);
+      if (k == 0) std::for_each(F.top_fronts.begin(), F.top_fronts.end(), front);
+      void* p_lab = nullptr;
+      ALG_TRY(ws_get(lane_ctx[k], WS_LAB, lab, &p_lab));
+    }
     if (words == 2)  // 2 rows x 2 kZnb columns of doubles per complex row
       ALG_TRY(dmalloc((void**)&d_zblock[k], sizeof(double) * 4 * kZnb * max_rows));
   }
@@ -1404,17 +1424,12 @@ int DeviceLu::factor_big(int b, int32_t s, int lane, const double* values, int t
     ALG_TRY(zfront_lu(lc, front, d.rows, d.size, cols, d_ipiv[lane], d_perm[lane], d_zblock[lane]));
   } else {
     LuPlan lp;
-    // block width of a large front's LU (ALG_SPLU_NB: measurement switch)
-    static const int splu_nb = [] {
-      const char* e = std::getenv("ALG_SPLU_NB");
-      return e ? std::max(16, std::atoi(e)) : 64;
-    }();
     // leaf-panel width (ALG_SPLU_NBL: measurement switch)
     static const int splu_nbl = [] {
       const char* e = std::getenv("ALG_SPLU_NBL");
       return e ? std::max(1, std::min(32, std::atoi(e))) : 16;
     }();
-    lp.nb = splu_nb;
+    lp.nb = splu_nb();
     lp.nbl = splu_nbl;
     lp.tc_prec = tc_prec;
     if constexpr (std::is_same<T, float>::value) {

@@ -60,6 +60,17 @@ def test_blocks_wider_and_narrower_than_a_launch(gpu, oracle, monkeypatch, nb):
     check(oracle, a, rows, cols)
 
 
+@pytest.mark.parametrize("rows,cols", [(129, 129), (193, 193), (400, 257), (1031, 1031), (22000, 300)])
+def test_left_columns_permuted_at_the_end(gpu, oracle, rows, cols):
+    """Three and more blocks with many interchanges: the columns left of a
+    block are permuted after the last one, from the blocks' composed labels (a
+    last block of one column, square and tall; nearly the most rows an FP64
+    panel takes)."""
+    rng = np.random.default_rng(rows + cols)
+    a = rng.uniform(-1.0, 1.0, (cols, rows)) * rng.permutation(np.geomspace(1.0, 2.0**20, rows))
+    check(oracle, a.reshape(-1).copy(), rows, cols)
+
+
 @pytest.mark.parametrize("lda_off,a_off", [(0, 0), (1, 0), (0, 1)])
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 65, 15), (64, 32, 16), (65, 33, 17), (200, 130, 64), (2100, 2051, 40),
                                    (4200, 1100, 129)])
