@@ -986,73 +986,82 @@ __global__ void iota_kernel(int* v, int n) {
 // CPW whole columns with lane l holding rows l, l + 32, ... in
 // registers; step k broadcasts x_k from its owner lane by a shuffle.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 constexpr int kTrsmThreads = 256;
-// CPW columns per warp: 8 for wide right-hand sides, 2 for narrow ones (more
-// CTAs and a shorter per-step chain when only a block's columns are solved).
+
+// CPW columns per warp, RPT rows per lane (kb <= 32 RPT; L's columns are
+// 32 RPT apart). Bound by the issue of the shuffles and multiply-subtracts
+// with 8 columns, by the chain shuffle -> multiply-subtract with 2.
+// The row group rk of the broadcast is unrolled, so that x_k needs no selection
+// among a lane's rows, and L arrives by asynchronous copies of its lower half.
+// Inside an LU of n = 16384, us per launch of 128 rows, many columns / a
+// block's columns (before: selection by k, L through registers): FP64
+// 66 / 35 -> 30 / 16, FP32 41 / 23 -> 24 / 12; 64 rows of a block's
+// columns, n = 5001 exact: 8.4 -> 5.2.
 template <typename T, bool EXACT, int RPT, int CPW>
 __global__ void __launch_bounds__(kTrsmThreads, 1) trsm_lower_unit_reg_kernel(T* a, int lda, int r0, int kb, int cb,
                                                                            int ce) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* L = reinterpret_cast<T*>(smem_raw);  // kb x kb, column-major
-  constexpr int kWarpCols = CPW;
+  T* L = reinterpret_cast<T*>(smem_raw);
+  constexpr int kLd = 32 * RPT;
   constexpr int kCtaCols = CPW * (kTrsmThreads / 32);
   const int c_first = cb + blockIdx.x * kCtaCols;
   const int ncol = min(kCtaCols, ce - c_first);
   if (ncol <= 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T x[kWarpCols][RPT];
+  // L's strictly lower part (the rest is not read, rows beyond kb to no effect)
+  {
+    const int i = threadIdx.x % kLd;
+    const T* src = a + (size_t)(r0 + i) + (size_t)r0 * lda;
+    if (i < kb)
+      for (int k = threadIdx.x / kLd; k < i; k += kTrsmThreads / kLd) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(L + k * kLd + i);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src + (size_t)k * lda),
+                     "n"(sizeof(T)) : "memory");
+      }
+    cp_async_commit_group();
+  }
+  T x[CPW][RPT];
 #pragma unroll
-  for (int c = 0; c < kWarpCols; ++c) {
-    const int cc = warp * kWarpCols + c;
+  for (int c = 0; c < CPW; ++c) {
+    const int cc = warp * CPW + c;
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const int i = lane + 32 * r;
       x[c][r] = (cc < ncol && i < kb) ? a[(size_t)(r0 + i) + (size_t)(c_first + cc) * lda] : T(0);
     }
   }
-  // L's strictly lower part (the rest is never read), kBatch loads in flight
-  // per thread before any is stored
-  constexpr int kBatch = 16;
-  const int total = kb * kb;
-  for (int base = threadIdx.x; base < total; base += kTrsmThreads * kBatch) {
-    T tmp[kBatch];
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int idx = base + u * kTrsmThreads;
-      const int i = idx % kb, k = idx / kb;
-      tmp[u] = (idx < total && i > k) ? a[(size_t)(r0 + i) + (size_t)(r0 + k) * lda] : T(0);
-    }
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int idx = base + u * kTrsmThreads;
-      if (idx < total) L[idx] = tmp[u];
-    }
-  }
+  cp_async_wait_group<0>();
   __syncthreads();
-  for (int k = 0; k + 1 < kb; ++k) {
-    const int owner = k & 31, rk = k >> 5;
-    T u[kWarpCols];
 #pragma unroll
-    for (int c = 0; c < kWarpCols; ++c) {
-      T xv = x[c][0];
+  for (int rk = 0; rk < RPT; ++rk) {
+    const T* lk = L + (size_t)(32 * rk) * kLd + lane;
+    const int steps = min(32, kb - 1 - 32 * rk);
+#pragma unroll 4
+    for (int kk = 0; kk < steps; ++kk, lk += kLd) {
+      T l[RPT], u[CPW];
 #pragma unroll
-      for (int r = 1; r < RPT; ++r)
-        if (r == rk) xv = x[c][r];
-      u[c] = __shfl_sync(0xffffffffu, xv, owner);
-    }
+      for (int r = rk; r < RPT; ++r) l[r] = lk[32 * r];
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int i = lane + 32 * r;
-      if (i > k && i < kb) {
-        const T l = L[i + (size_t)k * kb];
+      for (int c = 0; c < CPW; ++c) u[c] = __shfl_sync(0xffffffffu, x[c][rk], kk);
+      if (lane > kk) {
 #pragma unroll
-        for (int c = 0; c < kWarpCols; ++c) x[c][r] = msub<EXACT>(x[c][r], l, u[c]);
+        for (int c = 0; c < CPW; ++c) x[c][rk] = msub<EXACT>(x[c][rk], l[rk], u[c]);
       }
+#pragma unroll
+      for (int r = rk + 1; r < RPT; ++r)
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) x[c][r] = msub<EXACT>(x[c][r], l[r], u[c]);
     }
   }
 #pragma unroll
-  for (int c = 0; c < kWarpCols; ++c) {
-    const int cc = warp * kWarpCols + c;
+  for (int c = 0; c < CPW; ++c) {
+    const int cc = warp * CPW + c;
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const int i = lane + 32 * r;
@@ -1163,11 +1172,6 @@ __global__ void __launch_bounds__(kTrsmThreads, 1) tri_block_inverse_kernel(cons
   }
 }
 
-__device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // ---------------------------------------------------------------------------
 // K3b: one step of the blocked many-right-hand-side solve. Y[k0:k0+kbe] holds

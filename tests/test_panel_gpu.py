@@ -60,6 +60,14 @@ def test_blocks_wider_and_narrower_than_a_launch(gpu, oracle, monkeypatch, nb):
     check(oracle, a, rows, cols)
 
 
+@pytest.mark.parametrize("nb,n", [(17, 90), (31, 95), (32, 1200), (33, 150), (65, 200), (97, 1300), (127, 400)])
+def test_triangular_solve_edges(gpu, oracle, monkeypatch, nb, n):
+    """Block rows of every row-group count with ragged last groups, few and
+    many columns right of the block."""
+    monkeypatch.setenv("ALG_NB", str(nb))
+    check(oracle, np.random.default_rng(nb + n).uniform(-1.0, 1.0, n * n), n, n)
+
+
 @pytest.mark.parametrize("rows,cols", [(129, 129), (193, 193), (400, 257), (1031, 1031), (22000, 300)])
 def test_left_columns_permuted_at_the_end(gpu, oracle, rows, cols):
     """Three and more blocks with many interchanges: the columns left of a
