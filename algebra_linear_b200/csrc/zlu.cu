@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "dense.cuh"
+#include "pivot.cuh"
 
 namespace alg {
 namespace {
@@ -74,11 +75,10 @@ constexpr int kPivThreads = 1024;
 // equal rows the first. ipiv[j] is written; a zero (or empty) pivot is
 // recorded in the status block and -1 returned instead. sb and si hold one
 // entry per warp.
-__device__ int zpick_pivot(const double2* __restrict__ col, int m, int j, int* __restrict__ ipiv, DevStatus* st,
-                           double* sb, int* si, int* piv_s) {
+__device__ __forceinline__ int zpick_pivot(const double2* col, int m, int j, int* __restrict__ ipiv, DevStatus* st,
+                                           unsigned long long* sb, int* si) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nt = blockDim.x;
-  // the diagonal's measure, loaded early by the thread that decides
-  const double vj = t == 0 ? zabs1(col[j]) : 0.0;
+  const double vj = zabs1(col[j]);
   // first maximum over this thread's rows below the diagonal; -1 means none
   double best = -1.0;
   int bi = INT_MAX;
@@ -89,58 +89,42 @@ __device__ int zpick_pivot(const double2* __restrict__ col, int m, int j, int* _
       bi = i;
     }
   }
-  // larger value wins, the lower row among equals
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ob = __shfl_down_sync(0xffffffffu, best, off);
-    const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-    if (ob > best || (ob == best && oi < bi)) {
-      best = ob;
-      bi = oi;
-    }
-  }
+  // larger value wins, the lower row among equals (no measure is negative, so
+  // their bits order as integers; none is (0, INT_MAX))
+  unsigned long long mk;
+  int mi;
+  warp_pivot(best < 0.0 ? 0ull : (unsigned long long)__double_as_longlong(best), bi, mk, mi);
   if (lane == 0) {
-    sb[warp] = best;
-    si[warp] = bi;
+    sb[warp] = mk;
+    si[warp] = mi;
   }
   __syncthreads();
-  if (t == 0) {
-    double gb = sb[0];
-    int gi = si[0];
-    for (int w = 1; w < nt / 32; ++w)
-      if (sb[w] > gb || (sb[w] == gb && si[w] < gi)) {
-        gb = sb[w];
-        gi = si[w];
-      }
-    int jp = j;
-    double pbest = vj;
-    if (gi != INT_MAX && gb > vj) {
-      jp = gi;
-      pbest = gb;
-    }
-    if (pbest <= 0.0) {  // ZERO_DETERMINANT = 0.0
-      atomicMin(&st->singular_col, j);
-      jp = -1;
-    } else {
-      ipiv[j] = jp;
-    }
-    *piv_s = jp;
+  warp_pivot(lane < nt / 32 ? sb[lane] : 0ull, lane < nt / 32 ? si[lane] : INT_MAX, mk, mi);
+  const double gb = __longlong_as_double((long long)mk);
+  int jp = j;
+  double pbest = vj;
+  if (mi != INT_MAX && gb > vj) {
+    jp = mi;
+    pbest = gb;
   }
-  __syncthreads();
-  return *piv_s;
+  if (pbest <= 0.0) {  // ZERO_DETERMINANT = 0.0
+    if (t == 0) atomicMin(&st->singular_col, j);
+    return -1;
+  }
+  if (t == 0) ipiv[j] = jp;
+  return jp;
 }
 
 // Step j of the factorization of an m x nc matrix (m >= nc): pivot, swap of
 // the whole rows (all nc columns), scaling of column j below the diagonal.
 __global__ void __launch_bounds__(kPivThreads) zpivot_kernel(double2* __restrict__ a, int lda, int m, int nc, int j,
                                                              int* __restrict__ ipiv, DevStatus* st) {
-  __shared__ double sb[kPivThreads / 32];
+  __shared__ unsigned long long sb[kPivThreads / 32];
   __shared__ int si[kPivThreads / 32];
-  __shared__ int piv_s;
   if (stopped(st)) return;
   const int t = threadIdx.x;
   double2* col = a + (size_t)j * lda;
-  const int jp = zpick_pivot(col, m, j, ipiv, st, sb, si, &piv_s);
+  const int jp = zpick_pivot(col, m, j, ipiv, st, sb, si);
   if (jp < 0) return;
   if (jp != j) {
     for (int k = t; k < nc; k += kPivThreads) {
@@ -192,6 +176,11 @@ __global__ void __launch_bounds__(256) zupdate_kernel(double2* __restrict__ a, i
 // loop leaves on its early return.
 constexpr int kZpw = 16;
 constexpr int kZpanelThreads = 384;
+// A panel of up to 880 rows of 16 columns runs in shared memory (one CTA's
+// chain of pivot search, division and update per column, bound by its latency
+// and the SM's FP64 issue): n = 777, 41 -> 31 us per panel on average; 512
+// threads 32 us, 768 (85 registers, spilled) 41 us.
+constexpr size_t kZpanelSmem = 220 * 1024;
 constexpr int kZtile = 64;
 
 // Steps of the block [k0, k0 + w) that ran: w, fewer when the panel stopped
@@ -222,22 +211,38 @@ __device__ __forceinline__ double2 lds_f64x2(const double2* p) {
   return r;
 }
 
-__global__ void __launch_bounds__(kZpanelThreads) zpanel_kernel(double2* __restrict__ a, int lda, int m, int k0, int w,
-                                                                int* __restrict__ ipiv, DevStatus* st) {
-  __shared__ double sb[kZpanelThreads / 32];
-  __shared__ int si[kZpanelThreads / 32];
-  __shared__ int piv_s;
+template <bool SMEM, int NT>
+__global__ void __launch_bounds__(NT) zpanel_kernel(double2* ga, int glda, int m, int k0, int w,
+                                                    int* __restrict__ ipiv, DevStatus* st) {
+  extern __shared__ double2 ztile[];  // rows [k0, m) of the block's columns (SMEM)
+  __shared__ unsigned long long sb[NT / 32];
+  __shared__ int si[NT / 32];
   __shared__ double2 urow[kZpw];
   __shared__ double2 usub[kZsub][kZpw];  // the sub-panel's rows of U right of it
   if (stopped(st)) return;
   const int t = threadIdx.x, kend = k0 + w;
+  const int rows = m - k0;
+  double2* const gblk = ga + k0 + (size_t)k0 * glda;
+  if constexpr (SMEM) {
+    for (int c = 0; c < w; ++c)
+      for (int i = t; i < rows; i += NT)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(ztile + c * rows + i)),
+                     "l"(gblk + i + (size_t)c * glda)
+                     : "memory");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+  }
+  // entry (i, j) of the matrix at a[i + j * lda]
+  const int lda = SMEM ? rows : glda;
+  double2* const a = SMEM ? ztile - (k0 + k0 * rows) : ga;
   for (int s0 = k0; s0 < kend; s0 += kZsub) {
     const int s1 = min(s0 + kZsub, kend);
     int jv = s1 - s0;  // the sub-panel's steps that ran
 #pragma unroll 1
     for (int j = s0; j < s1; ++j) {
       double2* col = a + (size_t)j * lda;
-      const int jp = zpick_pivot(col, m, j, ipiv, st, sb, si, &piv_s);
+      const int jp = zpick_pivot(col, m, j, ipiv, st, sb, si);
       if (jp < 0) {  // the same for every thread (read from shared memory)
         jv = j - s0;
         break;
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(kZpanelThreads) zpanel_kernel(double2* __restr
       const int jj = j - s0;
       const double2 d = urow[j - k0];
 #pragma unroll 1
-      for (int i = j + 1 + t; i < m; i += kZpanelThreads) {
+      for (int i = j + 1 + t; i < m; i += NT) {
         // the row's entries in the sub-panel's later columns loaded together
         // with the one below the pivot, before any store
         double2* row = a + i + (size_t)s0 * lda;
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(kZpanelThreads) zpanel_kernel(double2* __restr
       }
       __syncthreads();
 #pragma unroll 1
-      for (int i = s1 + t; i < m; i += kZpanelThreads) {
+      for (int i = s1 + t; i < m; i += NT) {
         double2 l[kZsub];
 #pragma unroll
         for (int k = 0; k < kZsub; ++k)
@@ -320,7 +325,11 @@ __global__ void __launch_bounds__(kZpanelThreads) zpanel_kernel(double2* __restr
       }
       __syncthreads();
     }
-    if (jv < s1 - s0) return;  // stopped at a zero pivot
+    if (jv < s1 - s0) break;  // stopped at a zero pivot
+  }
+  if constexpr (SMEM) {
+    for (int c = 0; c < w; ++c)
+      for (int i = t; i < rows; i += NT) gblk[i + (size_t)c * glda] = ztile[c * rows + i];
   }
 }
 
@@ -727,10 +736,19 @@ int zlu_factor_dev(alg_ctx* ctx, double2* d_a, int m, int nc, int lda, int* d_ip
   // ALG_ZLU_UNBLOCKED=1 (measurement switch): one pivot and one rank-1
   // launch per column instead of the blocked form; both give the same bits
   static const bool unblocked = std::getenv("ALG_ZLU_UNBLOCKED") != nullptr;
+  static const cudaError_t configured = cudaFuncSetAttribute(
+      zpanel_kernel<true, kZpanelThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZpanelSmem);
+  ALG_CUDA_TRY(configured);
   if (!unblocked) {
     for (int k0 = 0; k0 < nc; k0 += kZpw) {
       const int w = std::min(kZpw, nc - k0);
-      zpanel_kernel<<<1, kZpanelThreads, 0, ctx->stream>>>(d_a, lda, m, k0, w, d_ipiv, ctx->d_status);
+      const size_t tile = sizeof(double2) * (size_t)(m - k0) * w;
+      if (tile <= kZpanelSmem)
+        zpanel_kernel<true, kZpanelThreads><<<1, kZpanelThreads, tile, ctx->stream>>>(d_a, lda, m, k0, w, d_ipiv,
+                                                                                     ctx->d_status);
+      else
+        zpanel_kernel<false, kZpanelThreads><<<1, kZpanelThreads, 0, ctx->stream>>>(d_a, lda, m, k0, w, d_ipiv,
+                                                                                    ctx->d_status);
       int launches = 1;
       if (nc > w) {
         zswap_trsm_kernel<<<(nc - w + kZswapThreads - 1) / kZswapThreads, kZswapThreads, 0, ctx->stream>>>(d_a, lda, nc, k0, w, d_ipiv, ctx->d_status);
