@@ -40,7 +40,7 @@ def nvcc() -> str:
 
 
 def _headers_mtime() -> float:
-    hs = list(CSRC.glob("*.cuh")) + list((ROOT / "include").glob("*.h"))
+    hs = [*CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *(ROOT / "include").glob("*.h")]
     return max((h.stat().st_mtime for h in hs), default=0.0)
 
 

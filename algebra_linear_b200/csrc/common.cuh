@@ -8,6 +8,7 @@
 #include <climits>
 
 #include "algebra_linear_gpu.h"
+#include "per_device.h"
 
 namespace alg {
 
@@ -60,6 +61,15 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // Every spin-wait in this library gives up after this long, raises the
 // timeout flag of its status block and lets its kernel return.
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s
+
+// f() on the first call for the current device (a kernel's attributes).
+template <typename F>
+cudaError_t once_per_device(PerDevice& p, F&& f) {
+  int device = 0, value = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return static_cast<cudaError_t>(p.get(device, value, [&](int&) { return static_cast<int>(f()); }));
+}
 
 }  // namespace alg
 

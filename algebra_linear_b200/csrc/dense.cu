@@ -67,16 +67,15 @@ int launch_panel_w(alg_ctx* ctx, const PanelArgs<T>& args) {
     smem = panel_smem_bytes<T, W>((m + C - 1) / C);
   }
   if (smem > kMaxSmem) return ALG_BAD_SHAPE;  // panel too tall for one cluster
-  // kernel attributes set once per process (a thread-safe static initializer)
-  static const cudaError_t configured = [] {
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
     cudaError_t e = cudaFuncSetAttribute(panel_cluster_kernel<T, W, EXACT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(panel_cluster_kernel<T, W, EXACT>, cudaFuncAttributeNonPortableClusterSizeAllowed,
                                1);
     return e;
-  }();
-  ALG_CUDA_TRY(configured);
+  }));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
   cfg.blockDim = dim3(kPanelThreads, 1, 1);
@@ -122,15 +121,15 @@ bool block_panel_fits(int m) {
 
 template <typename T, int W, int NT, int RPT, bool EXACT>
 int launch_panel_reg(alg_ctx* ctx, const PanelArgs<T>& args, int C) {
-  static const cudaError_t configured = [] {
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
     cudaError_t e = cudaFuncSetAttribute(panel_reg_kernel<T, W, NT, RPT, EXACT>,
                                          cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(panel_reg_kernel<T, W, NT, RPT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kBlockPanelSmem);
     return e;
-  }();
-  ALG_CUDA_TRY(configured);
+  }));
   const int m = args.n - args.c0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
@@ -196,7 +195,8 @@ int launch_trsm_reg(alg_ctx* ctx, T* a, int lda, int r0, int kb, int cb, int ce)
        trsm_lower_unit_reg_kernel<T, EXACT, 4, 2>},
       {trsm_lower_unit_reg_kernel<T, EXACT, 1, 8>, trsm_lower_unit_reg_kernel<T, EXACT, 2, 8>,
        trsm_lower_unit_reg_kernel<T, EXACT, 4, 8>}};
-  static const cudaError_t configured = [] {
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
     for (const auto& row : kerns)
       for (Kern k : row) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -204,8 +204,7 @@ int launch_trsm_reg(alg_ctx* ctx, T* a, int lda, int r0, int kb, int cb, int ce)
         if (e != cudaSuccess) return e;
       }
     return cudaSuccess;
-  }();
-  ALG_CUDA_TRY(configured);
+  }));
   const Kern kern = kerns[few ? 0 : 1][rpt / 2];
   const size_t smem = sizeof(T) * (size_t)kb * 32 * rpt;
   const int cta_cols = (few ? 2 : 8) * (kTrsmThreads / 32);
@@ -252,9 +251,11 @@ bool dmma_disabled() {
 template <typename T, bool EXACT, int NJ, bool VEC>
 int launch_gemm_sub(alg_ctx* ctx, int M, int N, int K, const T* A, int lda, const T* B, int ldb, T* C, int ldc) {
   using Cfg = SubCfg<T, NJ>;
-  static const cudaError_t configured = cudaFuncSetAttribute(
-      gemm_sub_kernel<T, EXACT, NJ, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
-  ALG_CUDA_TRY(configured);
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
+    return cudaFuncSetAttribute(gemm_sub_kernel<T, EXACT, NJ, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)Cfg::kSmem);
+  }));
   dim3 grid((M + Cfg::kBM - 1) / Cfg::kBM, (N + Cfg::kBN - 1) / Cfg::kBN);
   gemm_sub_kernel<T, EXACT, NJ, VEC><<<grid, Cfg::kThreads, Cfg::kSmem, ctx->stream>>>(
       M, N, K, A, lda, B, ldb, C, ldc, Cfg::kCtas * ctx->sm_count);
@@ -544,9 +545,10 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
   cudaEventRecord(ev_a, sa);
   cudaStreamWaitEvent(user, ev_a, 0);
   if (at_end && rc == ALG_OK) {
-    static const cudaError_t configured = cudaFuncSetAttribute(
-        permute_left_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPermSmem);
-    ALG_CUDA_TRY(configured);
+    static PerDevice configured;
+    ALG_CUDA_TRY(once_per_device(configured, [] {
+      return cudaFuncSetAttribute(permute_left_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPermSmem);
+    }));
     const int tok = prof_begin(ctx, ALG_K_LASWP);
     compose_swaps_kernel<<<(m + 63) / 64, 64, 0, user>>>(lab, m, nb, nblk, comp, perm);
     permute_left_kernel<T><<<(nblk - 1) * nb, kPermThreads, sizeof(T) * (size_t)(m - nb), user>>>(a, lda, m, nb, comp);
@@ -582,7 +584,8 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
   T* uinv = linv + (size_t)nblk * kb * kb;
   constexpr size_t kInvSmem = sizeof(T) * kb * kb;
   constexpr size_t kStepSmem = StepCfg<T>::kSmem;
-  static const cudaError_t configured = [] {
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
     cudaError_t e = cudaFuncSetAttribute(tri_block_inverse_kernel<T, false, 4, 2>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
     if (e == cudaSuccess)
@@ -593,8 +596,7 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem);
     return e;
-  }();
-  ALG_CUDA_TRY(configured);
+  }));
   const int tok = prof_begin(ctx, ALG_K_SOLVE);
   {
     const dim3 ig(kb / (2 * (kTrsmThreads / 32)), nblk);

@@ -189,9 +189,11 @@ template <int MI, int NJ, bool VEC>
 int launch_dmma(alg_ctx* ctx, int M, int N, int K, const double* A, int lda, const double* B, int ldb, double* C,
                 int ldc) {
   using Cfg = DmmaCfg<MI, NJ>;
-  static const cudaError_t configured = cudaFuncSetAttribute(
-      dmma_gemm_sub_kernel<MI, NJ, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem);
-  ALG_CUDA_TRY(configured);
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
+    return cudaFuncSetAttribute(dmma_gemm_sub_kernel<MI, NJ, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)Cfg::kSmem);
+  }));
   dim3 grid((M + Cfg::kBM - 1) / Cfg::kBM, (N + Cfg::kBN - 1) / Cfg::kBN);
   dmma_gemm_sub_kernel<MI, NJ, VEC><<<grid, Cfg::kThreads, Cfg::kSmem, ctx->stream>>>(
       M, N, K, A, lda, B, ldb, C, ldc, (NJ == 4 ? 3 : 4) * ctx->sm_count);

@@ -1052,9 +1052,11 @@ int grid_for(alg_ctx* ctx, int64_t work, int threads) {
 
 template <typename T, int NT>
 int launch_small(const SmallArgs<T>& sa, int count, cudaStream_t st) {
-  static const cudaError_t configured = cudaFuncSetAttribute(
-      small_front_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_front_smem<T, NT>());
-  ALG_CUDA_TRY(configured);
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
+    return cudaFuncSetAttribute(small_front_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)small_front_smem<T, NT>());
+  }));
   small_front_kernel<T, NT><<<count, NT, small_front_smem<T, NT>(), st>>>(sa);
   count_launches();
   return ALG_OK;

@@ -299,15 +299,19 @@ __global__ void __launch_bounds__(kTThreads) trsv_dataflow_kernel(const T* __res
 template <typename T, bool EXACT, bool UPPER>
 int launch_trsv(alg_ctx* ctx, const T* lu, int lda, int n, T* x, int ldx, int nrhs, int* flags, int* abort_flag) {
   const int nb = (n + kTB - 1) / kTB;
-  static int max_blocks = 0;
-  if (max_blocks == 0) {
+  static PerDevice resident;  // CTAs of the kernel that a device holds at once
+  int device = 0, max_blocks = 0;
+  ALG_CUDA_TRY(cudaGetDevice(&device));
+  ALG_CUDA_TRY(static_cast<cudaError_t>(resident.get(device, max_blocks, [&](int& blocks) {
     int per_sm = 0;
-    ALG_CUDA_TRY(cudaFuncSetAttribute(trsv_dataflow_kernel<T, EXACT, UPPER>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem<T>));
-    ALG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsv_dataflow_kernel<T, EXACT, UPPER>,
-                                                               kTThreads, kTSmem<T>));
-    max_blocks = std::max(1, per_sm) * ctx->sm_count;
-  }
+    cudaError_t e = cudaFuncSetAttribute(trsv_dataflow_kernel<T, EXACT, UPPER>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem<T>);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsv_dataflow_kernel<T, EXACT, UPPER>, kTThreads,
+                                                        kTSmem<T>);
+    blocks = std::max(1, per_sm) * ctx->sm_count;
+    return static_cast<int>(e);
+  })));
   int grid = std::min(nb, max_blocks);
   uint64_t limit = ctx->wait_limit_ns ? ctx->wait_limit_ns : kWaitLimitNs;
   int stuck = 0;

@@ -599,14 +599,15 @@ namespace {
 
 template <int W>
 int launch_fused(alg_ctx* ctx, const TsluArgs& p, int groups0, int side_blocks, TsluScratch* ws, bool* done) {
-  // co-resident CTAs of the single launch, computed once per process (a
-  // thread-safe static initializer; 0 when the query fails)
-  static const int max_ctas = [ctx] {
+  static PerDevice resident;  // CTAs of the single launch that a device holds at once
+  int device = 0, max_ctas = 0;
+  ALG_CUDA_TRY(cudaGetDevice(&device));
+  ALG_CUDA_TRY(static_cast<cudaError_t>(resident.get(device, max_ctas, [&](int& ctas) {
     int per_sm = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tslu_fused_kernel<W>, kRows, 0) == cudaSuccess
-               ? per_sm * ctx->sm_count
-               : 0;
-  }();
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tslu_fused_kernel<W>, kRows, 0);
+    ctas = std::max(1, per_sm) * ctx->sm_count;
+    return static_cast<int>(e);
+  })));
   *done = false;
   const int grid = std::max(groups0, side_blocks);
   // the waiting CTAs hold their SMs until the root is done, which the

@@ -642,14 +642,14 @@ int zsolve_dev(alg_ctx* ctx, const double2* lu, int lda, int n, const int* ipiv,
   if (n <= kSweepMaxN) {
     const size_t fs = sizeof(double2) * ((size_t)n + kZsb * kZsb) + sizeof(int) * (size_t)n;
     const size_t bw = sizeof(double2) * ((size_t)n + 2 * ((size_t)n + 16));
-    static const cudaError_t configured = [] {
+    static PerDevice configured;
+    ALG_CUDA_TRY(once_per_device(configured, [] {
       cudaError_t e = cudaFuncSetAttribute(zforward_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            225 * 1024);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(zbackward_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
       return e;
-    }();
-    ALG_CUDA_TRY(configured);
+    }));
     zforward_smem_kernel<<<1, kSolveThreads, fs, ctx->stream>>>(lu, lda, n, ipiv, b);
     zbackward_smem_kernel<<<1, kZbackThreads, bw, ctx->stream>>>(lu, lda, n, b);
   } else {
@@ -736,9 +736,11 @@ int zlu_factor_dev(alg_ctx* ctx, double2* d_a, int m, int nc, int lda, int* d_ip
   // ALG_ZLU_UNBLOCKED=1 (measurement switch): one pivot and one rank-1
   // launch per column instead of the blocked form; both give the same bits
   static const bool unblocked = std::getenv("ALG_ZLU_UNBLOCKED") != nullptr;
-  static const cudaError_t configured = cudaFuncSetAttribute(
-      zpanel_kernel<true, kZpanelThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZpanelSmem);
-  ALG_CUDA_TRY(configured);
+  static PerDevice configured;
+  ALG_CUDA_TRY(once_per_device(configured, [] {
+    return cudaFuncSetAttribute(zpanel_kernel<true, kZpanelThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kZpanelSmem);
+  }));
   if (!unblocked) {
     for (int k0 = 0; k0 < nc; k0 += kZpw) {
       const int w = std::min(kZpw, nc - k0);
