@@ -144,13 +144,14 @@ __device__ __forceinline__ void mbar_arm(uint32_t bar, int bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
 }
 // Waits for the phase of the given parity; gives up after kWaitLimitNs and
-// returns false.
+// returns false. What completes the phase are other CTAs' st.async: acquire at
+// cluster scope (their completion releases at that scope).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, int parity) {
   uint32_t done = 0;
   uint64_t t0 = 0;
   for (int it = 1;; ++it) {
     asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
     if ((it & 63) == 0) {  // the timer is read only once the wait is long
@@ -480,8 +481,8 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(PanelAr
 //    the low word and the position.
 //  * The reciprocal of a candidate is formed beside the search and travels
 //    in its record, so no thread divides after the exchange.
-//  * A pivot is filed (its U entries, its multipliers, the interchange) by one
-//    warp, another each column; what it fetches is stored a column later.
+//  * A pivot is filed (its U entries, the interchange) by one warp, another
+//    each column.
 // Per column: candidate -> redux -> the warp's best lane stages its row ->
 // one CTA barrier -> the CTA's best record to every mailbox (16-byte st.async,
 // the CTAs spread over the warps, completing on the receiver's mbarrier) ->
@@ -490,11 +491,12 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(PanelAr
 // parity as in K1.
 //
 // With more than one leaf (bw > W) the columns right of the leaf wait in the
-// tile (tile[col][row]). A pivot row's entries there, and its multipliers,
-// are pulled from its owner's tile by the filing warp of every CTA (the owner's record vouches for its tile: it was sent after
-// the CTA barrier that follows the last update). At the leaf's end every CTA
-// solves U12 = L11^{-1} A12 for itself and updates its own rows, each entry's
-// terms in increasing k.
+// tile (tile[col][row]). At the leaf's end every CTA reads the pivot rows'
+// entries there, and their multipliers, from their owners' tiles, solves
+// U12 = L11^{-1} A12 for itself and updates its own rows, each entry's terms in
+// increasing k. A cluster barrier comes before those reads: the tiles are
+// written by ordinary stores, which a record's arrival does not order for
+// another CTA. Nothing changes a pivot row afterwards, so none follows them.
 //
 // Division: the multiplier is the correctly rounded quotient a/d
 // (mod.rs:154). With y = RN(1/d), q = RN(a*y) is within one ulp of a/d, the
@@ -559,6 +561,7 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
   __shared__ int side_src[2 * kBlockMaxW];
   __shared__ int side_dst[2 * kBlockMaxW];
   __shared__ int side_cnt;
+  __shared__ int piv_src[W];  // the leaf's pivot rows: owner << 16 | slot there
 
   // ---- load --------------------------------------------------------------
   T v[RPT][W];
@@ -606,17 +609,6 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
   for (int cl0 = 0; cl0 < bw; cl0 += W) {
     const int w = min(W, bw - cl0);
     const int tc = bw - cl0 - w;  // columns of the block right of the leaf
-    // the filed pivot row's multipliers and its entries right of the leaf,
-    // fetched in one column and stored in the next
-    T pull[2];
-    auto keep_pull = [&](int j) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int c = lane + 32 * i;
-        if (c < j) l11[j * W + c] = pull[i];
-        else if (c >= W && c < W + tc) ubuf[(c - W) * W + j] = pull[i];
-      }
-    };
 #pragma unroll 1
     for (int j = 0; j < w; ++j) {
       const int J = cl0 + j;  // column of the launch = row position of its pivot
@@ -677,7 +669,6 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
         __syncwarp();
         win = owner = warp_pick(&rec[par][0], C, lane, mp);
       }
-      if (multi && j > 0 && warp == ((j - 1) % NW)) keep_pull(j - 1);
       const Rec& wr = rec[par][win];
       const int pr = ok_wait ? mp : J;  // winning row's position (>= J)
       const T d = wr.row[0];
@@ -690,14 +681,7 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
           p.ipiv[p.c0 + J] = p.c0 + pr;
           if (d == T(0)) atomicMin(&p.status->singular_col, p.c0 + J);
         }
-        if (multi) {
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int c = lane + 32 * i;
-            if (c < j || (c >= W && c < W + tc))
-              ld_cluster(pull[i], mapa_u32(tile_base + (uint32_t)sizeof(T) * ((cl0 + c) * ldt + slot), owner));
-          }
-        }
+        if (lane == 0) piv_src[j] = owner << 16 | slot;
       }
       // ---- 4. rows J and pr change places; divide and update below J -------
       const bool fast = exp_fast_ok(d);
@@ -731,8 +715,20 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
         for (int k = 0; k < RPT; ++k) v[k][c - 1] = msub<EXACT>(v[k][c], l[k], u);
       }
     }
-    if (multi && warp == ((w - 1) % NW)) keep_pull(w - 1);
     if (tc > 0) {  // (then w == W)
+      if (C > 1) cl.sync();
+      else __syncthreads();
+#pragma unroll 4
+      for (int e = tid; e < W * (W + tc); e += NT) {
+        const int j = e % W, c = e / W;  // pivot row j, column c of the leaf and those right of it
+        if (c < j || c >= W) {
+          const int src = piv_src[j];
+          T v;
+          ld_cluster(v, mapa_u32(tile_base + (uint32_t)sizeof(T) * ((cl0 + c) * ldt + (src & 0xffff)), src >> 16));
+          if (c < W) l11[j * W + c] = v;
+          else ubuf[(c - W) * W + j] = v;
+        }
+      }
       __syncthreads();
       if (tid < tc) {
         T* x = ubuf + tid * W;
