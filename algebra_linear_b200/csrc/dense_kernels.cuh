@@ -16,6 +16,7 @@
 #include <math_constants.h>
 
 #include "common.cuh"
+#include "index_guard.h"
 #include "pivot.cuh"
 
 namespace alg {
@@ -423,6 +424,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(PanelAr
   if (tid == 0) S.side_cnt = 0;
   __syncthreads();
   for (int r = tid; r < nr; r += kPanelThreads) {
+    loc_s[r] = index_or(loc_s[r], p.c0, p.n, p.c0 + rb + r);
     if (loc_s[r] != p.c0 + rb + r) {
       const int s = atomicAdd(&S.side_cnt, 1);
       if (s < 4 * kPanelMaxW) S.side_rows[s] = r;
@@ -876,7 +878,7 @@ __global__ void __launch_bounds__(kSwapThreads) laswp_outside_kernel(
 #pragma unroll
     for (int i = 0; i < kSwapScan; ++i) {
       const int r = r0 + i * kSwapThreads;
-      src[i] = r < n ? lab[r] : r;
+      src[i] = r < n ? index_or(lab[r], k0, n, r) : r;
     }
 #pragma unroll
     for (int i = 0; i < kSwapScan; ++i) {
@@ -941,8 +943,7 @@ __global__ void compose_swaps_kernel(const int* lab, int n, int nb, int nblk, in
   if (r >= n) return;
   int s = r;
   for (int b = min(nblk - 1, r / nb); b >= 0; --b) {
-    const int t = lab[(size_t)b * n + s];
-    s = (unsigned)t < (unsigned)n ? t : s;  // (a panel that timed out may leave a label unset)
+    s = index_or(lab[(size_t)b * n + s], b * nb, n, s);
     if (b > 0) comp[(size_t)(b - 1) * n + r] = s;
   }
   if (perm != nullptr) perm[r] = s;
