@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
       const T y = wr.recip;
       // one warp files the pivot row ------------------------------------
       if (warp == (j % NW)) {
-        const int slot = ok_wait ? (int)wr.slot : 0;
+        const int slot = ok_wait ? index_or((int)wr.slot, 0, ldt, 0) : 0;
         if (owner == q && lane < w - j) tile[(J + lane) * ldt + slot] = wr.row[lane];
         if (lane == 0 && q == 0) {
           p.ipiv[p.c0 + J] = p.c0 + pr;
@@ -796,6 +796,7 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int r = tid + k * NT;
+    if (pos[k] >= 0) pos[k] = index_or(pos[k], 0, m, rb + r);
     lab[k] = p.c0 + rb + r;
     if (pos[k] >= 0 && !p.first_leaf) lab[k] = p.lab[p.c0 + rb + r];
     if (pos[k] >= 0 && pos[k] != rb + r) {

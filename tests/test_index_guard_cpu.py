@@ -56,3 +56,14 @@ def _kernel(name):
 def test_labels_are_checked_before_they_index(kernel, uses):
     found = re.findall(uses, _kernel(kernel))
     assert found == ["index_or"]
+
+
+def test_panel_positions_and_slots_are_checked():
+    # a record that another CTA sent out of step: its slot before it addresses
+    # the tile, the rows' positions before the rows are written there
+    body = _kernel("panel_reg_kernel")
+    assert re.findall(r"slot = ok_wait \? (\w+)\(\(int\)wr\.slot, 0, ldt, 0\)", body) == ["index_or"]
+    check = re.search(r"pos\[k\] = index_or\(pos\[k\], 0, m, rb \+ r\)", body)
+    assert check
+    for use in (r"side_dst\[s\] = p\.c0 \+ pos\[k\]", r"p\.a \+ \(size_t\)\(p\.c0 \+ pos\[k\]\)", r"p\.lab\[p\.c0 \+ pos\[k\]\]"):
+        assert re.search(use, body).start() > check.start()
