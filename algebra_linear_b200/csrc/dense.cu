@@ -571,8 +571,7 @@ constexpr int kBlockedSolveRhs = 16;
 // reads x1 and writes y into x2; the backward sweep reads x2 and writes x
 // into x1.
 template <typename T>
-int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb,
-                         const DevStatus* guard) {
+int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb) {
   if (n == 0 || nrhs == 0) return ALG_OK;
   constexpr int kb = kSolveKb;
   const int nblk = (n + kb - 1) / kb;
@@ -604,7 +603,7 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
     tri_block_inverse_kernel<T, true, 4, 2><<<ig, kTrsmThreads, kInvSmem, ctx->stream>>>(lu, lda, n, kb, uinv);
     const size_t cnt = (size_t)n * nrhs;
     const int g = (int)std::max<size_t>(1, std::min<size_t>((cnt + 255) / 256, (size_t)ctx->sm_count * 8));
-    gather_perm_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x1, n, guard);
+    gather_perm_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x1, n);
     count_launches(3);
     ALG_CUDA_TRY(cudaGetLastError());
   }
@@ -633,7 +632,7 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
   }
   count_launches(2 * nblk);
   ALG_CUDA_TRY(cudaGetLastError());
-  ALG_TRY(store_solution_dev<T>(ctx, x1, n, nrhs, b, ldb, guard));
+  ALG_TRY(store_solution_dev<T>(ctx, x1, n, nrhs, b, ldb, nullptr));
   prof_end(ctx, tok, 2.0 * n * n * nrhs, sizeof(T) * (double(n) * n + 4.0 * n * nrhs));
   return ALG_OK;
 }
@@ -644,7 +643,8 @@ int lu_solve_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* 
   if (nrhs > 65535) return ALG_BAD_SHAPE;
   // the exact form keeps the reference's per-entry order (the dataflow
   // sweeps); the fused forms solve many right-hand sides blocked
-  if (!EXACT && nrhs >= kBlockedSolveRhs) return lu_solve_blocked_dev<T>(ctx, lu, n, lda, perm, b, nrhs, ldb, guard);
+  if (!EXACT && nrhs >= kBlockedSolveRhs && guard == nullptr)
+    return lu_solve_blocked_dev<T>(ctx, lu, n, lda, perm, b, nrhs, ldb);
   return lu_solve_dataflow_dev<T, EXACT>(ctx, lu, n, lda, perm, b, nrhs, ldb, guard);
 }
 
@@ -682,13 +682,32 @@ int factor_any(alg_ctx* ctx, int update, double* d_a, int m, int nc, int lda, in
   return ALG_INVALID_ARGUMENT;
 }
 
-// guard: see lu_solve_dev. With it a solve follows its factorization without
-// the host looking at the status in between (one synchronisation a dgesv).
+// guard: see lu_solve_dev.
 int solve_any(alg_ctx* ctx, int update, const double* d_lu, int n, int lda, const int* d_perm,
               double* d_b, int nrhs, int ldb, const alg::DevStatus* guard) {
   if (update == ALG_UPDATE_EXACT)
     return alg::lu_solve_dev<double, true>(ctx, d_lu, n, lda, d_perm, d_b, nrhs, ldb, guard);
   return alg::lu_solve_dev<double, false>(ctx, d_lu, n, lda, d_perm, d_b, nrhs, ldb, guard);
+}
+
+// The solve after factor_any's factorization, and the status of both;
+// *singular: it met a zero pivot, and b is as it was. With up to one group of
+// the sweeps' right-hand sides the solve is launched at once, guarded, so a
+// dgesv has one synchronisation (n = 96: 168 us against 180). With more the host
+// looks first: the synchronisation is a small part of that solve, which a
+// singular matrix does not pay (nor what the solve would refuse or allocate).
+constexpr int kGuardedRhs = 4;
+
+int solve_factored(alg_ctx* ctx, int update, const double* d_lu, int n, int lda, const int* d_perm, double* d_b,
+                   int nrhs, int ldb, bool* singular) {
+  const bool guarded = nrhs <= kGuardedRhs;
+  int rc = ALG_OK;
+  if (guarded) rc = solve_any(ctx, update, d_lu, n, lda, d_perm, d_b, nrhs, ldb, ctx->d_status);
+  ALG_TRY(alg::status_fetch(ctx));  // a timed-out sweep is an error, not a result
+  *singular = ctx->h_status->singular_col != INT_MAX;
+  if (*singular || guarded) return *singular ? ALG_OK : rc;
+  ALG_TRY(solve_any(ctx, update, d_lu, n, lda, d_perm, d_b, nrhs, ldb, nullptr));
+  return alg::status_fetch(ctx);
 }
 
 // Sizes accepted by the int32-indexed kernels.
@@ -725,9 +744,8 @@ int host_lu(int update, double* a, size_t m, size_t nc, size_t* ipiv, double* de
   if (d_b) ALG_CUDA_TRY(cudaMemcpyAsync(d_b, b, sizeof(double) * m * nrhs, cudaMemcpyHostToDevice, ctx->stream));
   ALG_TRY(alg::status_reset(ctx));
   ALG_TRY(factor_any(ctx, update, d_a, M, N, M, d_ipiv, d_perm));
-  if (d_b) ALG_TRY(solve_any(ctx, update, d_a, M, M, d_perm, d_b, R, M, ctx->d_status));
-  ALG_TRY(alg::status_fetch(ctx));  // a timed-out sweep is an error, not a result
-  const bool singular = ctx->h_status->singular_col != INT_MAX;
+  bool singular = false;
+  ALG_TRY(solve_factored(ctx, update, d_a, M, M, d_perm, d_b, d_b ? R : 0, M, &singular));
   if (!singular && d_b)
     ALG_CUDA_TRY(cudaMemcpyAsync(b, d_b, sizeof(double) * m * nrhs, cudaMemcpyDeviceToHost, ctx->stream));
   ALG_CUDA_TRY(cudaMemcpyAsync(a, d_a, sizeof(double) * m * nc, cudaMemcpyDeviceToHost, ctx->stream));
@@ -933,9 +951,9 @@ int alg_dgesv_dev(alg_ctx* ctx, int update, double* d_a, int n, int lda, double*
   ALG_TRY(alg::ws_get(ctx, alg::WS_PERM, sizeof(int) * n, reinterpret_cast<void**>(&perm)));
   ALG_TRY(alg::status_reset(ctx));
   ALG_TRY(factor_any(ctx, update, d_a, n, n, lda, ipiv, perm));
-  ALG_TRY(solve_any(ctx, update, d_a, n, lda, perm, d_b, nrhs, ldb, ctx->d_status));
-  ALG_TRY(alg::status_fetch(ctx));  // synchronises; reports a timed-out sweep
-  return ctx->h_status->singular_col != INT_MAX ? ALG_SINGULAR : ALG_OK;
+  bool singular = false;
+  ALG_TRY(solve_factored(ctx, update, d_a, n, lda, perm, d_b, nrhs, ldb, &singular));
+  return singular ? ALG_SINGULAR : ALG_OK;
 }
 
 }  // extern "C"
