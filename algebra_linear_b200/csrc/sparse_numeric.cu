@@ -1166,8 +1166,10 @@ int DeviceLu::init(alg_ctx* c, const FrontPlan* p, int w) {
       if (k + 1 < (int)F.lane_ptr.size())
         std::for_each(F.lane_fronts.begin() + F.lane_ptr[k], F.lane_fronts.begin() + F.lane_ptr[k + 1], front);
       if (k == 0) std::for_each(F.top_fronts.begin(), F.top_fronts.end(), front);
+      // (only so that it need not grow front by front: without the room for it
+      // the factorization takes two labels a row, as far as it goes)
       void* p_lab = nullptr;
-      ALG_TRY(ws_get(lane_ctx[k], WS_LAB, lab, &p_lab));
+      if (ws_get(lane_ctx[k], WS_LAB, lab, &p_lab) != ALG_OK) cudaGetLastError();
     }
     if (words == 2)  // 2 rows x 2 kZnb columns of doubles per complex row
       ALG_TRY(dmalloc((void**)&d_zblock[k], sizeof(double) * 4 * kZnb * max_rows));
