@@ -115,6 +115,15 @@ __device__ __forceinline__ int warp_pick(const Rec* rec, int count, int lane, in
   return mt & 31;
 }
 
+// A barrier of the CTA's NT threads that its warps may reach at different places
+// in the code (__syncthreads must be met at one place by all of them). Each warp
+// comes to it whole; the form for warps that may not cost 1 % of a small front
+// of 192 columns (649 us the call with this one, 656 with that).
+template <int NT>
+__device__ __forceinline__ void cta_barrier() {
+  asm volatile("barrier.sync.aligned 1, %0;" ::"n"(NT) : "memory");
+}
+
 // One leaf of an LU by one CTA: columns [cl0, cl0 + w) (w <= W) of the m rows
 // in tile[col][row] (column stride ldt), rows tid + k NT of it by this thread
 // (m <= NT * RPT), pos[k] the row's position (-1: no row). The column chain
@@ -141,7 +150,7 @@ __device__ __noinline__ int cta_leaf(T* tile, int ldt, int m, int cl0, int w, in
   if (warp >= nw) {
 #pragma unroll 1
     for (int j = 0; j < w; ++j) {
-      __syncthreads();
+      cta_barrier<NT>();
       const int par = (cl0 + j) & 1;
       const T d = rec[par][warp_pick(&rec[par][0], nw, lane, mp)].row[0];
       if (RECIP) {
@@ -195,7 +204,7 @@ __device__ __noinline__ int cta_leaf(T* tile, int ldt, int m, int cl0, int w, in
           for (int c = 0; c < W; ++c) s.row[c] = v[k][c];
         }
     }
-    __syncthreads();
+    cta_barrier<NT>();
     const int win = warp_pick(&rec[par][0], nw, lane, mp);
     const PivotRec<T, W>& wr = rec[par][win];
     const T d = wr.row[0];
