@@ -390,10 +390,7 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
   int* perm_tmp = nullptr;
   ALG_TRY(ws_get(ctx, WS_PERM_TMP, sizeof(int) * kSwapMaxMoves, reinterpret_cast<void**>(&perm_tmp)));
   void* tslu_ws = nullptr;
-  if (std::is_same<T, float>::value && plan.tslu) {
-    ALG_TRY(ws_get(ctx, WS_TSLU, tslu_scratch_bytes(), &tslu_ws));
-    ALG_TRY(tslu_scratch_reset(ctx, tslu_ws));
-  }
+  if (std::is_same<T, float>::value && plan.tslu) ALG_TRY(ws_get(ctx, WS_TSLU, tslu_scratch_bytes(), &tslu_ws));
   if (perm != nullptr && !at_end) {
     iota_kernel<<<std::min(1024, (m + 255) / 256), 256, 0, ctx->stream>>>(perm, m);
     count_launches();

@@ -124,10 +124,6 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t a, int rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_async_b64(uint32_t remote, unsigned long long v, uint32_t remote_bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
-               :: "r"(remote), "l"(v), "r"(remote_bar) : "memory");
-}
 // One bulk copy (async proxy) of `bytes` from this CTA's shared memory into
 // the shared memory of a CTA of the cluster, completing on that CTA's mbarrier.
 // Addresses 16-byte aligned, bytes a multiple of 16.
@@ -1461,147 +1457,6 @@ __global__ void __launch_bounds__(128, SubCfg<T, NJ>::kCtas)
       const int mi = m0 + tx + 16 * r;
       if (mi < M && nj < N) Cm[(size_t)mi + (size_t)nj * ldc] = acc[r][c];
     }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// K5: triangular solves with the packed factors (getrs), blocked by kSolveB
-// rows. The forward sweep gives x_i the terms l_ij x_j in increasing j with
-// rounded product and difference — the reference's row-dot sequence
-// (mod.rs:341-347) — so it is bit-identical; the backward sweep applies the
-// terms of each block as soon as the block is solved (a different order from
-// the reference's row-dot, mod.rs:348-353, which no parallel schedule can keep).
-//
-// Launch b of a sweep updates every remaining row with block b's solved
-// unknowns; CTA 0 owns the rows of the next block and, after updating them,
-// solves that block's triangle so the next launch can use it.
-// ---------------------------------------------------------------------------
-constexpr int kSolveB = 64;
-constexpr int kSolveThreads = 256;
-
-// x = b[perm] for every right-hand side, then solve block 0's triangle.
-template <typename T>
-__global__ void __launch_bounds__(kSolveThreads) solve_gather_kernel(
-    const T* __restrict__ lu, int lda, int n, const int* __restrict__ perm,
-    const T* __restrict__ b, int ldb, T* __restrict__ x, int ldx) {
-  const int rhs = blockIdx.y;
-  const T* bc = b + (size_t)rhs * ldb;
-  T* xc = x + (size_t)rhs * ldx;
-  for (int i = blockIdx.x * kSolveThreads + threadIdx.x; i < n; i += gridDim.x * kSolveThreads) {
-    xc[i] = bc[perm[i]];
-  }
-}
-
-// The diagonal blocks are staged in shared memory (Ls, kSolveB x kSolveB)
-// before their sequential sweep, so the sweep never waits on global memory.
-template <typename T, bool EXACT>
-__device__ void solve_diag_block_lower(const T* lu, int lda, T* xc, int j0, int bs, T* xs, T* Ls) {
-  // unit lower triangle of rows/cols [j0, j0+bs)
-  for (int idx = threadIdx.x; idx < bs * bs; idx += blockDim.x) {
-    const int i = idx % bs, k = idx / bs;
-    Ls[i + k * kSolveB] = lu[(size_t)(j0 + i) + (size_t)(j0 + k) * lda];
-  }
-  for (int i = threadIdx.x; i < bs; i += blockDim.x) xs[i] = xc[j0 + i];
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // one warp: lanes own rows i = lane, lane+32; step k broadcasts x_k
-    for (int k = 0; k + 1 < bs; ++k) {
-      const T u = xs[k];
-      for (int i = k + 1 + threadIdx.x; i < bs; i += 32) xs[i] = msub<EXACT>(xs[i], Ls[i + k * kSolveB], u);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < bs; i += blockDim.x) xc[j0 + i] = xs[i];
-}
-
-template <typename T, bool EXACT>
-__device__ void solve_diag_block_upper(const T* lu, int lda, T* xc, int j0, int bs, T* xs, T* Ls) {
-  for (int idx = threadIdx.x; idx < bs * bs; idx += blockDim.x) {
-    const int i = idx % bs, k = idx / bs;
-    Ls[i + k * kSolveB] = lu[(size_t)(j0 + i) + (size_t)(j0 + k) * lda];
-  }
-  for (int i = threadIdx.x; i < bs; i += blockDim.x) xs[i] = xc[j0 + i];
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    for (int k = bs - 1; k >= 0; --k) {
-      if (threadIdx.x == 0) xs[k] = div_rn(xs[k], Ls[k + k * kSolveB]);
-      __syncwarp();
-      const T u = xs[k];
-      for (int i = threadIdx.x; i < k; i += 32) xs[i] = msub<EXACT>(xs[i], Ls[i + k * kSolveB], u);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < bs; i += blockDim.x) xc[j0 + i] = xs[i];
-}
-
-// Forward: rows [j0+bs, n) take block [j0, j0+bs)'s terms. CTA 0 owns the next
-// block's rows and then solves its triangle. j0 = -bs means "only solve block 0".
-template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kSolveThreads) solve_fwd_kernel(
-    const T* __restrict__ lu, int lda, int n, T* __restrict__ x, int ldx, int j0, int bs) {
-  __shared__ T xb[kSolveB];
-  __shared__ T xs[kSolveB];
-  __shared__ T Ls[kSolveB * kSolveB];
-  const int rhs = blockIdx.y;
-  T* xc = x + (size_t)rhs * ldx;
-  const int j1 = j0 + bs;                // first row below the block
-  const int nb1 = min(kSolveB, n - j1);  // rows in the next block
-  if (j0 >= 0) {
-    for (int k = threadIdx.x; k < bs; k += kSolveThreads) xb[k] = xc[j0 + k];
-    __syncthreads();
-    int i_begin, i_end;
-    if (blockIdx.x == 0) { i_begin = j1; i_end = j1 + nb1; }
-    else {
-      i_begin = j1 + nb1 + (blockIdx.x - 1) * kSolveThreads;
-      i_end = min(n, i_begin + kSolveThreads);
-    }
-    const int i = i_begin + threadIdx.x;
-    if (i < i_end) {
-      T acc = xc[i];
-      for (int k = 0; k < bs; ++k) acc = msub<EXACT>(acc, lu[(size_t)i + (size_t)(j0 + k) * lda], xb[k]);
-      xc[i] = acc;
-    }
-  }
-  if (blockIdx.x == 0 && nb1 > 0) {
-    __syncthreads();
-    solve_diag_block_lower<T, EXACT>(lu, lda, xc, j1, nb1, xs, Ls);
-  }
-}
-
-// Backward: rows [0, j0) take block [j0, j0+bs)'s terms. CTA 0 owns the
-// previous block's rows [j0-bp, j0) and then solves its triangle.
-// j0 = n means "only solve the last block" (bs is then that block's size).
-template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kSolveThreads) solve_bwd_kernel(
-    const T* __restrict__ lu, int lda, int n, T* __restrict__ x, int ldx, int j0, int bs,
-    int bp) {
-  __shared__ T xb[kSolveB];
-  __shared__ T xs[kSolveB];
-  __shared__ T Ls[kSolveB * kSolveB];
-  const int rhs = blockIdx.y;
-  T* xc = x + (size_t)rhs * ldx;
-  const int jp = j0 - bp;  // first row of the previous block
-  if (j0 < n) {
-    for (int k = threadIdx.x; k < bs; k += kSolveThreads) xb[k] = xc[j0 + k];
-    __syncthreads();
-    int i_begin, i_end;
-    if (blockIdx.x == 0) { i_begin = jp; i_end = j0; }
-    else {
-      i_begin = (blockIdx.x - 1) * kSolveThreads;
-      i_end = min(jp, i_begin + kSolveThreads);
-    }
-    const int i = i_begin + threadIdx.x;
-    if (i < i_end) {
-      T acc = xc[i];
-      for (int k = 0; k < bs; ++k) acc = msub<EXACT>(acc, lu[(size_t)i + (size_t)(j0 + k) * lda], xb[k]);
-      xc[i] = acc;
-    }
-  }
-  if (blockIdx.x == 0 && bp > 0) {
-    __syncthreads();
-    solve_diag_block_upper<T, EXACT>(lu, lda, xc, jp, bp, xs, Ls);
   }
 }
 

@@ -23,13 +23,10 @@
 // partial-pivoting LU (panel_reg_kernel) is that node's, 64 columns a launch.
 // The factorization differs from partial pivoting's (other pivots); the
 // mixed form's refinement in FP64 then brings the solution to the FP64
-// backward error, which is its contract. In the single-launch form every CTA
-// waits (bounded) for the root's release; the multi-launch form has no waits.
+// backward error, which is its contract. One launch per level and one for the
+// apply step: no CTA waits for another.
 #include <algorithm>
-#include <atomic>
 #include <climits>
-#include <cstddef>
-#include <cstdlib>
 
 #include "dense.cuh"
 
@@ -42,14 +39,7 @@ constexpr int kFan = 8;           // children merged by one CTA (8 x 32 = 256 ro
 constexpr int kMaxGroups = 1024;  // CTAs of the first level: up to 262 144 panel rows
 constexpr int kMaxMoves = 2 * kW;
 
-constexpr int kMaxLevels = 4;        // merge levels: 1024 -> 128 -> 16 -> 2 -> 1
-constexpr int kFusedMaxGroups = 32;  // panels of up to 8192 rows take the single launch
-
 struct TsluScratch {
-  // single-launch form: arrivals per parent and level (the last arrival merges
-  // and resets the count) and the root's release flag (the launch's epoch)
-  int counter[kMaxLevels][kMaxGroups / kFan];
-  unsigned ready;
   int cand_rows[2][kMaxGroups][kW];        // proposals of each CTA of a level, in step order
   int cand_cnt[2][kMaxGroups];
   float cand_vals[2][kMaxGroups][kW * kW];  // their original values, [col][k]
@@ -193,8 +183,7 @@ struct LevelIn {
   DevStatus* status;
 };
 
-// Proposals written by other CTAs are read through L2 (__ldcg): in the
-// single-launch form they were written during this launch by other SMs.
+// Proposals written by other CTAs are read through L2 (__ldcg).
 template <int W>
 __device__ void level_body(const LevelIn& in, int g, int src, int nchild, int dst, bool root, TsluScratch* ws) {
   __shared__ GeppShared box;
@@ -254,7 +243,6 @@ __device__ void level_body(const LevelIn& in, int g, int src, int nchild, int ds
         if (c < w) ws->cand_vals[dst][g][c * kW + step] = o[c];
     }
     if (t == 0) ws->cand_cnt[dst][g] = cnt;
-    __syncthreads();  // the block's shared state is reused by the next level
     return;
   }
   // ---- root: winners, L11 \ U11, the top rows' original values ------------
@@ -357,10 +345,9 @@ __device__ void level_body(const LevelIn& in, int g, int src, int nchild, int ds
     }
     if (lane == 0) ws->nmoves = nt + __popc(bo);
   }
-  __syncthreads();
 }
 
-// One level of the multi-launch form.
+// One level of the tree.
 template <int W>
 __global__ void __launch_bounds__(kRows, 1) tslu_level_kernel(LevelIn in, int src, int nchild, int dst, int root,
                                                            TsluScratch* ws) {
@@ -510,132 +497,16 @@ __global__ void __launch_bounds__(256) tslu_apply_kernel(float* a, int lda, int 
   apply_body<W>(a, lda, n, c0, w, kb0, kb1, lab, first_leaf, blockIdx.x, gridDim.x, side_blocks, side_blocks, ws);
 }
 
-__device__ __forceinline__ uint64_t tslu_timer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// The single-launch form (a cooperative launch, so every CTA is resident):
-// each CTA factors its 256-row block; the last of each kFan siblings to
-// arrive (an atomic count after a fence) merges their proposals and climbs
-// on; the CTA that factors the root publishes its results and releases the
-// launch's epoch; every CTA waits for it (bounded: 2 s, then the timeout flag)
-// and takes its share of the apply step.
-template <int W>
-__global__ void __launch_bounds__(kRows, 1) tslu_fused_kernel(LevelIn in, int groups0, int kb0, int kb1, int* lab,
-                                                           int side_blocks, unsigned epoch, TsluScratch* ws) {
-  __shared__ int last_s;
-  __shared__ int ok_s;
-  int g = blockIdx.x, groups = groups0, src = -1, dst = 0, nchild = 0, level = 0;
-  bool ran_root = false;
-  // CTAs beyond the level-0 blocks (there only for the side columns) take
-  // no part in the tree
-  for (; (int)blockIdx.x < groups0;) {
-    const bool root = groups == 1;
-    level_body<W>(in, g, src, nchild, dst, root, ws);
-    if (root) {
-      ran_root = true;
-      break;
-    }
-    __threadfence();
-    __syncthreads();
-    const int parent = g / kFan;
-    const int nkids = min(kFan, groups - parent * kFan);
-    if (threadIdx.x == 0) {
-      const int prev = atomicAdd(&ws->counter[level][parent], 1);
-      last_s = prev == nkids - 1 ? 1 : 0;
-      if (last_s) ws->counter[level][parent] = 0;  // ready for the next panel
-    }
-    __syncthreads();
-    if (!last_s) break;
-    __threadfence();
-    nchild = groups;
-    groups = (groups + kFan - 1) / kFan;
-    src = dst;
-    dst = 1 - dst;
-    g = parent;
-    ++level;
-  }
-  if (ran_root) {
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&ws->ready), "r"(epoch) : "memory");
-  }
-  if (threadIdx.x == 0) {
-    const uint64_t t0 = tslu_timer_ns();
-    int ok = 0;
-    for (;;) {
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ws->ready) : "memory");
-      if (v == epoch) {
-        ok = 1;
-        break;
-      }
-      if (tslu_timer_ns() - t0 > 2000000000ull) break;
-      __nanosleep(64);
-    }
-    ok_s = ok;
-    if (!ok) atomicExch(&in.status->timeout, 1);
-  }
-  __syncthreads();
-  if (!ok_s) return;
-  apply_body<W>(const_cast<float*>(in.a), in.lda, in.n, in.c0, in.w, kb0, kb1, lab, in.first_leaf, blockIdx.x,
-                gridDim.x, side_blocks, 0, ws);
-}
-
 }  // namespace
 
 size_t tslu_scratch_bytes() { return sizeof(TsluScratch); }
 
-// The arrival counts and the release flag start at zero (once per
-// factorization; the counts are left at zero by every merge).
-int tslu_scratch_reset(alg_ctx* ctx, void* scratch) {
-  ALG_CUDA_TRY(cudaMemsetAsync(scratch, 0, offsetof(TsluScratch, cand_rows), ctx->stream));
-  return ALG_OK;
-}
-
-namespace {
-
-template <int W>
-int launch_fused(alg_ctx* ctx, const TsluArgs& p, int groups0, int side_blocks, TsluScratch* ws, bool* done) {
-  static PerDevice resident;  // CTAs of the single launch that a device holds at once
-  int device = 0, max_ctas = 0;
-  ALG_CUDA_TRY(cudaGetDevice(&device));
-  ALG_CUDA_TRY(static_cast<cudaError_t>(resident.get(device, max_ctas, [&](int& ctas) {
-    int per_sm = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tslu_fused_kernel<W>, kRows, 0);
-    ctas = std::max(1, per_sm) * ctx->sm_count;
-    return static_cast<int>(e);
-  })));
-  *done = false;
-  const int grid = std::max(groups0, side_blocks);
-  // the waiting CTAs hold their SMs until the root is done, which the
-  // concurrent trailing update of a large matrix needs: tall panels take the
-  // multi-launch form (as do grids that cannot be co-resident)
-  if (groups0 > kFusedMaxGroups || grid > max_ctas) return ALG_OK;
-  static std::atomic<unsigned> epochs{1};
-  unsigned epoch = epochs.fetch_add(1);
-  if (epoch == 0) epoch = epochs.fetch_add(1);
-  LevelIn in{p.a, p.lda, p.n, p.c0, p.w, p.ipiv, p.lab, p.first_leaf, p.status};
-  int kb0 = p.kb0, kb1 = p.kb1;
-  int* lab = p.lab;
-  void* args[] = {(void*)&in, (void*)&groups0, (void*)&kb0, (void*)&kb1, (void*)&lab, (void*)&side_blocks,
-                  (void*)&epoch, (void*)&ws};
-  ALG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)tslu_fused_kernel<W>, dim3(grid), dim3(kRows), args, 0,
-                                           ctx->stream));
-  *done = true;
-  return ALG_OK;
-}
-
-}  // namespace
-
 // A leaf panel of the FP32 LU by tournament pivoting; the outputs of the
 // partial-pivoting cluster kernel (factored panel, ipiv, labels, side
-// columns) and U12 of the block panel's trailing columns (the in-block TRSM). Returns ALG_NOT_IMPLEMENTED when the panel does not fit its
-// limits (the caller then uses partial pivoting). One cooperative launch when
-// the level-0 CTAs fit on the device at once, else one launch per tree level
-// and one for the apply step. The scratch is reset once per factorization.
+// columns) and U12 of the block panel's trailing columns (the in-block TRSM).
+// Returns ALG_NOT_IMPLEMENTED when the panel does not fit its limits (the caller
+// then uses partial pivoting). One launch per tree level and one for the apply
+// step.
 int tslu_panel(alg_ctx* ctx, const TsluArgs& p, void* scratch) {
   const int m = p.n - p.c0, w = p.w;
   if (w > kW || w < 1 || m < w) return ALG_NOT_IMPLEMENTED;
@@ -647,19 +518,6 @@ int tslu_panel(alg_ctx* ctx, const TsluArgs& p, void* scratch) {
   double pflops = 0;
   for (int j = 0; j < w; ++j) pflops += double(m - j - 1) * (1.0 + 2.0 * (w - j - 1));
   const int tok = prof_begin(ctx, ALG_K_PANEL);
-  if (!std::getenv("ALG_TSLU_SPLIT")) {
-    bool done = false;
-    if (w <= 16)
-      ALG_TRY(launch_fused<16>(ctx, p, groups0, side_blocks, ws, &done));
-    else
-      ALG_TRY(launch_fused<32>(ctx, p, groups0, side_blocks, ws, &done));
-    if (done) {
-      count_launches(1);
-      prof_end(ctx, tok, pflops, 2.0 * sizeof(float) * m * w);
-      ALG_CUDA_TRY(cudaGetLastError());
-      return ALG_OK;
-    }
-  }
   LevelIn in{p.a, p.lda, p.n, p.c0, w, p.ipiv, p.lab, p.first_leaf, p.status};
   // level 0 reads the panel; each later level merges kFan proposals per CTA
   int groups = groups0, src = -1, dst = 0, nchild = 0, launches = 0;
