@@ -408,7 +408,7 @@ struct BatchArgs {
 // passes through L2 and HBM (n^3 / PB bytes of it per system and direction);
 // 20 000 systems of order 8..512, FP64: 81 ms before (panel columns with three
 // barriers each in shared memory, the update on the CUDA cores, sweeps of two
-// barriers a column), 29 ms now; 3 000 in the mixed form 11.1 and 6.0 ms.
+// barriers a column), 29.2 ms now; 3 000 in the mixed form 11.1 and 5.7 ms.
 template <int NT, int RPT, int PB>
 __global__ void __launch_bounds__(NT, RPT == 4 ? 2 : 512 / NT) batched_gesv_kernel(BatchArgs p) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -511,10 +511,10 @@ BatchKernel batch_kernel(int cap, int threads, int panel) {
 // The launch shape of a bucket when no autotuner chose one. With more systems
 // than SMs throughput counts: small CTAs, several to an SM, so that one
 // system's column chain runs beside another's update (1 500 systems of order
-// 257..512 in FP64: 128 x 16 11.2 ms, 256 x 16 11.9 ms, 512 x 32 11.8 ms; 3 000
-// of 129..256: 256 x 16 4.3 ms, 128 x 16 4.6 ms, 256 x 32 4.9 ms; 4 000 of
-// 65..128: 128 x 16 1.2 ms, 128 x 32 1.5 ms). The mixed form's longest systems
-// prefer the wide panel (128 x 32 12.0 ms, 128 x 16 12.8 ms). A few systems
+// 257..512 in FP64: 128 x 16 10.8 ms, 256 x 16 11.9 ms, 512 x 32 12.0 ms; 3 000
+// of 129..256: 256 x 16 4.43 ms, 128 x 16 4.45 ms, 256 x 32 4.8 ms; 4 000 of
+// 65..128: 128 x 16 1.24 ms, 128 x 32 1.41 ms). The mixed form's longest systems
+// prefer the wide panel (128 x 32 11.6 ms, 128 x 16 12.0 ms). A few systems
 // run one to an SM: a thread per row and the wide panel's fewer sweeps.
 void default_batch_shape(int cap, bool mixed, bool few, int* threads, int* panel) {
   if (few) {

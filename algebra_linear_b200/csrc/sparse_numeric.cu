@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_front_z_kernel(SmallArgs<
 // largest front (about 0.8 us a column) where a level has few fronts. The
 // 192-dof lattice (one front of 192 x 192): 2.90 ms with rank-1 updates in
 // global memory and three barriers a column, 0.37 ms now; the 300 x 300
-// grid's 27 levels, FP32: 18.6 ms before, 8.9 ms now (twice as many columns
+// grid's 27 levels, FP32: 18.6 ms before, 8.5 ms now (twice as many columns
 // per chunk changes neither). CTAs of 64, 128 and 256 threads for fronts of as
 // many rows: idle warps would lengthen every barrier.
 template <int NT>

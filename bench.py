@@ -42,12 +42,15 @@ sys.path.insert(0, str(ROOT))
 METRIC = "dgesv GFLOP/s, FP64 vs mixed-precision+IR at equal backward error; p99 latency"
 SEEDY = [1988, 1989, 1990, 1991]
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic
-# byte of a kernel class, from single-launch ncu captures at n = 8192; a
-# launch's traffic is this ratio times its algorithmic bytes (the panel:
-# 2 x 4 B x rows x 32 per leaf; the tensor-core update: 4 B x (2 M N + M K +
-# K N)), i.e. the capture scaled by the units the launch processes.
+# byte of a kernel class, from ncu captures of single launches; a launch's
+# traffic is this ratio times its algorithmic bytes, i.e. the capture scaled by
+# the units the launch processes. The panel's bytes are 2 x 4 B x rows x
+# columns; in the headline's LU (n = 16384) three quarters of them belong to the
+# panels of more than 8 192 rows (32 columns by tournament: three levels and the
+# apply step) and one quarter to the cluster's 64-column panels. The tensor-core
+# update: 4 B x (2 M N + M K + K N).
 TRAFFIC_PER_ALG_BYTE = {
-    "panel": (2.08 / 2.10, "profiles/tslu_fused_kernel_n8192.md"),
+    "panel": (0.75 * 3.99 / 2.61 + 0.25 * 3.61 / 4.13, "profiles/mixed_panels.md"),
     "gemm_tc": ((45.37 + 0.17) / 63.1, "profiles/gemm_tc_kernel_n8192.md"),
 }
 
@@ -359,7 +362,7 @@ def measured_peaks():
     return {}
 
 
-def roofline(res, form, peaks, gemm_peaks, cls=None):
+def roofline(res, form, peaks, gemm_peaks, n, cls=None):
     """Roofline of one kernel class of the event profile: the top class by
     time unless `cls` names one. Update classes (gemm, gemm_tc, trsm) are
     tensor/FP-pipe bound; the leaf panels, swaps and solves are reported
@@ -406,8 +409,9 @@ def roofline(res, form, peaks, gemm_peaks, cls=None):
         out["traffic"] = ratio * rec["bytes"] / max(rec["launches"], 1)
     if cls == "panel":
         out["note"] = "latency-bound column chain (pivot search per column); bytes = the panel read and written once"
-        # per column of the leaf chain: the measure of a latency-bound panel (HBM bytes say little)
-        out["ns_per_column"] = 1e6 * rec["ms"] / max(rec["launches"], 1) / (32 if form.startswith("mixed") else 16)
+        # per column: the measure of a latency-bound panel (HBM bytes say little).
+        # Every column passes through one panel launch; rec is one solve's total.
+        out["ns_per_column"] = 1e6 * rec["ms"] / n
     return out
 
 
@@ -1477,8 +1481,8 @@ def run_ours(args, world, rank, local, pg):
         "backward_error_bound": tol,
         "gpu_launches": hr["gpu_launches"],
         "clocks": hr["clocks"],
-        "roofline": roofline(hr, head, peaks, gemm_peaks),
-        "update_roofline": roofline(hr, head, peaks, gemm_peaks,
+        "roofline": roofline(hr, head, peaks, gemm_peaks, n),
+        "update_roofline": roofline(hr, head, peaks, gemm_peaks, n,
                                     cls="gemm_tc" if "gemm_tc" in (hr["profile"] or {}) else "gemm"),
         "cublas_gemm_peaks_tflops": gemm_peaks,
     }
