@@ -570,7 +570,8 @@ constexpr int kBlockedSolveRhs = 16;
 // reads x1 and writes y into x2; the backward sweep reads x2 and writes x
 // into x1.
 template <typename T>
-int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb) {
+int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs, int ldb,
+                         const DevStatus* guard) {
   if (n == 0 || nrhs == 0) return ALG_OK;
   constexpr int kb = kSolveKb;
   const int nblk = (n + kb - 1) / kb;
@@ -602,7 +603,7 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
     tri_block_inverse_kernel<T, true, 4, 2><<<ig, kTrsmThreads, kInvSmem, ctx->stream>>>(lu, lda, n, kb, uinv);
     const size_t cnt = (size_t)n * nrhs;
     const int g = (int)std::max<size_t>(1, std::min<size_t>((cnt + 255) / 256, (size_t)ctx->sm_count * 8));
-    gather_perm_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x1, n);
+    gather_perm_rows_kernel<T><<<g, 256, 0, ctx->stream>>>(b, ldb, perm, n, nrhs, x1, n, guard);
     count_launches(3);
     ALG_CUDA_TRY(cudaGetLastError());
   }
@@ -631,7 +632,7 @@ int lu_solve_blocked_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* p
   }
   count_launches(2 * nblk);
   ALG_CUDA_TRY(cudaGetLastError());
-  ALG_TRY(store_solution_dev<T>(ctx, x1, n, nrhs, b, ldb, nullptr));
+  ALG_TRY(store_solution_dev<T>(ctx, x1, n, nrhs, b, ldb, guard));
   prof_end(ctx, tok, 2.0 * n * n * nrhs, sizeof(T) * (double(n) * n + 4.0 * n * nrhs));
   return ALG_OK;
 }
@@ -642,8 +643,7 @@ int lu_solve_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* 
   if (nrhs > 65535) return ALG_BAD_SHAPE;
   // the exact form keeps the reference's per-entry order (the dataflow
   // sweeps); the fused forms solve many right-hand sides blocked
-  if (!EXACT && nrhs >= kBlockedSolveRhs && guard == nullptr)
-    return lu_solve_blocked_dev<T>(ctx, lu, n, lda, perm, b, nrhs, ldb);
+  if (!EXACT && nrhs >= kBlockedSolveRhs) return lu_solve_blocked_dev<T>(ctx, lu, n, lda, perm, b, nrhs, ldb, guard);
   return lu_solve_dataflow_dev<T, EXACT>(ctx, lu, n, lda, perm, b, nrhs, ldb, guard);
 }
 
@@ -690,16 +690,19 @@ int solve_any(alg_ctx* ctx, int update, const double* d_lu, int n, int lda, cons
 }
 
 // The solve after factor_any's factorization, and the status of both;
-// *singular: it met a zero pivot, and b is as it was. With up to one group of
-// the sweeps' right-hand sides the solve is launched at once, guarded, so a
-// dgesv has one synchronisation (n = 96: 168 us against 180). With more the host
-// looks first: the synchronisation is a small part of that solve, which a
-// singular matrix does not pay (nor what the solve would refuse or allocate).
-constexpr int kGuardedRhs = 4;
+// *singular: it met a zero pivot, and b is as it was. With few right-hand sides
+// the solve is launched at once, guarded, so a dgesv has one synchronisation
+// (n = 96: 168 us against 180; n = 777 fused with 64 right-hand sides 1 615
+// against 1 638). With more the host looks first: the synchronisation is then a
+// small part of the solve, and a singular matrix does not pay for it (nor meet
+// what it would refuse or allocate). The line: one group of the exact sweeps
+// (with four, a singular call with 16 right-hand sides took 2.2 ms at n = 300,
+// three quarters of it the solve), two column tiles of the blocked solve.
+int guarded_rhs(int update) { return update == ALG_UPDATE_EXACT ? 4 : 64; }
 
 int solve_factored(alg_ctx* ctx, int update, const double* d_lu, int n, int lda, const int* d_perm, double* d_b,
                    int nrhs, int ldb, bool* singular) {
-  const bool guarded = nrhs <= kGuardedRhs;
+  const bool guarded = nrhs <= guarded_rhs(update);
   int rc = ALG_OK;
   if (guarded) rc = solve_any(ctx, update, d_lu, n, lda, d_perm, d_b, nrhs, ldb, ctx->d_status);
   ALG_TRY(alg::status_fetch(ctx));  // a timed-out sweep is an error, not a result

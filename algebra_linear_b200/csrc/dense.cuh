@@ -62,7 +62,7 @@ size_t lu_label_bytes(int m, int nc, int nb, size_t elem_bytes);
 
 // Solves with the packed factors: b (n x nrhs, ldb) becomes x. Stream-ordered.
 // guard (may be null): the status block of the factorization; when that failed,
-// b stays as it is. (A guarded solve takes the sweeps, whatever nrhs is.)
+// b stays as it is.
 template <typename T, bool EXACT>
 int lu_solve_dev(alg_ctx* ctx, const T* lu, int n, int lda, const int* perm, T* b, int nrhs,
                  int ldb, const DevStatus* guard = nullptr);

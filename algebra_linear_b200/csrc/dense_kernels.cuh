@@ -1315,10 +1315,12 @@ __global__ void __launch_bounds__(256) block_solve_step_kernel(const T* __restri
     }
 }
 
-// x[i, c] = b[perm[i], c] (the row interchanges of P, n x ncols)
+// x[i, c] = b[perm[i], c] (the row interchanges of P, n x ncols); with a guard,
+// nothing when its factorization failed
 template <typename T>
 __global__ void gather_perm_rows_kernel(const T* __restrict__ b, int ldb, const int* __restrict__ perm, int n,
-                                        int ncols, T* __restrict__ x, int ldx) {
+                                        int ncols, T* __restrict__ x, int ldx, const DevStatus* guard) {
+  if (guard != nullptr && factor_failed(guard)) return;
   const size_t cnt = (size_t)n * ncols;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(e % n), c = (int)(e / n);
