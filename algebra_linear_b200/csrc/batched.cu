@@ -253,7 +253,7 @@ __device__ int cta_getrf(T* a, int n, T* rhs, int* ipiv, int* perm, unsigned cha
       }
       if (mt > 0) {  // (then w == PB)
         const int cm = min(cw, mt - cb);  // the chunk's matrix columns
-        cta_update<PB, NW, true>(tile + PB, ldt, u, ldu, a + (size_t)(kr + cb) * n + kr, n, mt, cm);
+        cta_update<PB, NW, true, sizeof(T) == 8 && (NT * RPT > 256)>(tile + PB, ldt, u, ldu, a + (size_t)(kr + cb) * n + kr, n, mt, cm);
         if (cm < cw)  // and the right-hand side
           for (int r = tid; r < mt; r += NT) {
             T acc = rhs[kr + r];
@@ -408,7 +408,7 @@ struct BatchArgs {
 // passes through L2 and HBM (n^3 / PB bytes of it per system and direction);
 // 20 000 systems of order 8..512, FP64: 81 ms before (panel columns with three
 // barriers each in shared memory, the update on the CUDA cores, sweeps of two
-// barriers a column), 29.2 ms now; 3 000 in the mixed form 11.1 and 5.7 ms.
+// barriers a column), 27.4 ms now; 3 000 in the mixed form 11.1 and 5.1 ms.
 template <int NT, int RPT, int PB>
 __global__ void __launch_bounds__(NT, RPT == 4 ? 2 : 512 / NT) batched_gesv_kernel(BatchArgs p) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -511,17 +511,17 @@ BatchKernel batch_kernel(int cap, int threads, int panel) {
 // The launch shape of a bucket when no autotuner chose one. With more systems
 // than SMs throughput counts: small CTAs, several to an SM, so that one
 // system's column chain runs beside another's update (1 500 systems of order
-// 257..512 in FP64: 128 x 16 10.8 ms, 256 x 16 11.9 ms, 512 x 32 12.0 ms; 3 000
-// of 129..256: 256 x 16 4.43 ms, 128 x 16 4.45 ms, 256 x 32 4.8 ms; 4 000 of
-// 65..128: 128 x 16 1.24 ms, 128 x 32 1.41 ms). The mixed form's longest systems
-// prefer the wide panel (128 x 32 11.6 ms, 128 x 16 12.0 ms). A few systems
+// 257..512 in FP64: 128 x 16 10.8 ms, 256 x 16 11.3 ms, 512 x 32 11.8 ms; 3 000
+// of 129..256: 128 x 16 3.36 ms, 256 x 16 3.45 ms, 256 x 32 4.0 ms; 4 000 of
+// 65..128: 128 x 16 0.98 ms, 128 x 32 1.32 ms). The mixed form's longest systems
+// prefer the wide panel (128 x 32 11.1 ms, 128 x 16 12.9 ms). A few systems
 // run one to an SM: a thread per row and the wide panel's fewer sweeps.
 void default_batch_shape(int cap, bool mixed, bool few, int* threads, int* panel) {
   if (few) {
     *threads = std::max(128, std::min(512, cap));
     *panel = 32;
   } else {
-    *threads = cap == 256 && !mixed ? 256 : 128;
+    *threads = 128;
     *panel = mixed && cap >= 512 ? 32 : 16;
   }
 }

@@ -55,8 +55,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // under a dominant diagonal is much larger than its products): error of the
 // sparse solution, geometric mean over 2-D and 3-D grids of 1 600 to 90 000
 // unknowns, 1.27 times larger in FP64, 1.29 times in unrefined FP32, twice as
-// large after refinement. The subtraction costs nothing (300 x 300 grid 22.7 ms
-// accumulated, 22.3 ms summed apart; 20 000 batched systems 29.6 and 29.2 ms).
+// large after refinement.
 // Rows and columns past the edge read padding and are not stored.
 struct TileF64 {  // FP64 tensor cores
   double c[4][2][2];
@@ -172,14 +171,28 @@ struct TileF32 {  // CUDA cores; a lane has rows 4 rg .. 4 rg + 3 and columns 4 
 };
 
 // All tiles of C (mt x cw) -= L U, dealt to the CTA's NW warps (ALIGNED: L
-// starts on 16 bytes; U always does); a warp loads
-// its next tile while it updates one (the loads' latency was most of the
-// update's time: n = 400, 670 us per system without).
-template <int K, int NW, bool ALIGNED, typename T>
+// starts on 16 bytes; U always does). A tile's C is asked for before its products
+// are summed and needed after them, which hides the round trip to L2. AHEAD: a
+// warp loads its next tile's C while it updates one, for matrices that come from
+// HBM (1 500 FP64 systems of order 257..512: 10.8 ms with it, 11.3 without);
+// elsewhere the second tile's registers cost more (3 000 of 129..256: 4.4 ms with
+// it, 3.4 without; FP64 small fronts of the 300 x 300 grid 11.5 and 9.4 ms, FP32
+// 8.4 and 8.0). Accumulated into C, with the next tile ahead: 11.2, 4.3, 11.2, 8.8.
+template <int K, int NW, bool ALIGNED, bool AHEAD, typename T>
 __device__ __noinline__ void cta_update(const T* L, int ldl, const T* U, int ldu, T* C, int n, int mt, int cw) {
   using Tile = std::conditional_t<sizeof(T) == 8, TileF64, TileF32>;
   const int tr = (mt + 31) / 32, tiles = tr * ((cw + 15) / 16);
   int cur = threadIdx.x >> 5;
+  if constexpr (!AHEAD) {
+    for (; cur < tiles; cur += NW) {
+      Tile t;
+      const int r0 = 32 * (cur % tr), c0 = 16 * (cur / tr);
+      t.load(C, n, r0, c0, mt, cw);
+      t.template update<K, ALIGNED>(L, ldl, U, ldu, r0, c0);
+      t.store(C, n, r0, c0, mt, cw);
+    }
+    return;
+  }
   if (cur >= tiles) return;
   Tile t0, t1;
   int r0 = 32 * (cur % tr), c0 = 16 * (cur / tr), r1 = 0, c1 = 0;

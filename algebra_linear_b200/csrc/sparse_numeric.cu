@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(kSmallThreads) small_front_z_kernel(SmallArgs<
 // cores / FP32 register tiles). Bound by the column chain of the level's
 // largest front (about 0.8 us a column) where a level has few fronts. The
 // 192-dof lattice (one front of 192 x 192): 2.90 ms with rank-1 updates in
-// global memory and three barriers a column, 0.37 ms now; the 300 x 300
-// grid's 27 levels, FP32: 18.6 ms before, 8.5 ms now (twice as many columns
+// global memory and three barriers a column, 0.32 ms now; the 300 x 300
+// grid's 27 levels, FP32: 18.6 ms before, 8.0 ms now (twice as many columns
 // per chunk changes neither). CTAs of 64, 128 and 256 threads for fronts of as
 // many rows: idle warps would lengthen every barrier.
 template <int NT>
@@ -475,8 +475,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) small_front_kernel(SmallArgs<T> 
         if (i < w && c < cw) fc[(k0 + i) + (int64_t)c * rows] = u[i * ldu + c];
       }
       if (mt > 0) {
-        if (w == PB) cta_update<PB, NW, true>(tile + PB, ldt, u, ldu, fc + kr, rows, mt, cw);
-        else cta_update<PB, NW, false>(tile + w, ldt, u, ldu, fc + kr, rows, mt, cw);
+        if (w == PB) cta_update<PB, NW, true, false>(tile + PB, ldt, u, ldu, fc + kr, rows, mt, cw);
+        else cta_update<PB, NW, false, false>(tile + w, ldt, u, ldu, fc + kr, rows, mt, cw);
       }
       __syncthreads();
     }
