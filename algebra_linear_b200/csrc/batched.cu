@@ -405,7 +405,7 @@ struct BatchArgs {
 
 // RPT rows per thread: systems of up to NT * RPT rows. Bound by the column
 // chain (latency) and, for the largest orders, by the trailing matrix's
-// passes through L2 and HBM (n^3 / PB bytes of it per system and direction);
+// passes through L2 and HBM (8 n^3 / 3 PB bytes of it per system and direction);
 // 20 000 systems of order 8..512, FP64: 81 ms before (panel columns with three
 // barriers each in shared memory, the update on the CUDA cores, sweeps of two
 // barriers a column), 27.4 ms now; 3 000 in the mixed form 11.1 and 5.1 ms.

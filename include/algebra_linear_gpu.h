@@ -232,7 +232,8 @@ int alg_dgesv_dev(alg_ctx* ctx, int update, double* d_a, int n, int lda,
  * strategy, column-serial panel); tournament pivoting (CALU's TSLU, Grigori,
  * Demmel and Xiang, SIMAX 2011: each leaf panel's pivot rows are chosen by a
  * reduction tree of partial-pivoting LUs over row blocks, so the column-serial
- * chain runs on 256-row blocks instead of the whole panel); or a random
+ * chain runs on 256-row blocks instead of the whole panel; panels of up to
+ * 8 192 rows fit one cluster, which pivots partially); or a random
  * butterfly transformation of A followed by LU without pivoting (Baboulin,
  * Dongarra, Herrmann, Tomov, ACM TOMS 2013; needs n divisible by 4; falls back
  * to pivoting on a zero pivot). AUTO: tournament pivoting for n >= 2048,
