@@ -45,7 +45,7 @@ namespace {
 // column step, the exchange between CTAs costs about 0.35 us a column.
 // ALG_PANEL_ROWS overrides it (tuning). 256 (one register row per thread up
 // to 4 096 rows): a 64-column block of 256 / 512 / 1 024 / 2 048 FP64 rows in
-// 59 / 77 / 78 / 80 us; 128 rows per CTA: 65 / 66 / 68 / 74 us. Inside a
+// 58 / 74 / 76 / 79 us; 128 rows per CTA: 62 / 64 / 67 / 72 us. Inside a
 // factorization the two are within 1 % of each other (exact n = 5001 13.09 and
 // 12.95 ms, 48^3 grid 134.1 and 134.6 ms, fused n = 16384 equal). 512 rows per
 // CTA leave no room for the block (97 us and more, leaf by leaf).
@@ -166,7 +166,7 @@ int launch_panel_reg(alg_ctx* ctx, const PanelArgs<T>& args, int C) {
 // its records, and a TRSM and an update launch per leaf):
 //   rows      256       1 024     4 096     6 000     16 384
 //   before    45 / 237  47 / 243  49 / 249   - / 292  102 /  -
-//   now       14 / 59   18 / 78   19 / 86    - / 110   32 /  -
+//   now       14 / 58   17 / 76   19 / 85    - / 108   32 /  -
 template <typename T, bool EXACT>
 int launch_panel(alg_ctx* ctx, const PanelArgs<T>& args) {
   constexpr int W = panel_leaf_w<T>();
@@ -409,7 +409,7 @@ int lu_factor_partial_dev(alg_ctx* ctx, T* a, int m, int nc, int ntot, int lda, 
       // a whole block per launch where it fits on the chip, else leaf by leaf.
       // With tournament pivoting too: a panel that one cluster holds is a
       // tree of one node, whose partial-pivoting LU is the panel's (FP32, 64
-      // columns of 5 000 rows: 96 us against 2 x 64 us for the three levels
+      // columns of 5 000 rows: 94 us against 2 x 64 us for the three levels
       // plus the update between; of 2 000 rows 70 us).
       const bool whole = nbl == panel_leaf_w<T>() && block_panel_fits<T>(m - c0);
       w = std::min(whole ? kBlockMaxW : nbl, k0 + kb - c0);

@@ -716,15 +716,24 @@ __global__ void __launch_bounds__(NT, 1) panel_reg_kernel(PanelArgs<T> p) {
     if (tc > 0) {  // (then w == W)
       if (C > 1) cl.sync();
       else __syncthreads();
-#pragma unroll 4
-      for (int e = tid; e < W * (W + tc); e += NT) {
-        const int j = e % W, c = e / W;  // pivot row j, column c of the leaf and those right of it
-        if (c < j || c >= W) {
-          const int src = piv_src[j];
-          T v;
-          ld_cluster(v, mapa_u32(tile_base + (uint32_t)sizeof(T) * ((cl0 + c) * ldt + (src & 0xffff)), src >> 16));
-          if (c < W) l11[j * W + c] = v;
-          else ubuf[(c - W) * W + j] = v;
+      // entry e: pivot row j = e % W, column c = e / W of the leaf and those right of it
+      constexpr int kPull = 8;  // in flight per thread
+      const int pulls = W * (W + tc);
+      for (int e0 = tid; e0 < pulls; e0 += kPull * NT) {
+        T pv[kPull];
+#pragma unroll
+        for (int i = 0; i < kPull; ++i) {
+          const int e = e0 + i * NT, j = e % W, c = e / W;
+          if (e < pulls && (c < j || c >= W)) {
+            const int src = piv_src[j];
+            ld_cluster(pv[i], mapa_u32(tile_base + (uint32_t)sizeof(T) * ((cl0 + c) * ldt + (src & 0xffff)), src >> 16));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kPull; ++i) {
+          const int e = e0 + i * NT, j = e % W, c = e / W;
+          if (e < pulls && c < j) l11[j * W + c] = pv[i];
+          if (e < pulls && c >= W) ubuf[(c - W) * W + j] = pv[i];
         }
       }
       __syncthreads();
